@@ -1304,6 +1304,7 @@ void Ctx::Destroy() {
   sg_pad_z.Release();
   pad_idx.Release();
   pad_val.Release();
+  dot_terms.Release();
   if (stream != nullptr) {
     // every block of the stream is idle after the synchronisation above
     CacheRetire(stream, device);

@@ -46,6 +46,7 @@ struct Ctx {
   DevBuf<unsigned char> sg_pad_z;        // padded fused Z values
   DevBuf<int32_t> pad_idx;               // padded rows of the union and drop steps
   DevBuf<unsigned char> pad_val;         // padded values of the union and drop steps
+  DevBuf<double> dot_terms;              // products of a dot in the reference's order
   double* host_scalars = nullptr;   // pinned, kScalarSlots
   int64_t* host_counts = nullptr;   // pinned, 8
   int32_t* host_flags = nullptr;    // pinned, 8
@@ -128,6 +129,14 @@ void ColumnSquares(Ctx& ctx, CscView<T> x, double* partial);
 // sum over rows present in both columns of x*y, ascending rows.
 template <class T>
 void ColumnDots(Ctx& ctx, CscView<T> x, CscView<T> y, double* partial);
+
+// Sums in the reference's order (ordered_sum.cu): out[b] = the sequential sum
+// through the columns [first[b], first[b + 1]) of x's squares, or of the
+// products x*y on the common pattern (device arrays; first has batches + 1).
+template <class T>
+void OrderedSquares(Ctx& ctx, const DevCsc<T>& x, const int64_t* first, int64_t batches, double* out);
+template <class T>
+void OrderedDots(Ctx& ctx, const DevCsc<T>& x, const DevCsc<T>& y, const int64_t* first, int64_t batches, double* out);
 
 // Union combination: out = ys*Y (+) xs*X (sparse_operations.cpp:22-49).
 // kAxpby prunes exact zeros; kHalfSum computes 0.5*(y + x) and keeps zeros

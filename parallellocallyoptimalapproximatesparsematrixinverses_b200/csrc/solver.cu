@@ -36,51 +36,6 @@ __device__ __forceinline__ double SafeQuotient(double num, double den) {
   return isfinite(q) ? q : 0.0;
 }
 
-// The reference's summation order: thread per column batch, sequential over
-// the batch's columns in storage order (AccSquares / AccDot of a batch).
-template <class T>
-__global__ void BatchSquaresKernel(CscView<T> x, const int64_t* __restrict__ first, int64_t batches,
-                                   double* __restrict__ out) {
-  for (int64_t b = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; b < batches;
-       b += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    double s = 0.0;
-    for (int64_t p = x.ptr[first[b]]; p < x.ptr[first[b + 1]]; ++p) {
-      const double v = static_cast<double>(x.val[p]);
-      s = Add(s, Mul(v, v));
-    }
-    out[b] = s;
-  }
-}
-
-template <class T>
-__global__ void BatchDotsKernel(CscView<T> x, CscView<T> y, const int64_t* __restrict__ first, int64_t batches,
-                                double* __restrict__ out) {
-  for (int64_t b = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; b < batches;
-       b += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    double s = 0.0;
-    for (int64_t j = first[b]; j < first[b + 1]; ++j) {
-      int64_t p = x.ptr[j];
-      int64_t q = y.ptr[j];
-      const int64_t pe = x.ptr[j + 1];
-      const int64_t qe = y.ptr[j + 1];
-      while (p < pe && q < qe) {
-        const int32_t rp = x.idx[p];
-        const int32_t rq = y.idx[q];
-        if (rp == rq) {
-          s = Add(s, Mul(static_cast<double>(x.val[p]), static_cast<double>(y.val[q])));
-          ++p;
-          ++q;
-        } else if (rp < rq) {
-          ++p;
-        } else {
-          ++q;
-        }
-      }
-    }
-    out[b] = s;
-  }
-}
-
 // Canonical device CSC (int64 offsets and rows) -> int32 rows in dst, with
 // *bad |= 1 for offsets that do not run from 0 to nnz or decrease, and
 // |= 2 for rows out of [0, n) or not strictly increasing in a column.
@@ -852,15 +807,11 @@ class Solver final : public SolverBase {
   // common pattern, each sequential through its batch.
   std::vector<double> BatchSums(const DevCsc<T>* x, const DevCsc<T>* y) {
     const int64_t count = static_cast<int64_t>(batch_first_.size()) - 1;
-    const int grid = GridFor(count, 64);
     if (y == nullptr) {
-      BatchSquaresKernel<T><<<grid, 64, 0, ctx_.stream>>>(View(*x), batch_first_dev_.data(), count,
-                                                          batch_sums_.data());
+      OrderedSquares(ctx_, *x, batch_first_dev_.data(), count, batch_sums_.data());
     } else {
-      BatchDotsKernel<T><<<grid, 64, 0, ctx_.stream>>>(View(*x), View(*y), batch_first_dev_.data(), count,
-                                                       batch_sums_.data());
+      OrderedDots(ctx_, *x, *y, batch_first_dev_.data(), count, batch_sums_.data());
     }
-    SPAI_LAUNCH_CHECK();
     std::vector<double> out(static_cast<size_t>(count));
     SPAI_CUDA(cudaMemcpyAsync(out.data(), batch_sums_.data(), sizeof(double) * count, cudaMemcpyDeviceToHost,
                               ctx_.stream));
