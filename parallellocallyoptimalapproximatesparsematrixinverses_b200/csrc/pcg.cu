@@ -1,32 +1,62 @@
 // PCG evaluator on sm_100a (reference methods_cython/backward_error.pyx:69-144).
 //
-// A whole solve is one CUDA graph launch: a prologue (x = 0, r = b, z = M r,
-// p = z, ||b|| and <r, z>), a device-side WHILE loop whose body is one PCG
-// iteration, and an epilogue (the true residual at exit).  Every scalar of
-// the recurrence -- alpha, beta, the residual history, the stop tests and the
-// status code -- lives in a device-resident PcgState and is decided by the
-// kernels themselves, so the loop needs no host round trip; the body's last
-// kernel sets the loop's condition.  The host reads the history back once,
-// after the solve.
+// A whole solve is one cooperative kernel.  Its blocks form clusters of
+// eight; a cluster owns whole 4096-row chunks of the canonical tree
+// (tree.cuh), block k of it the chunk's tree lanes 32k .. 32k+31, and warp w
+// of the block the w-th term of those lanes: every thread owns one row of a
+// chunk.  An iteration has two grid-wide reductions and nothing else that
+// waits:
 //
-// Dot products keep the library's canonical tree (tree.cuh): each dot kernel
-// runs one block per 4096-value chunk, its lanes forming the chunk sums in
-// the tree's order, and the last block to finish folds the chunk sums with
-// the same tree; the vector updates that precede a dot (x += alpha p and
-// r -= alpha A p, r = b - A x) are fused into it.  The CPU oracle therefore
-// reproduces every iterate bit for bit, as with the stepwise host loop this
-// replaces.
+//   1. p = z + beta p and ap = A p, the neighbours' p formed on the fly from
+//      z and the previous p; the dot <p, ap>.
+//   2. x += alpha p, r -= alpha ap and z = M r, the neighbours' r formed on
+//      the fly from the previous r and ap; the dots <r, r> and <r, z>.
 //
-// Graphs are built once per (device, n, precision of M) and kept: every
-// pointer a solve uses is read from the PcgState, so a new solve only uploads
-// that struct (about 250 bytes) before launching.
+// (p and r alternate between two buffers, so that no thread overwrites what a
+// neighbour still reads.)  A refresh -- at convergence or periodic -- adds
+// r = b - A x with its dot and z = M r with its dot.  Recomputing a
+// neighbour's value repeats the owner's operations on the same inputs, so it
+// has the owner's bits; the dots keep the tree's order, and the CPU oracle
+// reproduces every iterate bit for bit.
+//
+// A reduction: the 16 terms of a lane are added in order through shared
+// memory; the lane sums travel to the cluster's first block as asynchronous
+// remote stores counted by a barrier in its shared memory, whose warps fold
+// them to the chunk's sum.  With one chunk (n <= 4096) every block receives
+// and folds them, and a cluster barrier publishes the vectors.  Otherwise
+// every block announces its vectors on one counter (after a fence; that takes
+// about 1,200 cycles, so it runs beside the folding), the chunk sums go to
+// global memory as 16-byte words that carry the reduction's number, and every
+// block polls both and folds the tree's next level itself.  The polls are
+// bounded: a block that gives up poisons the counter, every other block sees
+// that at its next reduction, and the solve ends with an error.  Every block
+// decides the recurrence's scalars from the totals; the history keeps ||r||^2
+// until the end, so that no square root or division is on the way to the next
+// iteration unless the stop test is close.
+//
+// What bounds it: while every cluster owns one chunk (about 70,000 rows) the
+// latency of an iteration's two reductions and gathers; the rows of both
+// matrices then stay in shared memory for the whole solve where they fit.
+// Beyond, the L2 reads of the two matrices and the gathers; the matrices are
+// re-laid out once per solve in slices of 32 rows (entry e of the 32 rows side
+// by side), so that a warp reads full lines, and a slice whose longest row
+// would waste more than half of it stays in CSR.
+// Measured per iteration, against one graph node per product and per dot
+// (thread-per-row CSR products, dots on one block per chunk): 5.8 us against
+// 29 us at n = 3,969; 14 against 30 at 62,500; 17.4 against 39 at 90,000; 43
+// against 61 at 262,144 (M in FP32, about 18 entries a row).
 
 #include <cuda_runtime.h>
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
-#include <memory>
+#include <cstring>
+#include <map>
 #include <mutex>
+#include <stdexcept>
+#include <type_traits>
 #include <vector>
 
 #include "device.cuh"
@@ -37,398 +67,708 @@
 
 namespace spai {
 
-void CountLaunches(int64_t count);
-
 namespace {
 
-// Device-resident state of one solve.  The host writes the inputs before the
-// graph launch; the kernels own the recurrence fields.
-struct PcgState {
-  // A (FP64) and M (FP64 or FP32 values) as CSR with int32 column indices
-  const int64_t* a_ptr;
-  const int32_t* a_idx;
-  const double* a_val;
-  const int64_t* m_ptr;
-  const int32_t* m_idx;
-  const void* m_val;
+namespace cg = cooperative_groups;
+
+constexpr int kClusterBlocks = 8;   // kTreeLanes / kWarp: one warp-wide group of tree lanes per block
+constexpr int kSolveThreads = kWarp * kTreeTerms;  // one warp per term of a lane
+constexpr int kGroupRounds = 4;     // chunks of a cluster folded at a time
+constexpr unsigned kPollLimit = 1u << 22;       // polls (seconds) before the solve is abandoned
+constexpr unsigned long long kPoison = 1ull << 63;  // set in a cluster's counter by a block that gave up
+constexpr int kFlagStride = 16;                 // counters 128 bytes apart
+static_assert(kClusterBlocks * kWarp == kTreeLanes, "a cluster covers a chunk's lanes");
+
+// A row-compressed matrix and its sliced copy.
+template <class TV>
+struct SolveMatrix {
+  const int64_t* ptr;
+  const int32_t* idx;
+  const TV* val;
+  int64_t* slice;      // per slice of 32 rows: offset in the sliced copy, or -1 (rows stay in CSR)
+  int32_t* slice_idx;
+  TV* slice_val;
+  unsigned long long* used;  // entries of the sliced copy taken so far
+};
+
+// A chunk sum on its way between clusters: the value and the reduction it belongs to, in one 16-byte word.
+struct alignas(16) TaggedSum {
+  double sum;
+  unsigned long long tag;
+};
+
+struct SolveOutcome {
+  int64_t count;
+  int64_t status;
+  int32_t aborted;  // a poll ran into its limit
+  int32_t pad;
+};
+
+template <class TM>
+struct SolveArgs {
+  SolveMatrix<double> a;
+  SolveMatrix<TM> m;
   const double* b;
   double* x;
-  double* r;
+  double* r[2];
+  double* p[2];
   double* z;
-  double* p;
   double* ap;
-  double* history;        // max_iterations entries
-  double* partial;        // chunk sums: 2 * chunks
-  unsigned int* arrive;   // blocks of the running dot kernel that are done
+  double* history;
+  TaggedSum* partial;  // chunk sums: 2 alternating sets of 2 * chunks (tags zero at the start)
+  unsigned long long* arrived;  // per cluster (kFlagStride apart): blocks whose vectors are visible, over all reductions
+  SolveOutcome* outcome;
   int64_t n;
   int64_t chunks;
   int64_t max_iterations;
   int64_t refresh_period;
   double tolerance;
-  int64_t body_limit;     // hard cap on loop-body executions
-  // the recurrence (backward_error.pyx:100-143)
-  double r_z;
-  double alpha;
-  double beta;
-  double error;
-  double b_norm;
-  int64_t count;
-  int64_t status;
-  int64_t done;
-  int64_t refresh;
-  int64_t converged_refresh;
-  int64_t bodies;         // loop-body executions so far
+  int room;            // bytes of dynamic shared memory after SolveShared
 };
 
-// Which product a SpMV launch forms.
-enum SpmvWhat : int {
-  kMrInit = 0,       // prologue: z = M r and p = z
-  kApFromP = 1,      // loop: ap = A p
-  kApFromX = 2,      // loop, on a refresh: ap = A x
-  kMrLoop = 3,       // loop: z = M r
-  kApFromXFinal = 4  // epilogue: ap = A x
+// One row of a matrix: entry e at idx[e * stride], val[e * stride].
+template <class TV>
+struct RowRef {
+  const int32_t* idx;
+  const TV* val;
+  int stride;
+  int len;
+  int width;  // the longest row of its slice
 };
 
-// Which tree reduction (and fused update) a dot launch forms.
-enum DotWhat : int {
-  kInit = 0,     // r.r and r.z: ||b||, the first <r, z>, history[0]
-  kDen = 1,      // p.ap: alpha, or a breakdown
-  kStep = 2,     // x += alpha p, r -= alpha ap, then r.r: the residual and the refresh decision
-  kRefresh = 3,  // r = b - ap, then r.r (on a refresh only)
-  kRz = 4,       // r.z: beta, the history entry, the stop tests
-  kFinal = 5     // r = b - ap, then r.r: the true residual at exit and the status
-};
-
-__global__ void PcgInitKernel(PcgState* __restrict__ s) {
-  const int64_t n = s->n;
-  const double* __restrict__ b = s->b;
-  double* __restrict__ x = s->x;
-  double* __restrict__ r = s->r;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    x[i] = 0.0;
-    r[i] = b[i];
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    *s->arrive = 0u;
-    s->bodies = 0;
-  }
-}
-
-// One thread per row, entries in storage order (the reference's _row_dot).
-template <class TV, int kWhat>
-__global__ void __launch_bounds__(128) PcgSpmvKernel(PcgState* __restrict__ s) {
-  if (kWhat == kApFromP || kWhat == kMrLoop) {
-    if (s->done) return;
-  }
-  if (kWhat == kApFromX) {
-    if (s->done || !s->refresh) return;
-  }
-  constexpr bool kUseM = kWhat == kMrInit || kWhat == kMrLoop;
-  const int64_t* __restrict__ ptr = kUseM ? s->m_ptr : s->a_ptr;
-  const int32_t* __restrict__ idx = kUseM ? s->m_idx : s->a_idx;
-  const TV* __restrict__ val = kUseM ? static_cast<const TV*>(s->m_val) : reinterpret_cast<const TV*>(s->a_val);
-  const double* __restrict__ in = kWhat == kApFromP ? s->p : (kUseM ? s->r : s->x);
-  double* __restrict__ out = kUseM ? s->z : s->ap;
-  double* __restrict__ copy = kWhat == kMrInit ? s->p : nullptr;
-  const int64_t n = s->n;
-  for (int64_t row = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; row < n;
-       row += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    double sum = 0.0;
-    const int64_t end = ptr[row + 1];
-    for (int64_t k = ptr[row]; k < end; ++k) sum = Add(sum, Mul(static_cast<double>(val[k]), in[idx[k]]));
-    out[row] = sum;
-    if (kWhat == kMrInit) copy[row] = sum;
-  }
-}
-
-// One block of kTreeLanes threads per 4096-value chunk; the last block to
-// finish folds the chunk sums and applies the recurrence (thread 0).
-template <int kWhat>
-__global__ void __launch_bounds__(kTreeLanes) PcgDotKernel(PcgState* __restrict__ s) {
-  __shared__ double shared[kTreeLanes];
-  __shared__ int last;
-  if (kWhat == kDen || kWhat == kStep || kWhat == kRz) {
-    if (s->done) return;
-  }
-  if (kWhat == kRefresh) {
-    if (s->done || !s->refresh) return;
-  }
-  const int64_t n = s->n;
-  const int t = threadIdx.x;
-  const int64_t base = static_cast<int64_t>(blockIdx.x) * kTreeChunk + t;
-  double* __restrict__ r = s->r;
-  const double* __restrict__ z = s->z;
-  const double* __restrict__ p = s->p;
-  const double* __restrict__ ap = s->ap;
-  const double* __restrict__ b = s->b;
-  double* __restrict__ x = s->x;
-  const double alpha = kWhat == kStep ? s->alpha : 0.0;
-  double acc0 = 0.0;
-  double acc1 = 0.0;
+// Entries of a slice's rows: the longest row, and whether slicing wastes at most half.
+template <class TV>
+__device__ __forceinline__ int SliceWidth(const SolveMatrix<TV>& m, int64_t row, int64_t n, int64_t* first, int* len,
+                                          bool* dense) {
+  *first = row < n ? m.ptr[row] : 0;
+  *len = row < n ? static_cast<int>(m.ptr[row + 1] - *first) : 0;
+  const int width = __reduce_max_sync(0xffffffffu, *len);
+  long long total = *len;
 #pragma unroll
-  for (int m = 0; m < kTreeTerms; ++m) {
-    const int64_t i = base + static_cast<int64_t>(kTreeLanes) * m;
-    if (i < n) {
-      if (kWhat == kInit) {
-        const double ri = r[i];
-        acc0 = Add(acc0, Mul(ri, ri));
-        acc1 = Add(acc1, Mul(ri, z[i]));
-      } else if (kWhat == kDen) {
-        acc0 = Add(acc0, Mul(p[i], ap[i]));
-      } else if (kWhat == kStep) {
-        const double pi = p[i];
-        x[i] = Add(x[i], Mul(alpha, pi));
-        const double ri = __dsub_rn(r[i], Mul(alpha, ap[i]));
-        r[i] = ri;
-        acc0 = Add(acc0, Mul(ri, ri));
-      } else if (kWhat == kRefresh || kWhat == kFinal) {
-        const double ri = __dsub_rn(b[i], ap[i]);
-        r[i] = ri;
-        acc0 = Add(acc0, Mul(ri, ri));
-      } else {  // kRz
-        acc0 = Add(acc0, Mul(r[i], z[i]));
+  for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+  *dense = static_cast<long long>(width) * kWarp <= 2 * total + 2 * kWarp;
+  return width;
+}
+
+// Copies the 32 rows of a slice, one per lane, into the sliced layout when
+// that wastes at most half of it (the copy then never exceeds twice the
+// entries plus two per row, what the host reserves).
+template <class TV>
+__device__ void SliceRows(const SolveMatrix<TV>& m, int64_t slice, int64_t n, int lane) {
+  int64_t first;
+  int len;
+  bool dense;
+  const int width = SliceWidth(m, slice * kWarp + lane, n, &first, &len, &dense);
+  long long at = -1;
+  if (dense) {
+    if (lane == 0) at = static_cast<long long>(atomicAdd(m.used, static_cast<unsigned long long>(width) * kWarp));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    for (int e = 0; e < len; ++e) {
+      m.slice_idx[at + static_cast<int64_t>(e) * kWarp + lane] = m.idx[first + e];
+      m.slice_val[at + static_cast<int64_t>(e) * kWarp + lane] = m.val[first + e];
+    }
+  }
+  if (lane == 0) m.slice[slice] = at;
+}
+
+template <class TV>
+__device__ __forceinline__ RowRef<TV> FindRow(const SolveMatrix<TV>& m, int64_t row) {
+  const int64_t first = m.ptr[row];
+  const int len = static_cast<int>(m.ptr[row + 1] - first);
+  const int64_t at = m.slice[row >> 5];
+  if (at >= 0) return RowRef<TV>{m.slice_idx + at + (row & 31), m.slice_val + at + (row & 31), kWarp, len, len};
+  return RowRef<TV>{m.idx + first, m.val + first, 1, len, len};
+}
+
+__device__ __forceinline__ int32_t LoadStreamed(const int32_t* p) {
+  int32_t v;
+  asm volatile("ld.global.L1::no_allocate.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
+__device__ __forceinline__ float LoadStreamed(const float* p) {
+  float v;
+  asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+
+__device__ __forceinline__ double LoadStreamed(const double* p) {
+  double v;
+  asm volatile("ld.global.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+
+// The row times the vector that `in` yields, entries in storage order (the
+// reference's _row_dot).  kResident (rows in shared memory): up to 16 gathers
+// in flight, so that a row waits for one round trip; otherwise four, and the
+// entries pass the L1, which keeps the gathered vectors.
+template <bool kResident, class TV, class In>
+__device__ __forceinline__ double RowDot(const RowRef<TV>& row, In in) {
+  double sum = 0.0;
+  if constexpr (kResident) {
+    const auto group = [&](auto wide, int e0) {
+      constexpr int kWide = decltype(wide)::value;
+      double g[kWide];
+#pragma unroll
+      for (int e = 0; e < kWide; ++e) g[e] = e0 + e < row.len ? in(row.idx[(e0 + e) * row.stride]) : 0.0;
+#pragma unroll
+      for (int e = 0; e < kWide; ++e) {
+        if (e0 + e < row.len) sum = Add(sum, Mul(static_cast<double>(row.val[(e0 + e) * row.stride]), g[e]));
+      }
+    };
+    int e0 = 0;
+    for (; row.width - e0 > 8; e0 += 16) group(std::integral_constant<int, 16>(), e0);
+    if (e0 < row.width) group(std::integral_constant<int, 8>(), e0);
+  } else {
+    constexpr int kWide = 4;
+    for (int e0 = 0; e0 < row.len; e0 += kWide) {
+      int32_t c[kWide];
+      TV v[kWide];
+#pragma unroll
+      for (int e = 0; e < kWide; ++e) {
+        const bool have = e0 + e < row.len;
+        const int64_t at = static_cast<int64_t>(e0 + e) * row.stride;
+        c[e] = have ? LoadStreamed(row.idx + at) : 0;
+        v[e] = have ? LoadStreamed(row.val + at) : TV(0);
+      }
+      double g[kWide];
+#pragma unroll
+      for (int e = 0; e < kWide; ++e) g[e] = e0 + e < row.len ? in(c[e]) : 0.0;
+#pragma unroll
+      for (int e = 0; e < kWide; ++e) {
+        if (e0 + e < row.len) sum = Add(sum, Mul(static_cast<double>(v[e]), g[e]));
       }
     }
   }
-  double total0 = TreeButterfly(acc0, shared);
-  double total1 = kWhat == kInit ? TreeButterfly(acc1, shared) : 0.0;
-  if (gridDim.x > 1) {
-    const int64_t chunks = gridDim.x;
-    if (t == 0) {
-      s->partial[blockIdx.x] = total0;
-      if (kWhat == kInit) s->partial[chunks + blockIdx.x] = total1;
-      __threadfence();
-      last = atomicAdd(s->arrive, 1u) == gridDim.x - 1 ? 1 : 0;
+  return sum;
+}
+
+// The tree's butterfly over 256 values, eight per lane: v[g] is value 32 g + lane.
+__device__ __forceinline__ double FoldLanes(double (&v)[kClusterBlocks]) {
+#pragma unroll
+  for (int o = kClusterBlocks / 2; o > 0; o >>= 1) {
+#pragma unroll
+    for (int g = 0; g < o; ++g) v[g] = Add(v[g], v[g + o]);
+  }
+  double s = v[0];
+#pragma unroll
+  for (int o = kWarp / 2; o >= 1; o >>= 1) s = Add(s, __shfl_xor_sync(0xffffffffu, s, o));
+  return s;
+}
+
+__device__ __forceinline__ unsigned long long LoadAcquire(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ void StoreTagged(TaggedSum* p, double sum, unsigned long long tag) {
+  asm volatile("{\n\t.reg .b128 w;\n\tmov.b128 w, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], w;\n\t}"
+               :: "l"(p), "l"(__double_as_longlong(sum)), "l"(tag) : "memory");
+}
+
+__device__ __forceinline__ TaggedSum LoadTagged(const TaggedSum* p) {
+  long long bits;
+  TaggedSum t;
+  asm volatile("{\n\t.reg .b128 w;\n\tld.relaxed.gpu.global.b128 w, [%2];\n\tmov.b128 {%0, %1}, w;\n\t}"
+               : "=l"(bits), "=l"(t.tag) : "l"(p) : "memory");
+  t.sum = __longlong_as_double(bits);
+  return t;
+}
+
+__device__ __forceinline__ uint32_t SharedAddress(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+// The address of this block's shared variable `local` in block `rank` of the cluster.
+__device__ __forceinline__ uint32_t RemoteAddress(uint32_t local, int rank) {
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+  return remote;
+}
+
+// Stores v to a remote block's shared memory and counts its 8 bytes on that block's barrier.
+__device__ __forceinline__ void StoreCounted(uint32_t remote, uint32_t remote_barrier, double v) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];"
+               :: "r"(remote), "l"(__double_as_longlong(v)), "r"(remote_barrier) : "memory");
+}
+
+__device__ __forceinline__ void ExpectBytes(uint64_t* barrier, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(SharedAddress(barrier)), "r"(bytes)
+               : "memory");
+}
+
+// False when the barrier's phase did not end within the limit.
+__device__ __forceinline__ bool WaitPhase(uint64_t* barrier, unsigned parity) {
+  const uint32_t at = SharedAddress(barrier);
+  for (unsigned polls = 0; polls < kPollLimit; ++polls) {
+    unsigned ended;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ended) : "r"(at), "r"(parity) : "memory");
+    if (ended) return true;
+  }
+  return false;
+}
+
+// Shared memory of a block.
+struct alignas(16) SolveShared {
+  double totals[2][2];                                         // [reduction parity][dot]
+  uint64_t barrier[2];                                         // lane sums of a group have arrived
+  int widths[kTreeTerms];
+  int abort;
+};
+
+// kOneRound: every cluster owns one chunk, one block per SM, and the matrices'
+// rows stay in shared memory where they fit (latency counts); otherwise two
+// blocks per SM (bytes in flight count; one block of 128 registers and eight
+// entries in flight was 5 % slower at n = 262,144).
+template <class TM, bool kOneRound>
+__global__ void __launch_bounds__(kSolveThreads, kOneRound ? 1 : 2) PcgSolveKernel(const SolveArgs<TM> a) {
+  extern __shared__ __align__(16) unsigned char pcg_smem[];
+  SolveShared& sh = *reinterpret_cast<SolveShared*>(pcg_smem);
+  constexpr int kRounds = kOneRound ? 1 : kGroupRounds;
+  double* lanes = reinterpret_cast<double*>(pcg_smem + sizeof(SolveShared));  // [group parity][round][dot][tree lane]
+  double* terms = lanes + 2 * kRounds * 2 * kTreeLanes;                       // [group parity][round][dot][warp][lane]
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = static_cast<int>(cluster.block_rank());
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const int64_t clusters = gridDim.x / kClusterBlocks;
+  const int64_t mine = blockIdx.x / kClusterBlocks;
+  const bool solo = a.chunks == 1;
+  const int64_t in_chunk = static_cast<int64_t>(kTreeLanes) * warp + kWarp * rank + lane;
+  const int64_t n = a.n;
+  const int64_t rounds = (a.chunks - mine + clusters - 1) / clusters;
+  const int64_t groups = kOneRound ? 1 : (rounds + kRounds - 1) / kRounds;
+  unsigned group_count = 0;        // groups of rounds folded so far
+  unsigned long long reduction = 0;  // number of the running reduction, from 1
+  bool aborted = false;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2; ++i) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(SharedAddress(&sh.barrier[i])) : "memory");
+    }
+    sh.abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+
+  // the rows this thread owns (kOneRound), or where to find them
+  RowRef<double> row_a{nullptr, nullptr, 1, 0, 0};
+  RowRef<TM> row_m{nullptr, nullptr, 1, 0, 0};
+  if constexpr (kOneRound) {
+    const int64_t row = mine * kTreeChunk + in_chunk;
+    int64_t first_a;
+    int64_t first_m;
+    bool dense;
+    const int wa = SliceWidth(a.a, row, n, &first_a, &row_a.len, &dense);
+    const int wm = SliceWidth(a.m, row, n, &first_m, &row_m.len, &dense);
+    constexpr int kEntryA = sizeof(double) + sizeof(int32_t);
+    constexpr int kEntryM = sizeof(TM) + sizeof(int32_t);
+    // bytes of the 16 warps' slices (saturated: long rows never fit)
+    if (lane == 0) {
+      const long long bytes = static_cast<long long>(kWarp) * (static_cast<long long>(wa) * kEntryA +
+                                                               static_cast<long long>(wm) * kEntryM);
+      sh.widths[warp] = static_cast<int>(bytes < (1 << 20) ? (bytes + 15) / 16 * 16 : (1 << 20));
     }
     __syncthreads();
-    if (!last) return;
-    __threadfence();
-    total0 = TreeLevel(s->partial, chunks, shared);
-    if (kWhat == kInit) total1 = TreeLevel(s->partial + chunks, chunks, shared);
-    if (t == 0) *s->arrive = 0u;
-  }
-  if (t != 0) return;
-  const double tol = s->tolerance;
-  if (kWhat == kInit) {
-    s->b_norm = __dsqrt_rn(total0);
-    s->r_z = total1;
-    s->history[0] = 1.0;
-    s->count = 1;
-    s->status = 0;
-    s->error = 1.0;
-    s->refresh = 0;
-    s->converged_refresh = 0;
-    s->done = (1 < s->max_iterations && 1.0 > tol) ? 0 : 1;
-  } else if (kWhat == kDen) {
-    const double r_z = s->r_z;
-    const double den = total0;
-    if (!isfinite(r_z) || !isfinite(den) || r_z == 0.0 || den == 0.0) {
-      s->status = 2;
-      s->done = 1;
+    int before = 0;
+    int total = 0;
+    for (int w = 0; w < kTreeTerms; ++w) {
+      before += w < warp ? sh.widths[w] : 0;
+      total += sh.widths[w];
+    }
+    if (total <= a.room) {
+      unsigned char* base = reinterpret_cast<unsigned char*>(terms + 2 * kRounds * 2 * kTreeTerms * kWarp) + before;
+      double* va = reinterpret_cast<double*>(base);
+      TM* vm = reinterpret_cast<TM*>(va + static_cast<size_t>(wa) * kWarp);
+      int32_t* ia = reinterpret_cast<int32_t*>(vm + static_cast<size_t>(wm) * kWarp);
+      int32_t* im = ia + static_cast<size_t>(wa) * kWarp;
+      for (int e = 0; e < row_a.len; ++e) {
+        ia[e * kWarp + lane] = a.a.idx[first_a + e];
+        va[e * kWarp + lane] = a.a.val[first_a + e];
+      }
+      for (int e = 0; e < row_m.len; ++e) {
+        im[e * kWarp + lane] = a.m.idx[first_m + e];
+        vm[e * kWarp + lane] = a.m.val[first_m + e];
+      }
+      row_a = RowRef<double>{ia + lane, va + lane, kWarp, row_a.len, wa};
+      row_m = RowRef<TM>{im + lane, vm + lane, kWarp, row_m.len, wm};
     } else {
-      const double a = __ddiv_rn(r_z, den);
-      if (!isfinite(a)) {
-        s->status = 2;
-        s->done = 1;
-      } else {
-        s->alpha = a;
+      const int64_t slice = row >> 5;
+      if (slice * kWarp < n) {
+        SliceRows(a.a, slice, n, lane);
+        SliceRows(a.m, slice, n, lane);
+        __syncwarp();
+        if (row < n) {
+          row_a = FindRow(a.a, row);
+          row_m = FindRow(a.m, row);
+          row_a.width = wa;
+          row_m.width = wm;
+        }
       }
     }
-  } else if (kWhat == kStep) {
-    const double error = __ddiv_rn(__dsqrt_rn(total0), s->b_norm);
-    const bool converged = error <= tol;
-    const bool periodic = s->refresh_period > 0 && s->count % s->refresh_period == 0;
-    s->error = error;
-    s->converged_refresh = converged ? 1 : 0;
-    s->refresh = (converged || periodic) ? 1 : 0;
-  } else if (kWhat == kRefresh) {
-    s->error = __ddiv_rn(__dsqrt_rn(total0), s->b_norm);
-  } else if (kWhat == kRz) {
-    const double r_z_new = total0;
-    const double beta = s->converged_refresh ? 0.0 : __ddiv_rn(r_z_new, s->r_z);
-    s->r_z = r_z_new;
-    const double error = s->error;
-    const int64_t count = s->count;
-    s->history[count] = error;
-    s->count = count + 1;
-    if (!isfinite(error)) {
-      s->status = 3;
-      s->done = 1;
-    } else if (!isfinite(beta)) {
-      s->status = 2;
-      s->done = 1;
+  } else {
+    for (int64_t c = mine; c < a.chunks; c += clusters) {
+      const int64_t first = c * kTreeChunk + in_chunk - lane;
+      if (first < n) {
+        SliceRows(a.a, first >> 5, n, lane);
+        SliceRows(a.m, first >> 5, n, lane);
+      }
+    }
+    __syncwarp();
+  }
+  const auto a_row = [&](int64_t row) {
+    if constexpr (kOneRound) {
+      return row_a;
     } else {
-      s->beta = beta;
-      if (!(count + 1 < s->max_iterations && error > tol)) s->done = 1;
+      return FindRow(a.a, row);
     }
-  } else {  // kFinal
-    const double h = __ddiv_rn(__dsqrt_rn(total0), s->b_norm);
-    s->history[s->count - 1] = h;
-    if (!isfinite(h)) {
-      s->status = 3;
-    } else if (h <= tol) {
-      s->status = 1;
+  };
+  const auto m_row = [&](int64_t row) {
+    if constexpr (kOneRound) {
+      return row_m;
+    } else {
+      return FindRow(a.m, row);
+    }
+  };
+  cluster.sync();  // the barriers are initialised
+
+  // Runs body(row, d0, d1) for every row this thread owns and reduces d0 (and
+  // d1 when dots == 2) over all rows with the canonical tree into t0, t1; what
+  // the bodies wrote is visible to every block afterwards.
+  auto reduce = [&](int dots, auto body, double& t0, double& t1) {
+    ++reduction;
+    const int parity = static_cast<int>(reduction & 1);
+    int q = 0;
+    int64_t group_first = mine;
+    for (int64_t round = 0; round < rounds; ++round) {
+      const int64_t row = (mine + round * clusters) * kTreeChunk + in_chunk;
+      double d0 = 0.0;  // a missing row adds +0.0 to a sum started at +0.0: no change
+      double d1 = 0.0;
+      if (row < n) body(row, d0, d1);
+      const unsigned gp = group_count & 1;
+      double* mine_at = terms + ((gp * kRounds + q) * 2 * kTreeTerms + warp) * kWarp + lane;
+      mine_at[0] = d0;
+      if (dots == 2) mine_at[kTreeTerms * kWarp] = d1;
+      const bool last = round + 1 == rounds;
+      if (++q == kRounds || last) {
+        __syncthreads();
+        if (last && !solo && threadIdx.x == kSolveThreads - 1) {
+          // this block's vectors are written: announce them (beside the folding below)
+          __threadfence();
+          atomicAdd(a.arrived + mine * kFlagStride, 1ull);
+        }
+        if (warp < q * dots) {
+          const int rq = dots == 2 ? warp >> 1 : warp;
+          const int d = dots == 2 ? warp & 1 : 0;
+          const double* from = terms + ((gp * kRounds + rq) * 2 + d) * kTreeTerms * kWarp + lane;
+          double s = 0.0;
+#pragma unroll
+          for (int t = 0; t < kTreeTerms; ++t) s = Add(s, from[t * kWarp]);
+          const uint32_t slot = SharedAddress(lanes + ((gp * kRounds + rq) * 2 + d) * kTreeLanes + kWarp * rank + lane);
+          const uint32_t barrier = SharedAddress(&sh.barrier[gp]);
+          if (solo) {
+#pragma unroll
+            for (int k = 0; k < kClusterBlocks; ++k) StoreCounted(RemoteAddress(slot, k), RemoteAddress(barrier, k), s);
+          } else {
+            StoreCounted(RemoteAddress(slot, 0), RemoteAddress(barrier, 0), s);
+          }
+        }
+        if (solo) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        if (solo || rank == 0) {
+          if (threadIdx.x == 0) {
+            ExpectBytes(&sh.barrier[gp], static_cast<unsigned>(sizeof(double) * kTreeLanes) * dots * q);
+          }
+          if (warp < q * dots) {
+            if (!WaitPhase(&sh.barrier[gp], (group_count >> 1) & 1)) sh.abort = 1;
+            const int rq = dots == 2 ? warp >> 1 : warp;
+            const int d = dots == 2 ? warp & 1 : 0;
+            const double* from = lanes + ((gp * kRounds + rq) * 2 + d) * kTreeLanes;
+            double v[kClusterBlocks];
+#pragma unroll
+            for (int g = 0; g < kClusterBlocks; ++g) v[g] = from[kWarp * g + lane];
+            const double s = FoldLanes(v);
+            if (lane == 0) {
+              if (solo) {
+                sh.totals[parity][d] = s;
+              } else {
+                StoreTagged(a.partial + (2 * parity + d) * a.chunks + group_first + rq * clusters, s, reduction);
+              }
+            }
+          }
+        }
+        ++group_count;
+        group_first += clusters * q;
+        q = 0;
+        if (!last) cluster.sync();  // the next group but one reuses this group's lanes
+      }
+    }
+    if (solo) {
+      asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+      __syncthreads();
+      t0 = sh.totals[parity][0];
+      t1 = sh.totals[parity][1];
+      aborted = sh.abort != 0;
+      return;
+    }
+    if (warp < dots) {
+      const TaggedSum* sums = a.partial + (2 * parity + warp) * a.chunks;
+      double v[kClusterBlocks];
+      bool lost = false;
+#pragma unroll
+      for (int g = 0; g < kClusterBlocks; ++g) {
+        double s = 0.0;
+        for (int64_t i = kWarp * g + lane; i < a.chunks; i += kTreeLanes) {
+          TaggedSum t = LoadTagged(sums + i);
+          for (unsigned polls = 0; t.tag != reduction && !lost; t = LoadTagged(sums + i)) {
+            lost = ++polls >= kPollLimit;
+          }
+          s = Add(s, t.sum);
+        }
+        v[g] = s;
+      }
+      if (lost) sh.abort = 1;
+      __syncwarp();
+      const double s = FoldLanes(v);
+      if (lane == 0) sh.totals[parity][warp] = s;
+    } else if (warp == 2) {
+      for (int64_t c = lane; c < clusters; c += kWarp) {
+        for (unsigned polls = 0;;) {
+          const unsigned long long seen = LoadAcquire(a.arrived + c * kFlagStride);
+          if (seen >= reduction * kClusterBlocks) {
+            if (seen & kPoison) sh.abort = 1;
+            break;
+          }
+          if (++polls >= kPollLimit) {
+            sh.abort = 1;
+            break;
+          }
+        }
+      }
+    }
+    __syncthreads();
+    t0 = sh.totals[parity][0];
+    t1 = sh.totals[parity][1];
+    aborted = sh.abort != 0;
+    if (aborted && threadIdx.x == 0) atomicOr(a.arrived + mine * kFlagStride, kPoison);
+  };
+
+  double t0 = 0.0;
+  double t1 = 0.0;
+  const bool writer = blockIdx.x == 0 && threadIdx.x == 0;
+  // prologue: x = 0, r = b, z = M r, p = z
+  reduce(2, [&](int64_t row, double& d0, double& d1) {
+    const double ri = a.b[row];
+    a.x[row] = 0.0;
+    a.r[0][row] = ri;
+    const double zi = RowDot<kOneRound>(m_row(row), [&](int32_t c) { return a.b[c]; });
+    a.z[row] = zi;
+    d0 = Mul(ri, ri);
+    d1 = Mul(ri, zi);
+  }, t0, t1);
+  const double b_norm = __dsqrt_rn(t0);
+  // The stop test error = sqrt(rr) / b_norm <= tolerance without the root and
+  // the division while rr is clearly above: where nothing can over- or
+  // underflow, both round within a few ulp, far less than the margin.
+  const double tol = a.tolerance;
+  const bool in_range = b_norm > 1e-100 && b_norm < 1e100 && (tol == 0.0 || (tol > 1e-40 && tol < 1e40));
+  const double clear_above = Mul(Mul(Mul(tol, b_norm), Mul(tol, b_norm)), 1.000001);
+  double r_z = t1;
+  double beta = 0.0;
+  double rr = t0;
+  int64_t count = 1;
+  int64_t status = 0;
+  bool done = !(1 < a.max_iterations && 1.0 > tol);
+  bool first = true;  // p = z on the first iteration, z + beta p afterwards
+  int pb = 0;         // buffer that holds the current p (written in step 1)
+  int rb = 0;         // buffer that holds the current r
+  while (!done && !aborted) {
+    // 1. the direction and A p
+    const double* p_old = pb == 0 ? a.p[0] : a.p[1];
+    double* p_new = pb == 0 ? a.p[1] : a.p[0];
+    const auto direction = [&](int64_t i) {
+      const double zi = a.z[i];
+      return first ? zi : Add(zi, Mul(beta, p_old[i]));
+    };
+    reduce(1, [&](int64_t row, double& d0, double&) {
+      // every load before the first store: a store would wait for its own row's loads
+      const double z_own = a.z[row];
+      const double p_own = first ? 0.0 : p_old[row];
+      const double ap = RowDot<kOneRound>(a_row(row), [&](int32_t c) { return direction(c); });
+      const double pi = first ? z_own : Add(z_own, Mul(beta, p_own));
+      p_new[row] = pi;
+      a.ap[row] = ap;
+      d0 = Mul(pi, ap);
+    }, t0, t1);
+    if (aborted) break;
+    pb ^= 1;
+    first = false;
+    const double den = t0;
+    if (!isfinite(r_z) || !isfinite(den) || r_z == 0.0 || den == 0.0) {
+      status = 2;
+      break;
+    }
+    const double alpha = __ddiv_rn(r_z, den);
+    if (!isfinite(alpha)) {
+      status = 2;
+      break;
+    }
+    // 2. the step, the residual and z = M r
+    const double* r_old = rb == 0 ? a.r[0] : a.r[1];
+    double* r_new = rb == 0 ? a.r[1] : a.r[0];
+    const auto residual = [&](int64_t i) { return __dsub_rn(r_old[i], Mul(alpha, a.ap[i])); };
+    reduce(2, [&](int64_t row, double& d0, double& d1) {
+      const double x_own = a.x[row];
+      const double p_own = p_new[row];
+      const double r_own = r_old[row];
+      const double ap_own = a.ap[row];
+      const double zi = RowDot<kOneRound>(m_row(row), [&](int32_t c) { return residual(c); });
+      const double ri = __dsub_rn(r_own, Mul(alpha, ap_own));
+      a.x[row] = Add(x_own, Mul(alpha, p_own));
+      r_new[row] = ri;
+      a.z[row] = zi;
+      d0 = Mul(ri, ri);
+      d1 = Mul(ri, zi);
+    }, t0, t1);
+    if (aborted) break;
+    rb ^= 1;
+    rr = t0;
+    double r_z_new = t1;
+    bool finite = true;
+    bool above = in_range && rr > clear_above && rr > 1e-200 && rr < 1e200;
+    bool converged = false;
+    if (!above) {
+      const double error = __ddiv_rn(__dsqrt_rn(rr), b_norm);
+      converged = error <= tol;
+      finite = isfinite(error);
+      above = error > tol;
+    }
+    const bool periodic = a.refresh_period > 0 && count % a.refresh_period == 0;
+    if (converged || periodic) {
+      // the true residual replaces the recurrence's
+      reduce(1, [&](int64_t row, double& d0, double&) {
+        const double ax = RowDot<kOneRound>(a_row(row), [&](int32_t c) { return a.x[c]; });
+        const double ri = __dsub_rn(a.b[row], ax);
+        r_new[row] = ri;
+        d0 = Mul(ri, ri);
+      }, t0, t1);
+      if (aborted) break;
+      rr = t0;
+      const double error = __ddiv_rn(__dsqrt_rn(rr), b_norm);
+      finite = isfinite(error);
+      above = error > tol;
+      reduce(1, [&](int64_t row, double& d0, double&) {
+        const double zi = RowDot<kOneRound>(m_row(row), [&](int32_t c) { return r_new[c]; });
+        a.z[row] = zi;
+        d0 = Mul(r_new[row], zi);
+      }, t0, t1);
+      if (aborted) break;
+      r_z_new = t0;
+    }
+    beta = converged ? 0.0 : __ddiv_rn(r_z_new, r_z);
+    r_z = r_z_new;
+    if (writer) a.history[count] = rr;
+    ++count;
+    if (!finite) {
+      status = 3;
+      done = true;
+    } else if (!isfinite(beta)) {
+      status = 2;
+      done = true;
+    } else {
+      done = !(count < a.max_iterations && above);
     }
   }
+  // epilogue: the true residual at exit
+  if (!aborted) {
+    reduce(1, [&](int64_t row, double& d0, double&) {
+      const double ax = RowDot<kOneRound>(a_row(row), [&](int32_t c) { return a.x[c]; });
+      const double ri = __dsub_rn(a.b[row], ax);
+      d0 = Mul(ri, ri);
+    }, t0, t1);
+  }
+  if (blockIdx.x == 0) {
+    __syncthreads();
+    // the history's norms, from the squares the writer left
+    for (int64_t i = 1 + threadIdx.x; i < count - 1; i += kSolveThreads) {
+      a.history[i] = __ddiv_rn(__dsqrt_rn(a.history[i]), b_norm);
+    }
+    if (writer) {
+      const double h = __ddiv_rn(__dsqrt_rn(t0), b_norm);
+      if (count > 1) a.history[0] = 1.0;
+      a.history[count - 1] = h;
+      if (!isfinite(h)) {
+        status = 3;
+      } else if (h <= tol) {
+        status = 1;
+      }
+      a.outcome->count = count;
+      a.outcome->status = status;
+      a.outcome->aborted = aborted ? 1 : 0;
+    }
+  }
+  // No block leaves while a neighbour may still store to its shared memory.
+  // After an abort a neighbour may be one reduction ahead: its cluster
+  // barriers there are matched here, and its own exit is the last one.
+  if (aborted) {
+    for (int64_t g = 1; g < groups; ++g) cluster.sync();
+  }
+  cluster.sync();
 }
 
-// p = z + beta p, then the loop's condition for the next body execution.
-__global__ void PcgDirectionKernel(PcgState* __restrict__ s, cudaGraphConditionalHandle loop) {
-  const bool done = s->done != 0;
-  if (!done) {
-    const int64_t n = s->n;
-    const double beta = s->beta;
-    const double* __restrict__ z = s->z;
-    double* __restrict__ p = s->p;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-      p[i] = Add(z[i], Mul(beta, p[i]));
-    }
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    const int64_t bodies = s->bodies + 1;
-    s->bodies = bodies;
-    // the body count bounds the loop whatever the recurrence does
-    cudaGraphSetConditional(loop, (!done && bodies < s->body_limit) ? 1u : 0u);
-  }
+// Dynamic shared memory of a solve block: the double buffers of lane sums and terms follow SolveShared, then (one
+// round) the matrices.
+template <bool kOneRound>
+constexpr size_t SolveBytes() {
+  return sizeof(SolveShared) +
+         sizeof(double) * 2 * (kOneRound ? 1 : kGroupRounds) * 2 * (kTreeLanes + kTreeTerms * kWarp);
 }
+constexpr size_t kBlockSharedBytes = 227 * 1024;  // what a block may use on sm_100
 
-// Kernel nodes of one graph: prologue, per body execution, epilogue.
-constexpr int64_t kPrologueKernels = 3;
-constexpr int64_t kBodyKernels = 8;
-constexpr int64_t kEpilogueKernels = 2;
+// Launch attributes of a solve: clusters of eight, all blocks resident at once.
+struct SolveLaunch {
+  cudaLaunchConfig_t config = {};
+  cudaLaunchAttribute attributes[2] = {};
 
-// One instantiated solve graph with its state and scratch; used by one solve at a time.
-struct PcgGraph {
-  int device = -1;
-  int64_t n = 0;
-  bool fp32_m = false;
-  bool busy = false;
-  PcgState* state = nullptr;       // device
-  PcgState* host_state = nullptr;  // pinned
-  double* partial = nullptr;
-  unsigned int* arrive = nullptr;
-  cudaGraphExec_t exec = nullptr;
+  SolveLaunch(cudaStream_t stream, size_t smem) {
+    attributes[0].id = cudaLaunchAttributeClusterDimension;
+    attributes[0].val.clusterDim.x = kClusterBlocks;
+    attributes[0].val.clusterDim.y = 1;
+    attributes[0].val.clusterDim.z = 1;
+    attributes[1].id = cudaLaunchAttributeCooperative;
+    attributes[1].val.cooperative = 1;
+    config.attrs = attributes;
+    config.numAttrs = 2;
+    config.blockDim = dim3(kSolveThreads);
+    config.gridDim = dim3(kClusterBlocks);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+  }
 };
 
-std::mutex g_graph_mutex;
-std::vector<std::unique_ptr<PcgGraph>> g_graphs;  // kept for the process lifetime
-
-template <class TM>
-void CaptureGraph(PcgGraph& g, int sm_count) {
-  const int64_t n = g.n;
-  const int64_t chunks = CeilDiv(n, kTreeChunk);
-  const int64_t cap = static_cast<int64_t>(sm_count) * 16;
-  const int spmv_grid = static_cast<int>(std::min<int64_t>(CeilDiv(n, 128), cap));
-  const int vec_grid = static_cast<int>(std::min<int64_t>(CeilDiv(n, 256), cap));
-  const unsigned dot_grid = static_cast<unsigned>(chunks);
-  cudaStream_t main_stream = nullptr;
-  cudaStream_t body_stream = nullptr;
-  cudaGraph_t graph = nullptr;
-  SPAI_CUDA(cudaStreamCreateWithFlags(&main_stream, cudaStreamNonBlocking));
-  try {
-    SPAI_CUDA(cudaStreamCreateWithFlags(&body_stream, cudaStreamNonBlocking));
-    SPAI_CUDA(cudaStreamBeginCapture(main_stream, cudaStreamCaptureModeThreadLocal));
-    PcgState* s = g.state;
-    PcgInitKernel<<<vec_grid, 256, 0, main_stream>>>(s);
-    PcgSpmvKernel<TM, kMrInit><<<spmv_grid, 128, 0, main_stream>>>(s);
-    PcgDotKernel<kInit><<<dot_grid, kTreeLanes, 0, main_stream>>>(s);
-    SPAI_CUDA(cudaGetLastError());
-    cudaStreamCaptureStatus status;
-    cudaGraph_t capture_graph = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t num_deps = 0;
-    SPAI_CUDA(cudaStreamGetCaptureInfo(main_stream, &status, nullptr, &capture_graph, &deps, &num_deps));
-    cudaGraphConditionalHandle loop;
-    SPAI_CUDA(cudaGraphConditionalHandleCreate(&loop, capture_graph, 1, cudaGraphCondAssignDefault));
-    cudaGraphNodeParams params = {};
-    params.type = cudaGraphNodeTypeConditional;
-    params.conditional.handle = loop;
-    params.conditional.type = cudaGraphCondTypeWhile;
-    params.conditional.size = 1;
-    cudaGraphNode_t loop_node;
-    SPAI_CUDA(cudaGraphAddNode(&loop_node, capture_graph, deps, num_deps, &params));
-    SPAI_CUDA(cudaStreamUpdateCaptureDependencies(main_stream, &loop_node, 1, cudaStreamSetCaptureDependencies));
-    cudaGraph_t body = params.conditional.phGraph_out[0];
-    SPAI_CUDA(cudaStreamBeginCaptureToGraph(body_stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    PcgSpmvKernel<double, kApFromP><<<spmv_grid, 128, 0, body_stream>>>(s);
-    PcgDotKernel<kDen><<<dot_grid, kTreeLanes, 0, body_stream>>>(s);
-    PcgDotKernel<kStep><<<dot_grid, kTreeLanes, 0, body_stream>>>(s);
-    PcgSpmvKernel<double, kApFromX><<<spmv_grid, 128, 0, body_stream>>>(s);
-    PcgDotKernel<kRefresh><<<dot_grid, kTreeLanes, 0, body_stream>>>(s);
-    PcgSpmvKernel<TM, kMrLoop><<<spmv_grid, 128, 0, body_stream>>>(s);
-    PcgDotKernel<kRz><<<dot_grid, kTreeLanes, 0, body_stream>>>(s);
-    PcgDirectionKernel<<<vec_grid, 256, 0, body_stream>>>(s, loop);
-    SPAI_CUDA(cudaGetLastError());
-    cudaGraph_t body_out = nullptr;
-    SPAI_CUDA(cudaStreamEndCapture(body_stream, &body_out));
-    PcgSpmvKernel<double, kApFromXFinal><<<spmv_grid, 128, 0, main_stream>>>(s);
-    PcgDotKernel<kFinal><<<dot_grid, kTreeLanes, 0, main_stream>>>(s);
-    SPAI_CUDA(cudaGetLastError());
-    SPAI_CUDA(cudaStreamEndCapture(main_stream, &graph));
-    SPAI_CUDA(cudaGraphInstantiate(&g.exec, graph, 0));
-  } catch (...) {
-    cudaStreamCaptureStatus st;
-    for (cudaStream_t stream : {body_stream, main_stream}) {
-      if (stream != nullptr && cudaStreamIsCapturing(stream, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone) {
-        cudaGraph_t dropped = nullptr;
-        cudaStreamEndCapture(stream, &dropped);
-        if (dropped != nullptr && stream == main_stream) cudaGraphDestroy(dropped);
-      }
-    }
-    if (graph != nullptr) cudaGraphDestroy(graph);
-    if (body_stream != nullptr) cudaStreamDestroy(body_stream);
-    cudaStreamDestroy(main_stream);
-    cudaGetLastError();
-    throw;
-  }
-  cudaGraphDestroy(graph);
-  cudaStreamDestroy(body_stream);
-  cudaStreamDestroy(main_stream);
+template <bool kOneRound>
+constexpr size_t LaunchBytes() {
+  return kOneRound ? kBlockSharedBytes : SolveBytes<false>();
 }
 
-// A free graph for (device, n, precision of M), built on first use.
-template <class TM>
-PcgGraph* AcquireGraph(int device, int64_t n, int sm_count) {
-  const bool fp32 = sizeof(TM) == sizeof(float);
-  {
-    std::lock_guard<std::mutex> lock(g_graph_mutex);
-    for (auto& g : g_graphs) {
-      if (!g->busy && g->device == device && g->n == n && g->fp32_m == fp32) {
-        g->busy = true;
-        return g.get();
-      }
-    }
-  }
-  auto g = std::make_unique<PcgGraph>();
-  g->device = device;
-  g->n = n;
-  g->fp32_m = fp32;
-  g->busy = true;
-  try {
-    SPAI_CUDA(cudaMalloc(reinterpret_cast<void**>(&g->state), sizeof(PcgState)));
-    SPAI_CUDA(cudaMallocHost(reinterpret_cast<void**>(&g->host_state), sizeof(PcgState)));
-    SPAI_CUDA(cudaMalloc(reinterpret_cast<void**>(&g->partial), sizeof(double) * 2 * CeilDiv(n, kTreeChunk)));
-    SPAI_CUDA(cudaMalloc(reinterpret_cast<void**>(&g->arrive), sizeof(unsigned int)));
-    SPAI_CUDA(cudaMemset(g->arrive, 0, sizeof(unsigned int)));
-    CaptureGraph<TM>(*g, sm_count);
-  } catch (...) {
-    if (g->exec != nullptr) cudaGraphExecDestroy(g->exec);
-    if (g->state != nullptr) cudaFree(g->state);
-    if (g->host_state != nullptr) cudaFreeHost(g->host_state);
-    if (g->partial != nullptr) cudaFree(g->partial);
-    if (g->arrive != nullptr) cudaFree(g->arrive);
-    throw;
-  }
-  std::lock_guard<std::mutex> lock(g_graph_mutex);
-  g_graphs.push_back(std::move(g));
-  return g_graphs.back().get();
-}
-
-void ReleaseGraph(PcgGraph* g) {
-  std::lock_guard<std::mutex> lock(g_graph_mutex);
-  g->busy = false;
+// Clusters of the solve kernel that fit on the current device at once (asked once per device).
+template <class TM, bool kOneRound>
+int64_t ResidentClusters(int device) {
+  static std::mutex mutex;
+  static std::map<int, int> known;
+  std::lock_guard<std::mutex> lock(mutex);
+  const auto it = known.find(device);
+  if (it != known.end()) return it->second;
+  const auto kernel = PcgSolveKernel<TM, kOneRound>;
+  SPAI_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(LaunchBytes<kOneRound>())));
+  SolveLaunch launch(nullptr, LaunchBytes<kOneRound>());
+  launch.config.numAttrs = 1;  // the cluster shape alone decides residency
+  int clusters = 0;
+  SPAI_CUDA(cudaOccupancyMaxActiveClusters(&clusters, kernel, &launch.config));
+  if (clusters < 1) throw CudaError("PCG: no cluster of the solve kernel fits on the device");
+  known[device] = clusters;
+  return clusters;
 }
 
 // One thread per row, entries in storage order (the reference's _row_dot).
@@ -463,62 +803,100 @@ void RunPcg(Ctx& ctx, const DevCsc<double>& a, const DevCsc<TM>& m, const double
   if (n <= 0) throw std::invalid_argument("PCG needs n > 0");
   if (n > kTreeChunk * kTreeChunk) throw std::invalid_argument("PCG supports at most 4096^2 rows");
   if (opt.max_iterations <= 0) throw std::invalid_argument("max_iterations must be positive");
-  DevBuf<double> r, z, p, ap, history;
-  r.Reserve(static_cast<size_t>(n), ctx.stream);
-  z.Reserve(static_cast<size_t>(n), ctx.stream);
-  p.Reserve(static_cast<size_t>(n), ctx.stream);
-  ap.Reserve(static_cast<size_t>(n), ctx.stream);
-  history.Reserve(static_cast<size_t>(opt.max_iterations), ctx.stream);
-  PcgGraph* g = AcquireGraph<TM>(ctx.device, n, ctx.sm_count);
-  try {
-    PcgState& h = *g->host_state;
-    h = PcgState{};
-    h.a_ptr = a.ptr.data();
-    h.a_idx = a.idx.data();
-    h.a_val = a.val.data();
-    h.m_ptr = m.ptr.data();
-    h.m_idx = m.idx.data();
-    h.m_val = m.val.data();
-    h.b = b;
-    h.x = x;
-    h.r = r.data();
-    h.z = z.data();
-    h.p = p.data();
-    h.ap = ap.data();
-    h.history = history.data();
-    h.partial = g->partial;
-    h.arrive = g->arrive;
-    h.n = n;
-    h.chunks = CeilDiv(n, kTreeChunk);
-    h.max_iterations = opt.max_iterations;
-    h.refresh_period = opt.refresh_period;
-    h.tolerance = opt.tolerance;
-    h.body_limit = opt.max_iterations + 2;
-    SPAI_CUDA(cudaMemcpyAsync(g->state, g->host_state, sizeof(PcgState), cudaMemcpyHostToDevice, ctx.stream));
-    {
-      prof::Scope scope(ctx.stream, "pcg_solve", 0.0);
-      SPAI_CUDA(cudaGraphLaunch(g->exec, ctx.stream));
-    }
-    SPAI_CUDA(cudaMemcpyAsync(g->host_state, g->state, sizeof(PcgState), cudaMemcpyDeviceToHost, ctx.stream));
-    result.history.assign(static_cast<size_t>(opt.max_iterations), 0.0);
-    SPAI_CUDA(cudaMemcpyAsync(result.history.data(), history.data(), sizeof(double) * opt.max_iterations,
-                              cudaMemcpyDeviceToHost, ctx.stream));
-    ctx.Sync();
-    const int64_t count = h.count;
-    if (count < 1 || count > opt.max_iterations) throw CudaError("PCG graph returned an invalid iteration count");
-    result.history.resize(static_cast<size_t>(count));
-    result.status = h.status;
-    result.spmv_count = 2 + 3 * (count - 1);
-    // algorithmic bytes of the solve: per iteration A and M once plus the vector traffic (17 n doubles)
-    const double per_iteration = static_cast<double>(a.nnz) * 12.0 + static_cast<double>(m.nnz) * (sizeof(TM) + 4) +
-                                 8.0 * 17.0 * static_cast<double>(n);
-    prof::AddBytes("pcg_solve", per_iteration * static_cast<double>(count));
-    CountLaunches(kPrologueKernels + kBodyKernels * h.bodies + kEpilogueKernels);
-  } catch (...) {
-    ReleaseGraph(g);
-    throw;
+  const int64_t chunks = CeilDiv(n, kTreeChunk);
+  const int64_t slices = CeilDiv(n, kWarp);
+  const cudaStream_t st = ctx.stream;
+  // r, p (two of each), z, ap, the history and the chunk sums
+  DevBuf<double> vectors, history;
+  DevBuf<TaggedSum> partial;
+  vectors.Reserve(static_cast<size_t>(6 * n), st);
+  history.Reserve(static_cast<size_t>(opt.max_iterations), st);
+  partial.Reserve(static_cast<size_t>(4 * chunks), st);
+  // the sliced copies (at most twice the entries plus two per row, see SliceRows) and their slice offsets
+  const size_t a_room = static_cast<size_t>(2 * a.nnz + 2 * (n + kWarp));
+  const size_t m_room = static_cast<size_t>(2 * m.nnz + 2 * (n + kWarp));
+  DevBuf<int64_t> slice_at;
+  DevBuf<int32_t> a_idx, m_idx;
+  DevBuf<double> a_val;
+  DevBuf<TM> m_val;
+  slice_at.Reserve(static_cast<size_t>(2 * slices), st);
+  a_idx.Reserve(a_room, st);
+  a_val.Reserve(a_room, st);
+  m_idx.Reserve(m_room, st);
+  m_val.Reserve(m_room, st);
+  // two slice cursors and the outcome, zeroed
+  struct Control {
+    unsigned long long used[2];
+    SolveOutcome outcome;
+  };
+  DevBuf<Control> control;
+  control.Reserve(1, st);
+  SPAI_CUDA(cudaMemsetAsync(control.data(), 0, sizeof(Control), st));
+  SPAI_CUDA(cudaMemsetAsync(partial.data(), 0, sizeof(TaggedSum) * static_cast<size_t>(4 * chunks), st));
+  Control* c = control.data();
+  SolveArgs<TM> args{};
+  args.a = SolveMatrix<double>{a.ptr.data(), a.idx.data(), a.val.data(), slice_at.data(), a_idx.data(), a_val.data(),
+                               &c->used[0]};
+  args.m = SolveMatrix<TM>{m.ptr.data(), m.idx.data(), m.val.data(), slice_at.data() + slices, m_idx.data(),
+                           m_val.data(), &c->used[1]};
+  args.b = b;
+  args.x = x;
+  double* v = vectors.data();
+  args.r[0] = v;
+  args.r[1] = v + n;
+  args.p[0] = v + 2 * n;
+  args.p[1] = v + 3 * n;
+  args.z = v + 4 * n;
+  args.ap = v + 5 * n;
+  args.history = history.data();
+  args.partial = partial.data();
+  args.outcome = &c->outcome;
+  args.n = n;
+  args.chunks = chunks;
+  args.max_iterations = opt.max_iterations;
+  args.refresh_period = opt.refresh_period;
+  args.tolerance = opt.tolerance;
+  // one chunk per cluster while the clusters that fit at once cover every chunk
+  auto kernel = PcgSolveKernel<TM, true>;
+  size_t smem = LaunchBytes<true>();
+  int64_t clusters = ResidentClusters<TM, true>(ctx.device);
+  if (clusters < chunks) {
+    kernel = PcgSolveKernel<TM, false>;
+    smem = LaunchBytes<false>();
+    clusters = ResidentClusters<TM, false>(ctx.device);
   }
-  ReleaseGraph(g);
+  args.room = static_cast<int>(kBlockSharedBytes - SolveBytes<true>());
+  clusters = std::min(clusters, chunks);
+  DevBuf<unsigned long long> arrived;
+  const size_t flags = static_cast<size_t>(clusters * kFlagStride);
+  arrived.Reserve(flags, st);
+  SPAI_CUDA(cudaMemsetAsync(arrived.data(), 0, sizeof(unsigned long long) * flags, st));
+  args.arrived = arrived.data();
+  {
+    prof::Scope scope(st, "pcg_solve", 0.0);
+    SolveLaunch launch(st, smem);
+    launch.config.gridDim = dim3(static_cast<unsigned>(clusters * kClusterBlocks));
+    SPAI_CUDA(cudaLaunchKernelEx(&launch.config, kernel, args));
+    SPAI_LAUNCH_CHECK();
+  }
+  static_assert(sizeof(SolveOutcome) <= 8 * sizeof(int64_t), "the outcome fits the pinned counts");
+  SPAI_CUDA(cudaMemcpyAsync(ctx.host_counts, args.outcome, sizeof(SolveOutcome), cudaMemcpyDeviceToHost, st));
+  result.history.assign(static_cast<size_t>(opt.max_iterations), 0.0);
+  SPAI_CUDA(cudaMemcpyAsync(result.history.data(), history.data(), sizeof(double) * opt.max_iterations,
+                            cudaMemcpyDeviceToHost, st));
+  ctx.Sync();
+  SolveOutcome outcome;
+  std::memcpy(&outcome, ctx.host_counts, sizeof(outcome));
+  if (outcome.aborted != 0) throw CudaError("PCG: the blocks of the solve stopped answering one another");
+  const int64_t count = outcome.count;
+  if (count < 1 || count > opt.max_iterations) throw CudaError("PCG returned an invalid iteration count");
+  result.history.resize(static_cast<size_t>(count));
+  result.status = outcome.status;
+  result.spmv_count = 2 + 3 * (count - 1);
+  // algorithmic bytes of the solve: per iteration A and M once plus the vector traffic (17 n doubles)
+  const double per_iteration = static_cast<double>(a.nnz) * 12.0 + static_cast<double>(m.nnz) * (sizeof(TM) + 4) +
+                               8.0 * 17.0 * static_cast<double>(n);
+  prof::AddBytes("pcg_solve", per_iteration * static_cast<double>(count));
 }
 
 template void RunPcg<double>(Ctx&, const DevCsc<double>&, const DevCsc<double>&, const double*, double*,
