@@ -20,6 +20,7 @@
 #include <stdexcept>
 #include <vector>
 
+#include "colgroup.cuh"
 #include "colkit.cuh"
 #include "device.cuh"
 #include "mr_fused.cuh"
@@ -34,14 +35,14 @@ void CountLaunches(int64_t count);
 
 namespace {
 
-constexpr int kDropWarps = 4;       // warps per block of the drop kernel
-constexpr int kDropWindowWords = 512;  // bitmap words of the drop kernel: windows of 16,384 rows
+constexpr int kGroupWarps = 2;      // warps per block of the drop and residual kernels
+constexpr int kDropWindowWords = 512;  // bitmap words of a drop column on its own: windows of 16,384 rows
 constexpr int kDropWindowRows = kDropWindowWords * 32;
-constexpr int kResidualWarps = 4;   // warps per block of the residual kernel
-constexpr int kWindowWords = 1024;  // bitmap words of the residual kernel: windows of 32,768 rows
+constexpr int kWindowWords = 1024;  // bitmap words of a residual column on its own: windows of 32,768 rows
 constexpr int kWindowRows = kWindowWords * 32;
 constexpr int kRowsCap = 1024;      // longest row list of one product column
 constexpr int kMaxTopK = 32;
+constexpr int kMaxGroupWords = 2048;  // windows of column groups: up to 65,536 rows (16-bit offsets)
 constexpr int kDropRowsCap = 512;  // candidate rows of one drop column; also bounds Z's slots per column
 
 // Overflow bits (FusedState::overflow).
@@ -91,6 +92,10 @@ struct FusedArgs {
   int z_hash_slots;   // residual kernel: Z(:, j)
   int d_mt_slots;     // drop kernel: M(j, :)
   int d_r_slots;      // drop kernel: R(j, :)
+  int words;           // 32-row words of the column groups' windows (0: every column on its own)
+  int64_t bandwidth;   // largest |i - k| over the entries of A
+  size_t drop_bytes;      // shared memory of a warp
+  size_t residual_bytes;
   int64_t max_iterations;
   double tolerance;
   const int32_t* a_cols_ell;
@@ -176,18 +181,156 @@ __host__ __device__ size_t DropWarpBytes(int own, int mt, int r) {
          Round16(static_cast<size_t>(kDropRowsCap) * 2) +
          Round16(static_cast<size_t>(mt + r) * 4) + Round16(static_cast<size_t>(mt + r) * sizeof(T)) +
          Round16(static_cast<size_t>(own) * 4) + Round16(static_cast<size_t>(own) * sizeof(T)) +
-         Round16(kDropCap * sizeof(double)) + Round16(kDropCap * sizeof(int32_t)) + Round16(kDropCap) +
-         Round16(4 * kWarp * sizeof(int32_t));
+         Round16(kDropCap * sizeof(T)) + Round16(kDropCap * sizeof(int32_t));
 }
 
+// The drop decision of one column and its survivors: DecideDrops' rules
+// (select.cuh) on `count` nonzero values vals[r] of rows row_of(r), NB
+// entries per lane.  The relative threshold needs the sequential sum of
+// squares only when the smallest magnitude could lie below it; the cut of the
+// top-k is found by bisection on the magnitudes' bits, ties going to the
+// larger row.
+template <class T, int NB, class Row>
+__device__ __forceinline__ int DropAndWriteIn(const FusedArgs<T>& a, Row row_of, const T* vals, int count, int64_t j,
+                                              int64_t other, int lane, int* overflow) {
+  using Key = typename MagnitudeOf<T>::Key;
+  T val[NB];
+  Key key[NB];  // 0: dropped or absent
+  int32_t row[NB];
+  unsigned diagonal = 0u;
+  Key largest = 0;
+  Key smallest = ~Key(0);
+#pragma unroll
+  for (int t = 0; t < NB; ++t) {
+    const int r = t * kWarp + lane;
+    val[t] = r < count ? vals[r] : T(0);
+    row[t] = r < count ? row_of(r) : -1;
+    key[t] = MagnitudeBits(val[t]);
+    if (key[t] != 0) {
+      largest = key[t] > largest ? key[t] : largest;
+      smallest = key[t] < smallest ? key[t] : smallest;
+    }
+    if (static_cast<int64_t>(row[t]) == j) diagonal |= 1u << t;
+  }
+  // thr = eps sqrt(sum v^2) <= eps sqrt(256) max|v| (1 + rounding): below 17 eps max|v|
+  const Key top = LargestKey(largest);
+  const Key bottom = SmallestKey(smallest);
+  const double hi = MagnitudeValue(top);
+  const double lo = MagnitudeValue(bottom);
+  int kept = count;
+  if (!(hi < 1e150 && lo > 17.0 * kDblEps * hi)) {
+    double thr = 0.0;
+    if (lane == 0) {
+      double sq = 0.0;
+#pragma unroll 1
+      for (int r = 0; r < count; ++r) {
+        const double v = static_cast<double>(vals[r]);
+        sq = Add(sq, Mul(v, v));
+      }
+      thr = Mul(kDblEps, sqrt(sq));
+    }
+    thr = __shfl_sync(0xffffffffu, thr, 0);
+    kept = 0;
+#pragma unroll
+    for (int t = 0; t < NB; ++t) {
+      const bool keep = ((diagonal >> t) & 1u) != 0u || fabs(static_cast<double>(val[t])) >= thr;
+      if (!keep) key[t] = 0;
+      kept += __popc(__ballot_sync(0xffffffffu, key[t] != 0));
+    }
+  }
+  if (kept > a.topk) {
+    // the diagonal stays; of the other candidates the `wanted` largest (|v|, row)
+    const bool has_diagonal = __any_sync(0xffffffffu, diagonal != 0u);
+    const int wanted = a.topk - (has_diagonal ? 1 : 0);
+    Key cand[NB];
+#pragma unroll
+    for (int t = 0; t < NB; ++t) cand[t] = ((diagonal >> t) & 1u) != 0u ? Key(0) : key[t];
+    Key below = bottom;   // at least `wanted` candidates are >= below
+    Key above = top + 1;  // fewer than `wanted` are >= above
+    int at_above = 0;
+    if (wanted <= 0) below = ~Key(0);
+#pragma unroll 1
+    while (wanted > 0) {
+      const Key mid = below + ((above - below) >> 1);
+      int n = 0;
+#pragma unroll
+      for (int t = 0; t < NB; ++t) n += __popc(__ballot_sync(0xffffffffu, cand[t] >= mid));
+      if (n == wanted) {
+        below = mid;
+        break;
+      }
+      if (n > wanted) {
+        below = mid;
+      } else {
+        above = mid;
+        at_above = n;
+      }
+      if (above - below <= 1) {
+        // several candidates share the cut's magnitude: the larger rows win
+        int need = wanted - at_above;
+#pragma unroll
+        for (int t = NB - 1; t >= 0; --t) {
+          unsigned equal = __ballot_sync(0xffffffffu, cand[t] == below);
+#pragma unroll 1
+          for (int surplus = __popc(equal) - need; surplus > 0; --surplus) {
+            if (lane == __ffs(equal) - 1) cand[t] = 0;
+            equal &= equal - 1u;
+          }
+          need -= __popc(equal);
+        }
+        break;
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < NB; ++t) {
+      const bool keep = ((diagonal >> t) & 1u) != 0u || (cand[t] != 0 && cand[t] >= below);
+      if (!keep) key[t] = 0;
+    }
+  }
+  int32_t* out_rows = a.m_rows + j * a.topk;
+  T* out_vals = a.m_vals + j * a.topk;
+  int at = 0;
+#pragma unroll
+  for (int t = 0; t < NB; ++t) {
+    const bool mine = key[t] != 0;
+    const unsigned mask = __ballot_sync(0xffffffffu, mine);
+    if (mine) {
+      const int o = at + __popc(mask & LaneMaskBelow());
+      out_rows[o] = row[t];
+      out_vals[o] = val[t];
+      const int slot = atomicAdd(&a.mt_cnt[other][row[t]], 1);
+      if (slot < a.cap_mt) {
+        a.mt_cols[other][static_cast<int64_t>(row[t]) * a.cap_mt + slot] = static_cast<int32_t>(j);
+        a.mt_vals[other][static_cast<int64_t>(row[t]) * a.cap_mt + slot] = val[t];
+      } else {
+        *overflow |= kOverflowMt;
+      }
+    }
+    at += __popc(mask);
+  }
+  if (lane == 0) a.m_cnt[j] = at;
+  return at;
+}
+
+// The same for any count <= kDropCap.
+template <class T, class Row>
+__device__ __forceinline__ int DropAndWrite(const FusedArgs<T>& a, Row row_of, const T* vals, int count, int64_t j,
+                                            int64_t other, int lane, int* overflow) {
+  static_assert(kDropCap == 8 * kWarp, "eight entries per lane hold the longest column");
+  if (count <= 2 * kWarp) return DropAndWriteIn<T, 2>(a, row_of, vals, count, j, other, lane, overflow);
+  if (count <= 4 * kWarp) return DropAndWriteIn<T, 4>(a, row_of, vals, count, j, other, lane, overflow);
+  return DropAndWriteIn<T, 8>(a, row_of, vals, count, j, other, lane, overflow);
+}
+
+// One column on its own, for columns whose rows do not fit the group's window.
+// Returns the overflow bits; *written grows by the column's entries.
 template <class T>
-__global__ void __launch_bounds__(kDropWarps * kWarp) FusedDropKernel(FusedArgs<T> a) {
-  extern __shared__ __align__(16) unsigned char fused_drop_smem[];
+__device__ __noinline__ int DropColumn(const FusedArgs<T>& a, unsigned char* base, int64_t j,
+                                       unsigned long long* written_out) {
   constexpr int kSummary = (kDropWindowWords + kWarp * kWarp - 1) / (kWarp * kWarp) * kWarp;
   const int lane = threadIdx.x & 31;
   const int table = a.d_mt_slots + a.d_r_slots;
   const int own = a.topk + a.cap_z;  // M(:, j) and Z(:, j), staged
-  unsigned char* base = fused_drop_smem + (threadIdx.x >> 5) * DropWarpBytes<T>(own, a.d_mt_slots, a.d_r_slots);
   uint32_t* bm = reinterpret_cast<uint32_t*>(base);
   base += Round16(static_cast<size_t>(kDropWindowWords) * 4);
   uint32_t* summary = reinterpret_cast<uint32_t*>(base);
@@ -204,16 +347,9 @@ __global__ void __launch_bounds__(kDropWarps * kWarp) FusedDropKernel(FusedArgs<
   T* mv = reinterpret_cast<T*>(base);  // and values
   T* zv = mv + a.topk;
   base += Round16(static_cast<size_t>(own) * sizeof(T));
-  DropSlab s;
-  s.vals = reinterpret_cast<double*>(base);
-  base += Round16(kDropCap * sizeof(double));
-  s.keys = reinterpret_cast<int32_t*>(base);
-  base += Round16(kDropCap * sizeof(int32_t));
-  s.keep = base;
-  base += Round16(kDropCap);
-  s.xk = reinterpret_cast<int32_t*>(base);  // staging of the top-k selection
-  s.yk = s.xk;
-  s.mx_prefix = nullptr;
+  T* s_vals = reinterpret_cast<T*>(base);  // the nonzero entries of S(:, j)
+  base += Round16(kDropCap * sizeof(T));
+  int32_t* s_rows = reinterpret_cast<int32_t*>(base);
   int32_t* k_mt = keys;
   int32_t* k_r = k_mt + a.d_mt_slots;
   T* v_mt = vals;
@@ -227,24 +363,23 @@ __global__ void __launch_bounds__(kDropWarps * kWarp) FusedDropKernel(FusedArgs<
   const int64_t parity = state->parity;
   const int64_t other = parity ^ 1;
   const T alpha = static_cast<T>(state->alpha);
-  const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-  unsigned long long written = 0;
   int overflow = 0;
-  for (int64_t j = warp; j < a.n; j += warps) {
+  __syncwarp();
+  {
     const int nm = a.m_cnt[j];
     const int nz = a.z_cnt[j];
     const int nmt = a.mt_cnt[parity][j];
     if (nmt > a.cap_mt) {
-      overflow |= kOverflowMt;
-      continue;
+      return kOverflowMt;
     }
     ClearTable(keys, table, lane);
     // M(:, j) and Z(:, j) into shared memory (sorted by row), then M(j, :) into its hash
+#pragma unroll 1
     for (int e = lane; e < nm; e += kWarp) {
       mr[e] = a.m_rows[j * a.topk + e];
       mv[e] = a.m_vals[j * a.topk + e];
     }
+#pragma unroll 1
     for (int e = lane; e < nz; e += kWarp) {
       zr[e] = a.z_rows[j * a.cap_z + e];
       zv[e] = a.z_vals[j * a.cap_z + e];
@@ -264,6 +399,7 @@ __global__ void __launch_bounds__(kDropWarps * kWarp) FusedDropKernel(FusedArgs<
       lo = min(lo, zr[0]);
       hi = max(hi, zr[nz - 1]);
     }
+#pragma unroll 1
     for (int e = lane; e < nmt; e += kWarp) {
       const int at = FindOrInsert(k_mt, b_mt, mtc[e], &fresh);
       v_mt[at] = mtv[e];
@@ -306,6 +442,7 @@ __global__ void __launch_bounds__(kDropWarps * kWarp) FusedDropKernel(FusedArgs<
       }
     };
     load_row(0, cur_i, cur_v);
+#pragma unroll 1
     for (int u = 0; u < a.ell && !r_full; ++u) {
       const int32_t k = __shfl_sync(0xffffffffu, k_lane, u);
       const int nk = __shfl_sync(0xffffffffu, nk_lane, u);
@@ -345,24 +482,27 @@ __global__ void __launch_bounds__(kDropWarps * kWarp) FusedDropKernel(FusedArgs<
       }
     }
     if (r_full) {
-      overflow |= kOverflowRow;
-      continue;
+      return kOverflowRow;
     }
     lo = __reduce_min_sync(0xffffffffu, lo);
     hi = __reduce_max_sync(0xffffffffu, hi);
     // S(:, j) in row order, one window of kDropWindowRows rows at a time
     int count = 0;
     bool too_long = false;
+#pragma unroll 1
     for (int32_t seg_lo = lo; seg_lo <= hi; seg_lo += kDropWindowRows) {
       const int32_t seg_hi = hi - seg_lo < kDropWindowRows ? hi : seg_lo + (kDropWindowRows - 1);
       const int words = (seg_hi - seg_lo) / 32 + 1;
       if (lane == 0 && j >= seg_lo && j <= seg_hi) MarkRow(bm, summary, static_cast<int>(j - seg_lo));
+#pragma unroll 1
       for (int e = lane; e < nm; e += kWarp) {
         if (mr[e] >= seg_lo && mr[e] <= seg_hi) MarkRow(bm, summary, mr[e] - seg_lo);
       }
+#pragma unroll 1
       for (int e = lane; e < nz; e += kWarp) {
         if (zr[e] >= seg_lo && zr[e] <= seg_hi) MarkRow(bm, summary, zr[e] - seg_lo);
       }
+#pragma unroll 1
       for (int t = lane; t < table; t += kWarp) {
         const int32_t key = keys[t];
         if (key != kEmpty && key >= seg_lo && key <= seg_hi) MarkRow(bm, summary, key - seg_lo);
@@ -373,6 +513,7 @@ __global__ void __launch_bounds__(kDropWarps * kWarp) FusedDropKernel(FusedArgs<
         too_long = true;
         break;
       }
+#pragma unroll 1
       for (int r0 = 0; r0 < found; r0 += kWarp) {
         const int r = r0 + lane;
         bool emit = false;
@@ -424,13 +565,13 @@ __global__ void __launch_bounds__(kDropWarps * kWarp) FusedDropKernel(FusedArgs<
           } else if (trans) {
             v = Mul(T(0.5), Add(T(0), u_tr));
           }
-          emit = own || trans;
+          emit = !(v == T(0));  // exact zeros are dropped
         }
         const unsigned mask = __ballot_sync(0xffffffffu, emit);
         if (emit) {
           const int o = count + __popc(mask & LaneMaskBelow());
-          s.keys[o] = i;
-          s.vals[o] = static_cast<double>(v);
+          s_rows[o] = i;
+          s_vals[o] = v;
         }
         count += __popc(mask);
       }
@@ -438,49 +579,358 @@ __global__ void __launch_bounds__(kDropWarps * kWarp) FusedDropKernel(FusedArgs<
     }
     if (too_long) {
       // leave the bitmap clear for the next column before skipping this one
+#pragma unroll 1
       for (int32_t seg_lo = lo; seg_lo <= hi; seg_lo += kDropWindowRows) {
         const int32_t seg_hi = hi - seg_lo < kDropWindowRows ? hi : seg_lo + (kDropWindowRows - 1);
         ClearWords(bm, (seg_hi - seg_lo) / 32 + 1, lane);
         ClearWords(summary, SummaryWords((seg_hi - seg_lo) / 32 + 1), lane);
       }
       __syncwarp();
-      overflow |= kOverflowSide;
-      continue;
+      return kOverflowSide;
     }
     __syncwarp();
-    const int kept = DecideDrops(s, count, j, a.topk, lane);
-    // survivors: M(:, j) in place, and M^T into the other set
-    int32_t* out_rows = a.m_rows + j * a.topk;
-    T* out_vals = a.m_vals + j * a.topk;
-    int at = 0;
-    for (int b0 = 0; b0 < count; b0 += kWarp) {
-      const int i = b0 + lane;
-      const bool keep = i < count && s.keep[i] != 0;
-      const unsigned mask = __ballot_sync(0xffffffffu, keep);
-      if (keep) {
-        const int o = at + __popc(mask & LaneMaskBelow());
-        const int32_t row = s.keys[i];
-        const T v = static_cast<T>(s.vals[i]);
-        out_rows[o] = row;
-        out_vals[o] = v;
-        const int slot = atomicAdd(&a.mt_cnt[other][row], 1);
-        if (slot < a.cap_mt) {
-          a.mt_cols[other][static_cast<int64_t>(row) * a.cap_mt + slot] = static_cast<int32_t>(j);
-          a.mt_vals[other][static_cast<int64_t>(row) * a.cap_mt + slot] = v;
-        } else {
-          overflow |= kOverflowMt;
-        }
+    const int kept = DropAndWrite<T>(a, [&](int r) { return s_rows[r]; }, s_vals, count, j, other, lane, &overflow);
+    *written_out += static_cast<unsigned long long>(kept);
+    __syncwarp();
+  }
+  return overflow;
+}
+
+// ---------------------------------------------------------------------------
+// The drop step of C adjacent columns (colgroup.cuh).  With absent entries
+// held as 0 every case of the union and of the half sum is one expression:
+//   U(i, j) = M(i, j) + alpha Z(i, j), U(j, i) = M(j, i) + alpha pr_j R(j, i),
+//   S(i, j) = 0.5 (U(i, j) + U(j, i)),
+// because x + 0 is x and an entry that is zero on both sides is dropped.
+// 32 / C lanes walk the entries of one column; its terms of row j of R arrive
+// in ascending k, one row of M^T after another.
+
+constexpr int kGroupDropRows = 256;  // candidate rows of a group (ranks fit the window's byte prefixes)
+
+template <class T, int C>
+__host__ __device__ size_t DropGroupBytes(int words) {
+  return WindowBytes(words) + Round16(static_cast<size_t>(kGroupDropRows) * 2) +
+         2 * static_cast<size_t>(kGroupDropRows) * sizeof(GroupValues<T, C>);
+}
+
+// Entries s, s + kLanes, ... of a slot list: the first kHeld of them in
+// registers (rows loaded once, values when asked for), the rest read where
+// they are used.  (The group kernels' loops are otherwise kept rolled:
+// unrolled throughout, the drop kernel's code outgrew the instruction caches
+// and it ran 1.5 times as long.)
+template <class T, int kLanes, int kHeld>
+struct HeldSlots {
+  const int32_t* rows;
+  const T* vals;
+  int n;
+  int s;
+  int32_t row[kHeld];
+  T val[kHeld];
+
+  __device__ __forceinline__ HeldSlots(const int32_t* r, const T* v, int count, int lane_in_column)
+      : rows(r), vals(v), n(count), s(lane_in_column) {
+#pragma unroll
+    for (int h = 0; h < kHeld; ++h) row[h] = s + h * kLanes < n ? rows[s + h * kLanes] : -1;
+  }
+  __device__ __forceinline__ void LoadValues() {
+#pragma unroll
+    for (int h = 0; h < kHeld; ++h) val[h] = row[h] >= 0 ? vals[s + h * kLanes] : T(0);
+  }
+  template <class F>
+  __device__ __forceinline__ void Rows(F f) const {
+#pragma unroll
+    for (int h = 0; h < kHeld; ++h) {
+      if (row[h] >= 0) f(row[h]);
+    }
+#pragma unroll 1
+    for (int e = s + kHeld * kLanes; e < n; e += kLanes) f(rows[e]);
+  }
+  template <class F>
+  __device__ __forceinline__ void Entries(F f) const {
+#pragma unroll
+    for (int h = 0; h < kHeld; ++h) {
+      if (row[h] >= 0) f(row[h], val[h]);
+    }
+#pragma unroll 1
+    for (int e = s + kHeld * kLanes; e < n; e += kLanes) f(rows[e], vals[e]);
+  }
+};
+
+// False when the group does not fit (nothing written): its columns go one by one.
+template <class T, int kEll, int C>
+__device__ __forceinline__ bool DropGroup(const FusedArgs<T>& a, unsigned char* base, int64_t j0, T alpha,
+                                          int64_t parity, int lane, unsigned long long* written, int* overflow) {
+  constexpr int kLanes = kWarp / C;  // lanes of one column
+  RowWindow w = WindowAt(base, a.words, static_cast<int32_t>(j0) - a.words * 16);
+  uint16_t* rows = reinterpret_cast<uint16_t*>(base);
+  base += Round16(static_cast<size_t>(kGroupDropRows) * 2);
+  using Values = GroupValues<T, C>;
+  Values* own = reinterpret_cast<Values*>(base);
+  Values* trans = own + kGroupDropRows;
+  uint16_t* list = reinterpret_cast<uint16_t*>(own);  // free until the ranks are known
+  const int c = lane / kLanes;
+  const int s = lane % kLanes;
+  const int home = lane - s;  // first lane of the column
+  const int64_t j = j0 + c;
+  const bool valid = j < a.n;
+  const int nm = valid ? a.m_cnt[j] : 0;
+  const int nz = valid ? a.z_cnt[j] : 0;
+  const int nmt = valid ? a.mt_cnt[parity][j] : 0;
+  const int32_t* m_rows = a.m_rows + j * a.topk;
+  const int32_t* z_rows = a.z_rows + j * a.cap_z;
+  const int32_t* mt_all = a.mt_cols[parity];
+  const T* mt_vals = a.mt_vals[parity];
+  bool lost = nmt > a.cap_mt;
+  // lane s of the column holds entries s, s + kLanes, ... of row j of A and the lengths of those rows of M^T
+  constexpr int kHeld = (kEll + kLanes - 1) / kLanes;
+  int32_t k_held[kHeld];
+  int n_held[kHeld];
+  T a_held[kHeld];
+#pragma unroll
+  for (int h = 0; h < kHeld; ++h) {
+    const int u = h * kLanes + s;
+    k_held[h] = valid && u < kEll ? a.a_rows_ell[j * kEll + u] : -1;
+    a_held[h] = k_held[h] >= 0 ? a.a_rows_ell_val[j * kEll + u] : T(0);
+    n_held[h] = k_held[h] >= 0 ? a.mt_cnt[parity][k_held[h]] : 0;
+    lost = lost || n_held[h] > a.cap_mt;
+  }
+  if (__any_sync(0xffffffffu, lost)) {
+    *overflow |= kOverflowMt;
+    return true;  // the whole solve is redone on the unfused kernels
+  }
+  HeldSlots<T, kLanes, kMaxTopK / kLanes> m_list(m_rows, a.m_vals + j * a.topk, nm, s);
+  HeldSlots<T, kLanes, 64 / kLanes> z_list(z_rows, a.z_vals + j * a.cap_z, nz, s);
+  HeldSlots<T, kLanes, 32 / kLanes> mt_list(mt_all + j * a.cap_mt, mt_vals + j * a.cap_mt, nmt, s);
+  // the first entries of the rows k of M, k in row j of A (rows of M^T), for operators of up to eight
+  // entries a row; the others are read where they are used
+  constexpr bool kRowsHeld = kEll <= 8;
+  constexpr int kPer = kRowsHeld ? 24 / kLanes + (24 % kLanes != 0 ? 1 : 0) : 1;  // at least 24 entries of each
+  constexpr int kRows = kRowsHeld ? kEll : 1;
+  int32_t r_row[kRows][kPer];
+  T r_val[kRows][kPer];
+  const auto row_of_mt = [&](int u, int32_t* k, int* nk, T* a_jk) {
+    const int h = u / kLanes;
+    int32_t kh = k_held[0];
+    int nh = n_held[0];
+    T ah = a_held[0];
+#pragma unroll
+    for (int q = 1; q < kHeld; ++q) {
+      kh = h == q ? k_held[q] : kh;
+      nh = h == q ? n_held[q] : nh;
+      ah = h == q ? a_held[q] : ah;
+    }
+    *k = __shfl_sync(0xffffffffu, kh, home + u % kLanes);
+    *nk = __shfl_sync(0xffffffffu, nh, home + u % kLanes);
+    *a_jk = __shfl_sync(0xffffffffu, ah, home + u % kLanes);
+  };
+  if constexpr (kRowsHeld) {
+#pragma unroll
+    for (int u = 0; u < kEll; ++u) {
+      int32_t k;
+      int nk;
+      T a_jk;
+      row_of_mt(u, &k, &nk, &a_jk);
+#pragma unroll
+      for (int q = 0; q < kPer; ++q) {
+        const int e = q * kLanes + s;
+        r_row[u][q] = e < nk ? mt_all[static_cast<int64_t>(k) * a.cap_mt + e] : -1;
       }
-      at += __popc(mask);
     }
-    if (lane == 0) a.m_cnt[j] = kept;
-    written += static_cast<unsigned long long>(kept);
+  }
+  bool fits = true;
+  const auto mark = [&](int32_t row) {
+    if (w.Holds(row)) {
+      w.Mark(row);
+    } else {
+      fits = false;
+    }
+  };
+  if (valid && s == 0) mark(static_cast<int32_t>(j));
+  m_list.Rows(mark);
+  z_list.Rows(mark);
+  mt_list.Rows(mark);
+  constexpr int kSkip = kRowsHeld ? kPer * kLanes : 0;  // entries of a row of M^T that registers hold
+  if constexpr (kRowsHeld) {
+#pragma unroll
+    for (int u = 0; u < kEll; ++u) {
+#pragma unroll
+      for (int q = 0; q < kPer; ++q) {
+        if (r_row[u][q] >= 0) mark(r_row[u][q]);
+      }
+    }
+  }
+#pragma unroll 1
+  for (int u = 0; u < kEll; ++u) {
+    int32_t k;
+    int nk;
+    T a_jk;
+    row_of_mt(u, &k, &nk, &a_jk);
+    const int32_t* from = mt_all + static_cast<int64_t>(k) * a.cap_mt;
+#pragma unroll 1
+    for (int e = kSkip + s; e < nk; e += kLanes) mark(from[e]);
+  }
+  // the values travel while the rows are ranked
+  m_list.LoadValues();
+  z_list.LoadValues();
+  mt_list.LoadValues();
+  if constexpr (kRowsHeld) {
+#pragma unroll
+    for (int u = 0; u < kEll; ++u) {
+      const int32_t k = __shfl_sync(0xffffffffu, k_held[0], home + u % kLanes);
+      static_assert(kEll <= kLanes || !kRowsHeld, "one held entry per lane");
+#pragma unroll
+      for (int q = 0; q < kPer; ++q) {
+        r_val[u][q] = r_row[u][q] >= 0 ? mt_vals[static_cast<int64_t>(k) * a.cap_mt + q * kLanes + s] : T(0);
+      }
+    }
+  }
+  int count = kGroupDropRows + 1;
+  if (__all_sync(0xffffffffu, fits)) count = RankRows<true>(w, rows, list, kGroupDropRows, lane);
+  if (count > kGroupDropRows) {
+    ClearWindow(w, lane);
+    return false;
+  }
+#pragma unroll 1
+  for (int r = lane; r < count; r += kWarp) {
+#pragma unroll
+    for (int q = 0; q < C; ++q) own[r].v[q] = trans[r].v[q] = T(0);
+  }
+  __syncwarp();
+  // U(:, j): M, then + alpha Z
+  m_list.Entries([&](int32_t i, T v) { own[w.Rank(i)].v[c] = v; });
+  __syncwarp();
+  z_list.Entries([&](int32_t i, T v) {
+    T& u = own[w.Rank(i)].v[c];
+    u = Add(u, Mul(alpha, v));
+  });
+  // row j of A M, terms in ascending k: one row of M^T after another
+  const auto add = [&](int32_t i, T v, T a_jk) {
+    T& t = trans[w.Rank(i)].v[c];
+    t = Add(t, Mul(a_jk, v));
+  };
+  const auto add_rest = [&](int32_t k, int nk, T a_jk) {
+    const int64_t at = static_cast<int64_t>(k) * a.cap_mt;
+#pragma unroll 1
+    for (int e = kSkip + s; e < nk; e += kLanes) add(mt_all[at + e], mt_vals[at + e], a_jk);
+  };
+  if constexpr (kRowsHeld) {
+#pragma unroll
+    for (int u = 0; u < kEll; ++u) {
+      int32_t k;
+      int nk;
+      T a_jk;
+      row_of_mt(u, &k, &nk, &a_jk);
+#pragma unroll
+      for (int q = 0; q < kPer; ++q) {
+        if (r_row[u][q] >= 0) add(r_row[u][q], r_val[u][q], a_jk);
+      }
+      if (__any_sync(0xffffffffu, nk > kSkip)) add_rest(k, nk, a_jk);
+      __syncwarp();
+    }
+  } else {
+#pragma unroll 1
+    for (int u = 0; u < kEll; ++u) {
+      int32_t k;
+      int nk;
+      T a_jk;
+      row_of_mt(u, &k, &nk, &a_jk);
+      add_rest(k, nk, a_jk);
+      __syncwarp();
+    }
+  }
+  // alpha Z(j, :) = alpha pr_j (e_j - that), then + M(j, :)
+  T pr[C];
+#pragma unroll
+  for (int q = 0; q < C; ++q) pr[q] = j0 + q < a.n ? a.pr[j0 + q] : T(0);
+#pragma unroll 1
+  for (int r = lane; r < count; r += kWarp) {
+    const int64_t i = static_cast<int64_t>(w.lo) + rows[r];
+    Values t = trans[r];
+#pragma unroll
+    for (int q = 0; q < C; ++q) {
+      T rv = -t.v[q];
+      if (i == j0 + q) rv = Add(rv, T(1));
+      t.v[q] = rv == T(0) ? T(0) : Mul(alpha, Mul(pr[q], rv));
+    }
+    trans[r] = t;
+  }
+  __syncwarp();
+  mt_list.Entries([&](int32_t i, T v) {
+    T& t = trans[w.Rank(i)].v[c];
+    t = Add(v, t);
+  });
+  __syncwarp();
+#pragma unroll 1
+  for (int r = lane; r < count; r += kWarp) {
+    Values u = own[r];
+    const Values t = trans[r];
+#pragma unroll
+    for (int q = 0; q < C; ++q) u.v[q] = Mul(T(0.5), Add(u.v[q], t.v[q]));
+    own[r] = u;
+  }
+  __syncwarp();
+  // each column's nonzero entries, compacted (over trans, which is done with), then decided
+  T* column_vals = reinterpret_cast<T*>(trans);
+  uint16_t* column_rows = reinterpret_cast<uint16_t*>(column_vals + kGroupDropRows);
+  static_assert(kGroupDropRows * (sizeof(T) + sizeof(uint16_t)) <= kGroupDropRows * sizeof(Values), "the column fits");
+#pragma unroll 1
+  for (int q = 0; q < C; ++q) {
+    if (j0 + q >= a.n) break;
+    int entries = 0;
+#pragma unroll 1
+    for (int r0 = 0; r0 < count; r0 += kWarp) {
+      const int r = r0 + lane;
+      const T v = r < count ? reinterpret_cast<const T*>(own)[r * C + q] : T(0);
+      const bool some = !(v == T(0));
+      const unsigned mask = __ballot_sync(0xffffffffu, some);
+      if (some) {
+        const int o = entries + __popc(mask & LaneMaskBelow());
+        column_vals[o] = v;
+        column_rows[o] = rows[r];
+      }
+      entries += __popc(mask);
+    }
     __syncwarp();
+    const int kept = DropAndWrite<T>(a, [&](int r) { return w.lo + static_cast<int32_t>(column_rows[r]); },
+                                     column_vals, entries, j0 + q, parity ^ 1, lane, overflow);
+    *written += static_cast<unsigned long long>(kept);
+    __syncwarp();
+  }
+  ClearRows(w, rows, count, lane);
+  return true;
+}
+
+template <class T, int kEll, int C>
+__global__ void __launch_bounds__(kGroupWarps * kWarp) FusedDropKernel(const __grid_constant__ FusedArgs<T> a) {
+  extern __shared__ __align__(16) unsigned char fused_drop_smem[];
+  const int lane = threadIdx.x & 31;
+  unsigned char* base = fused_drop_smem + (threadIdx.x >> 5) * a.drop_bytes;
+  const int64_t parity = a.state->parity;
+  const T alpha = static_cast<T>(a.state->alpha);
+  const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  unsigned long long written = 0;
+  int overflow = 0;
+  bool clear = false;  // whether the window starts clear
+#pragma unroll 1
+  for (int64_t j0 = warp * C; j0 < a.n; j0 += warps * C) {
+    if (a.words > 0) {
+      if (!clear) {
+        unsigned char* at = base;
+        RowWindow w = WindowAt(at, a.words, 0);
+        ClearWindow(w, lane);
+        clear = true;
+      }
+      if (DropGroup<T, kEll, C>(a, base, j0, alpha, parity, lane, &written, &overflow)) continue;
+    }
+    clear = false;
+#pragma unroll 1
+    for (int64_t j = j0; j < j0 + C && j < a.n; ++j) overflow |= DropColumn<T>(a, base, j, &written);
   }
   overflow = __reduce_or_sync(0xffffffffu, overflow);
   if (lane == 0) {
-    if (written != 0ull) atomicAdd(&state->nnz_m, written);
-    if (overflow != 0) atomicOr(&state->overflow, overflow);
+    if (written != 0ull) atomicAdd(&a.state->nnz_m, written);
+    if (overflow != 0) atomicOr(&a.state->overflow, overflow);
   }
 }
 
@@ -515,12 +965,12 @@ __device__ __forceinline__ double SumStaged(double s, const double* src, int cou
   return s;
 }
 
+// One column on its own, for columns whose rows do not fit the group's window.
 template <class T, int kEll>
-__global__ void __launch_bounds__(kResidualWarps * kWarp) FusedResidualKernel(FusedArgs<T> a) {
-  extern __shared__ __align__(16) unsigned char fused_res_smem[];
+__device__ __noinline__ void ResidualColumn(const FusedArgs<T>& a, unsigned char* base, int64_t j,
+                                            unsigned long long* written_out) {
   const int lane = threadIdx.x & 31;
   constexpr int kSummary = (kWindowWords + kWarp * kWarp - 1) / (kWarp * kWarp) * kWarp;
-  unsigned char* base = fused_res_smem + (threadIdx.x >> 5) * ResidualSlabBytes<T>(a.m_hash_slots, a.z_hash_slots);
   uint32_t* bm = reinterpret_cast<uint32_t*>(base);
   base += Round16(static_cast<size_t>(kWindowWords) * 4);
   uint32_t* summary = reinterpret_cast<uint32_t*>(base);
@@ -542,14 +992,8 @@ __global__ void __launch_bounds__(kResidualWarps * kWarp) FusedResidualKernel(Fu
   ClearWords(bm, kWindowWords, lane);
   ClearWords(summary, kSummary, lane);
   __syncwarp();
-  const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-  unsigned long long written = 0;
-  int overflow = 0;
-  const int64_t read_set = a.state->parity;  // the M^T set the drop kernel has just read
-  for (int64_t j = warp; j < a.n; j += warps) {
+  {
     // ---- R(:, j) = e_j - A M(:, j) ----------------------------------------
-    if (lane == 0) a.mt_cnt[read_set][j] = 0;  // that set refills from zero in the next drop kernel
     const int nm = a.m_cnt[j];
     ClearTable(mkeys, a.m_hash_slots, lane);
     __syncwarp();
@@ -646,7 +1090,7 @@ __global__ void __launch_bounds__(kResidualWarps * kWarp) FusedResidualKernel(Fu
       a.sq[j] = sq;
       a.z_cnt[j] = kept;
     }
-    written += static_cast<unsigned long long>(kept);
+    *written_out += static_cast<unsigned long long>(kept);
     const bool z_displaced = !__all_sync(0xffffffffu, z_placed);
     // ---- projection: tt = ||Pr A Z(:, j)||^2, bt = <Z(:, j), Pr A Z(:, j)> --
     lo = INT32_MAX;
@@ -722,11 +1166,262 @@ __global__ void __launch_bounds__(kResidualWarps * kWarp) FusedResidualKernel(Fu
     if (lane == 1) a.bt[j] = proj;
     __syncwarp();
   }
-  overflow = __reduce_or_sync(0xffffffffu, overflow);
-  if (lane == 0) {
-    if (written != 0ull) atomicAdd(&a.state->nnz_z, written);
-    if (overflow != 0) atomicOr(&a.state->overflow, overflow);
+}
+
+// ---------------------------------------------------------------------------
+// The residual and projection of C adjacent columns (colgroup.cuh).  Two
+// windows: one ranks the rows k of M and later the rows of A Z, the other the
+// rows of R, whose ranks hold Z for the projection's lookups.  A product row i
+// walks row i of A in ascending k, one lookup per k for all columns; a column
+// that lacks k adds A(i, k) * 0, which changes at most the sign of a zero (the
+// host takes this path only when A and Pr are finite).  The 3 C column sums
+// run sequentially in row order, side by side on C or 2 C lanes.
+
+constexpr int kGroupResidualRows = 192;  // rows of R of a group
+constexpr int kGroupProductRows = 512;   // rows of A Z of a group taken at a time
+constexpr int kStageStride = kWarp + 2;  // doubles between two columns' staged terms: lanes hit different banks
+
+template <class T, int C>
+__host__ __device__ size_t ResidualGroupBytes(int words, int topk) {
+  return 2 * WindowBytes(words) + Round16(static_cast<size_t>(kGroupResidualRows) * 2) +
+         Round16(static_cast<size_t>(kGroupProductRows) * 2) + Round16(2 * C * kStageStride * sizeof(double)) +
+         Round16(static_cast<size_t>(C * topk + kGroupResidualRows + 2) * sizeof(GroupValues<T, C>));
+}
+
+// acc[q] += A(i, k) b_k[q] over row i of A, ascending k; an absent k reads the
+// zeros at vals[zero], so that no lookup waits for another's outcome.  kUse:
+// A's longest row (the slots past it are padding everywhere).
+template <class T, int C, int kEll, int kUse, class Sum>
+__device__ __forceinline__ void GroupRow(const FusedArgs<T>& a, const RowWindow& w, const GroupValues<T, C>* vals,
+                                         int zero, int32_t i, Sum& acc) {
+  const int4* ks = reinterpret_cast<const int4*>(a.a_rows_ell + static_cast<int64_t>(i) * kEll);
+  const T* vs = a.a_rows_ell_val + static_cast<int64_t>(i) * kEll;
+#pragma unroll
+  for (int u = 0; u < kEll / 4; ++u) {
+    const int4 k4 = ks[u];
+    T v4[4];
+    LoadFour(vs + 4 * u, v4);
+    const int32_t kk[4] = {k4.x, k4.y, k4.z, k4.w};  // padding (-1) is never marked
+    GroupValues<T, C> b[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (4 * u + e < kUse) b[e] = vals[w.FindOr(kk[e], zero)];
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (4 * u + e < kUse) {
+#pragma unroll
+        for (int q = 0; q < C; ++q) acc[q] = Add(acc[q], Mul(v4[e], b[e].v[q]));
+      }
+    }
   }
+}
+
+// False when the group does not fit (nothing written).
+template <class T, int kEll, int kUse, int C>
+__device__ __forceinline__ bool ResidualGroup(const FusedArgs<T>& a, unsigned char* base, int64_t j0, int lane,
+                                              unsigned long long* written) {
+  constexpr int kLanes = kWarp / C;
+  using Values = GroupValues<T, C>;
+  const int32_t lo = static_cast<int32_t>(j0) - a.words * 16;
+  RowWindow wm = WindowAt(base, a.words, lo);  // rows of M, then of A Z
+  RowWindow wr = WindowAt(base, a.words, lo);  // rows of R
+  uint16_t* rows = reinterpret_cast<uint16_t*>(base);
+  base += Round16(static_cast<size_t>(kGroupResidualRows) * 2);
+  uint16_t* prod = reinterpret_cast<uint16_t*>(base);
+  base += Round16(static_cast<size_t>(kGroupProductRows) * 2);
+  double* stage = reinterpret_cast<double*>(base);
+  base += Round16(2 * C * kStageStride * sizeof(double));
+  Values* mv = reinterpret_cast<Values*>(base);  // M by rank
+  Values* zv = mv + C * a.topk + 1;              // Z by rank
+  uint16_t* list = prod;                         // scratch of the first two rankings
+  const int c = lane / kLanes;
+  const int s = lane % kLanes;
+  const int64_t j = j0 + c;
+  const bool valid = j < a.n;
+  const int nm = valid ? a.m_cnt[j] : 0;
+  bool fits = true;
+  const auto mark = [&](RowWindow& w, int32_t row) {
+    if (w.Holds(row)) {
+      w.MarkNew(row);
+    } else {
+      fits = false;
+    }
+  };
+  if (valid && s == 0) mark(wr, static_cast<int32_t>(j));
+#pragma unroll 1
+  for (int e = s; e < nm; e += kLanes) {
+    const int32_t k = a.m_rows[j * a.topk + e];
+    mark(wm, k);
+    const int4* src = reinterpret_cast<const int4*>(a.a_cols_ell + static_cast<int64_t>(k) * kEll);
+#pragma unroll
+    for (int u = 0; u < kEll / 4; ++u) {
+      const int4 r4 = src[u];
+      if (r4.x >= 0) mark(wr, r4.x);
+      if (r4.y >= 0) mark(wr, r4.y);
+      if (r4.z >= 0) mark(wr, r4.z);
+      if (r4.w >= 0) mark(wr, r4.w);
+    }
+  }
+  int count = kGroupResidualRows + 1;
+  if (__all_sync(0xffffffffu, fits)) count = RankRows<true>(wr, rows, list, kGroupResidualRows, lane);
+  if (count > kGroupResidualRows) {
+    ClearWindow(wm, lane);
+    ClearWindow(wr, lane);
+    return false;
+  }
+  const int distinct = RankRows<true>(wm, nullptr, list, min(C * a.topk, kGroupProductRows), lane);
+#pragma unroll 1
+  for (int r = lane; r <= distinct; r += kWarp) {  // the zeros of absent rows past the end
+#pragma unroll
+    for (int q = 0; q < C; ++q) mv[r].v[q] = T(0);
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (int e = s; e < nm; e += kLanes) mv[wm.Rank(a.m_rows[j * a.topk + e])].v[c] = a.m_vals[j * a.topk + e];
+  __syncwarp();
+  // ---- R(:, j) = e_j - A M(:, j), Z = Pr R, ||R(:, j)||^2 on lane c ----------
+  int kept[C];
+#pragma unroll
+  for (int q = 0; q < C; ++q) kept[q] = 0;
+  double sq = 0.0;
+#pragma unroll 1
+  for (int r0 = 0; r0 <= count; r0 += kWarp) {
+    const int r = r0 + lane;
+    const int32_t i = r < count ? lo + static_cast<int32_t>(rows[r]) : -1;
+    T acc[C];
+#pragma unroll
+    for (int q = 0; q < C; ++q) acc[q] = T(-0.0);
+    T pri = T(0);
+    if (i >= 0) {
+      pri = a.pr[i];
+      GroupRow<T, C, kEll, kUse>(a, wm, mv, distinct, i, acc);
+    }
+    Values z;
+#pragma unroll
+    for (int q = 0; q < C; ++q) {
+      T v = -acc[q];
+      if (static_cast<int64_t>(i) == j0 + q) v = Add(v, T(1));
+      const bool keep = i >= 0 && j0 + q < a.n && !(v == T(0));  // Eigen prune(0.0)
+      z.v[q] = keep ? Mul(pri, v) : T(0);
+      const double sd = keep ? static_cast<double>(v) : 0.0;
+      stage[q * kStageStride + lane] = Mul(sd, sd);
+      const unsigned mask = __ballot_sync(0xffffffffu, keep);
+      if (keep) {
+        const int64_t o = (j0 + q) * a.cap_z + kept[q] + __popc(mask & LaneMaskBelow());
+        a.z_rows[o] = i;
+        a.z_vals[o] = z.v[q];
+      }
+      kept[q] += __popc(mask);
+    }
+    if (r <= count) zv[r] = z;  // zeros past the end
+    __syncwarp();
+    if (lane < C && r0 < count) sq = SumStaged(sq, stage + lane * kStageStride, min(kWarp, count - r0));
+    __syncwarp();
+  }
+#pragma unroll
+  for (int q = 0; q < C; ++q) {
+    if (lane == q && j0 + q < a.n) {
+      a.sq[j0 + q] = sq;
+      a.z_cnt[j0 + q] = kept[q];
+    }
+    *written += static_cast<unsigned long long>(kept[q]);
+  }
+  // M's rows leave their window
+#pragma unroll 1
+  for (int e = s; e < nm; e += kLanes) wm.bits[(a.m_rows[j * a.topk + e] - lo) >> 5] = 0u;
+#pragma unroll 1
+  for (int t = lane; t < GroupSummaryWords(a.words); t += kWarp) wm.summary[t] = 0u;
+  __syncwarp();
+  // ---- projection: ||Pr A Z(:, j)||^2 on lane c, <Z(:, j), Pr A Z(:, j)> on lane C + c
+  const int64_t first = max(static_cast<int64_t>(lo) + rows[0] - a.bandwidth, int64_t{0});
+  const int64_t last = min(static_cast<int64_t>(lo) + rows[count - 1] + a.bandwidth, a.n - 1);
+  double proj = 0.0;
+  int span = a.words * 32;  // rows of the running piece
+#pragma unroll 1
+  for (int64_t piece = first; piece <= last;) {
+    wm.lo = static_cast<int32_t>(piece);
+    const int32_t end = static_cast<int32_t>(min(last, piece + span - 1));
+#pragma unroll 1
+    for (int r = lane; r < count; r += kWarp) {
+      const int4* src = reinterpret_cast<const int4*>(a.a_cols_ell + (static_cast<int64_t>(lo) + rows[r]) * kEll);
+#pragma unroll
+      for (int u = 0; u < kEll / 4; ++u) {
+        const int4 r4 = src[u];
+        if (r4.x >= wm.lo && r4.x <= end) wm.MarkNew(r4.x);
+        if (r4.y >= wm.lo && r4.y <= end) wm.MarkNew(r4.y);
+        if (r4.z >= wm.lo && r4.z <= end) wm.MarkNew(r4.z);
+        if (r4.w >= wm.lo && r4.w <= end) wm.MarkNew(r4.w);
+      }
+    }
+    static_assert(2 * C * kStageStride * sizeof(double) >= kGroupProductRows * sizeof(uint16_t), "the list fits stage");
+    const int np = RankRows<false>(wm, prod, reinterpret_cast<uint16_t*>(stage), kGroupProductRows, lane);
+    if (np > kGroupProductRows) {
+      ClearWindow(wm, lane);
+      span >>= 1;  // fewer rows at a time; a piece of 256 rows always fits
+      continue;
+    }
+#pragma unroll 1
+    for (int r0 = 0; r0 < np; r0 += kWarp) {
+      const int r = r0 + lane;
+      if (r < np) {
+        const int32_t i = static_cast<int32_t>(piece) + static_cast<int32_t>(prod[r]);
+        T acc[C];
+#pragma unroll
+        for (int q = 0; q < C; ++q) acc[q] = T(-0.0);
+        GroupRow<T, C, kEll, kUse>(a, wr, zv, count, i, acc);
+        const T pri = a.pr[i];
+        const Values z = zv[wr.FindOr(i, count)];
+#pragma unroll
+        for (int q = 0; q < C; ++q) {
+          const double td = static_cast<double>(Mul(pri, acc[q]));
+          stage[q * kStageStride + lane] = Mul(td, td);
+          // rows that Z(:, j) lacks add 0, which leaves a sum started at +0.0 unchanged
+          stage[(C + q) * kStageStride + lane] = z.v[q] == T(0) ? 0.0 : Mul(static_cast<double>(z.v[q]), td);
+        }
+      }
+      __syncwarp();
+      if (lane < 2 * C) proj = SumStaged(proj, stage + lane * kStageStride, min(kWarp, np - r0));
+      __syncwarp();
+    }
+    ClearRows(wm, prod, np, lane);
+    piece += span;
+  }
+  if (lane < C && j0 + lane < a.n) a.tt[j0 + lane] = proj;
+  if (lane >= C && lane < 2 * C && j0 + lane - C < a.n) a.bt[j0 + lane - C] = proj;
+  ClearRows(wr, rows, count, lane);
+  return true;
+}
+
+template <class T, int kEll, int kUse, int C>
+__global__ void __launch_bounds__(kGroupWarps * kWarp) FusedResidualKernel(const __grid_constant__ FusedArgs<T> a) {
+  extern __shared__ __align__(16) unsigned char fused_res_smem[];
+  const int lane = threadIdx.x & 31;
+  unsigned char* base = fused_res_smem + (threadIdx.x >> 5) * a.residual_bytes;
+  const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  const int64_t read_set = a.state->parity;  // the M^T set the drop kernel has just read
+  unsigned long long written = 0;
+  bool clear = false;  // whether the windows start clear
+#pragma unroll 1
+  for (int64_t j0 = warp * C; j0 < a.n; j0 += warps * C) {
+    if (lane < C && j0 + lane < a.n) a.mt_cnt[read_set][j0 + lane] = 0;  // refilled from zero by the next drop kernel
+    if (a.words > 0) {
+      if (!clear) {
+        unsigned char* at = base;
+        RowWindow wm = WindowAt(at, a.words, 0);
+        RowWindow wr = WindowAt(at, a.words, 0);
+        ClearWindow(wm, lane);
+        ClearWindow(wr, lane);
+        clear = true;
+      }
+      if (ResidualGroup<T, kEll, kUse, C>(a, base, j0, lane, &written)) continue;
+    }
+    clear = false;
+#pragma unroll 1
+    for (int64_t j = j0; j < j0 + C && j < a.n; ++j) ResidualColumn<T, kEll>(a, base, j, &written);
+  }
+  if (lane == 0 && written != 0ull) atomicAdd(&a.state->nnz_z, written);
 }
 
 // ---------------------------------------------------------------------------
@@ -1001,12 +1696,12 @@ class FusedMr final : public FusedMrBase {
     for (int64_t body = 0; body <= p.max_iterations; ++body) {
       {
         prof::Scope scope(st, "fused_drop", 0.0);
-        FusedDropKernel<T><<<drop_grid_, kDropWarps * kWarp, drop_smem_, st>>>(args_);
+        drop_kernel_<<<drop_grid_, kGroupWarps * kWarp, drop_smem_, st>>>(args_);
         SPAI_LAUNCH_CHECK();
       }
       {
         prof::Scope scope(st, "fused_residual", 0.0);
-        res_kernel_<<<res_grid_, kResidualWarps * kWarp, res_smem_, st>>>(args_);
+        res_kernel_<<<res_grid_, kGroupWarps * kWarp, res_smem_, st>>>(args_);
         SPAI_LAUNCH_CHECK();
       }
       {
@@ -1068,6 +1763,8 @@ class FusedMr final : public FusedMrBase {
     a.z_hash_slots = NextPow2Int(std::max(2 * cap_z, kWarp));
     a.d_mt_slots = NextPow2Int(std::max(2 * cap_mt, kWarp));
     a.d_r_slots = DropRowSlots(p);
+    a.words = GroupWords(p);
+    a.bandwidth = p.bandwidth;
     a.max_iterations = p.max_iterations;
     a.tolerance = p.tolerance;
     a.a_cols_ell = p.a_cols_ell;
@@ -1101,7 +1798,7 @@ class FusedMr final : public FusedMrBase {
 
   static bool SameArgs(const FusedArgs<T>& x, const FusedArgs<T>& y) {
     bool same = x.n == y.n && x.topk == y.topk && x.cap_z == y.cap_z && x.cap_mt == y.cap_mt &&
-                x.ell == y.ell && x.m_hash_slots == y.m_hash_slots && x.d_r_slots == y.d_r_slots &&
+                x.ell == y.ell && x.words == y.words && x.bandwidth == y.bandwidth && x.m_hash_slots == y.m_hash_slots && x.d_r_slots == y.d_r_slots &&
                 x.d_mt_slots == y.d_mt_slots &&
                 x.z_hash_slots == y.z_hash_slots && x.max_iterations == y.max_iterations &&
                 x.tolerance == y.tolerance && x.a_cols_ell == y.a_cols_ell && x.a_rows_ell == y.a_rows_ell &&
@@ -1116,36 +1813,83 @@ class FusedMr final : public FusedMrBase {
     return same;
   }
 
-  // Kernel choice, shared memory and grids (once per problem shape).
-  void Configure(const FusedMrProblem& p) {
-    switch (p.ell_width) {
-      case 4: res_kernel_ = FusedResidualKernel<T, 4>; break;
-      case 8: res_kernel_ = FusedResidualKernel<T, 8>; break;
-      case 12: res_kernel_ = FusedResidualKernel<T, 12>; break;
-      case 16: res_kernel_ = FusedResidualKernel<T, 16>; break;
+  // Words of a group's window: a little over four bandwidths of A on either
+  // side of the group, which covers the drop step's and the residual's rows of
+  // nearly every column (M reaches two to three bandwidths, R one more).  Wider
+  // operators, and operators with entries that are not finite (a column group
+  // multiplies them by the 0 of an absent entry), go column by column.
+  static int GroupWords(const FusedMrProblem& p) {
+    if (!p.finite) return 0;
+    const int64_t words = CeilDiv(8 * p.bandwidth + p.bandwidth / 4, 32) + 8;
+    return words > kMaxGroupWords ? 0 : static_cast<int>(CeilDiv(words, 32) * 32);
+  }
+
+  // Columns per group: four, or two while four would leave the chip's warps
+  // idle (below 16 groups of four per SM; at n = 4,096 a launch takes 15 us in
+  // groups of two, the latency of one group, and took 31 us column by column).
+  // kUse: the longest row of A, compile time for the 5-point and 7-point
+  // operators (2-D rows would else look up three slots of padding in eight).
+  template <int kEll, int kUse, int C>
+  void Choose() {
+    res_kernel_ = FusedResidualKernel<T, kEll, kUse, C>;
+    drop_kernel_ = FusedDropKernel<T, kEll, C>;
+    columns_ = C;
+    size_t drop = DropWarpBytes<T>(args_.topk + args_.cap_z, args_.d_mt_slots, args_.d_r_slots);
+    size_t residual = ResidualSlabBytes<T>(args_.m_hash_slots, args_.z_hash_slots);
+    if (args_.words > 0) {
+      drop = std::max(drop, DropGroupBytes<T, C>(args_.words));
+      residual = std::max(residual, ResidualGroupBytes<T, C>(args_.words, args_.topk));
+    }
+    args_.drop_bytes = Round16(drop);
+    args_.residual_bytes = Round16(residual);
+  }
+
+  template <int C>
+  void ChooseEll(int ell, int64_t longest) {
+    switch (ell) {
+      case 4: Choose<4, 4, C>(); break;
+      case 8:  // the 5-point and 7-point rows have kernels of their own length
+        if (longest <= 5) {
+          Choose<8, 5, C>();
+        } else if (longest <= 7) {
+          Choose<8, 7, C>();
+        } else {
+          Choose<8, 8, C>();
+        }
+        break;
+      case 12: Choose<12, 12, C>(); break;
+      case 16: Choose<16, 16, C>(); break;
       default: throw std::invalid_argument("fused MR: unsupported ELL width");
     }
-    drop_smem_ = static_cast<size_t>(kDropWarps) *
-                 DropWarpBytes<T>(args_.topk + args_.cap_z, args_.d_mt_slots, args_.d_r_slots);
-    res_smem_ = static_cast<size_t>(kResidualWarps) * ResidualSlabBytes<T>(args_.m_hash_slots, args_.z_hash_slots);
-    SPAI_CUDA(cudaFuncSetAttribute(FusedDropKernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  }
+
+  // Kernel choice, shared memory and grids (once per problem shape).
+  void Configure(const FusedMrProblem& p) {
+    int device = 0;
+    SPAI_CUDA(cudaGetDevice(&device));
+    int sms = 0;
+    SPAI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    if (args_.n >= int64_t{4} * 16 * sms) {
+      ChooseEll<4>(p.ell_width, p.a_longest);
+    } else {
+      ChooseEll<2>(p.ell_width, p.a_longest);
+    }
+    drop_smem_ = static_cast<size_t>(kGroupWarps) * args_.drop_bytes;
+    res_smem_ = static_cast<size_t>(kGroupWarps) * args_.residual_bytes;
+    SPAI_CUDA(cudaFuncSetAttribute(drop_kernel_, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(drop_smem_)));
     SPAI_CUDA(cudaFuncSetAttribute(res_kernel_, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(res_smem_)));
     int drop_blocks = 0;
     int res_blocks = 0;
-    SPAI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&drop_blocks, FusedDropKernel<T>, kDropWarps * kWarp,
+    SPAI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&drop_blocks, drop_kernel_, kGroupWarps * kWarp,
                                                             drop_smem_));
-    SPAI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res_blocks, res_kernel_, kResidualWarps * kWarp,
+    SPAI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res_blocks, res_kernel_, kGroupWarps * kWarp,
                                                             res_smem_));
     if (drop_blocks < 1 || res_blocks < 1) throw std::runtime_error("fused MR: kernels do not fit on an SM");
-    int device = 0;
-    SPAI_CUDA(cudaGetDevice(&device));
-    int sms = 0;
-    SPAI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    drop_grid_ = static_cast<unsigned>(std::min<int64_t>(CeilDiv(args_.n, kDropWarps), int64_t{sms} * drop_blocks));
-    res_grid_ =
-        static_cast<unsigned>(std::min<int64_t>(CeilDiv(args_.n, kResidualWarps), int64_t{sms} * res_blocks));
+    const int64_t blocks = CeilDiv(args_.n, int64_t{kGroupWarps} * columns_);
+    drop_grid_ = static_cast<unsigned>(std::min<int64_t>(blocks, int64_t{sms} * drop_blocks));
+    res_grid_ = static_cast<unsigned>(std::min<int64_t>(blocks, int64_t{sms} * res_blocks));
     decide_grid_ = static_cast<unsigned>(CeilDiv(args_.n, kTreeChunk));
   }
 
@@ -1175,8 +1919,8 @@ class FusedMr final : public FusedMrBase {
       SPAI_CUDA(cudaStreamUpdateCaptureDependencies(cs, &loop_node, 1, cudaStreamSetCaptureDependencies));
       cudaGraph_t body = params.conditional.phGraph_out[0];
       SPAI_CUDA(cudaStreamBeginCaptureToGraph(bs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-      FusedDropKernel<T><<<drop_grid_, kDropWarps * kWarp, drop_smem_, bs>>>(a);
-      res_kernel_<<<res_grid_, kResidualWarps * kWarp, res_smem_, bs>>>(a);
+      drop_kernel_<<<drop_grid_, kGroupWarps * kWarp, drop_smem_, bs>>>(a);
+      res_kernel_<<<res_grid_, kGroupWarps * kWarp, res_smem_, bs>>>(a);
       FusedDecideKernel<T><<<decide_grid_, kTreeLanes, 0, bs>>>(a, loop, true);
       SPAI_CUDA(cudaGetLastError());
       cudaGraph_t body_out = nullptr;
@@ -1220,7 +1964,9 @@ class FusedMr final : public FusedMrBase {
   std::unique_ptr<FusedState, PinnedFree> host_state_holder_;
   FusedArgs<T> args_{};
   cudaGraphExec_t exec_ = nullptr;
-  void (*res_kernel_)(FusedArgs<T>) = nullptr;
+  void (*res_kernel_)(const FusedArgs<T>) = nullptr;
+  void (*drop_kernel_)(const FusedArgs<T>) = nullptr;
+  int columns_ = 1;
   size_t drop_smem_ = 0;
   size_t res_smem_ = 0;
   unsigned drop_grid_ = 1;

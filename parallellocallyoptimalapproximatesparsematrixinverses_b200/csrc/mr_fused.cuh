@@ -46,6 +46,8 @@ struct FusedMrProblem {
   const int32_t* a_rows_ell = nullptr;   // columns of A(i, :)
   const void* a_rows_ell_val = nullptr;  // values of A(i, :) (T)
   const void* pr = nullptr;              // diag(Pr) (T)
+  int64_t bandwidth = 0;                 // largest |i - k| over the entries of A
+  bool finite = true;                    // every value of A and Pr is finite
   int64_t max_iterations = 0;
   double tolerance = 0.0;
 };

@@ -77,6 +77,34 @@ __global__ void LongestKernel(const int64_t* __restrict__ ptr_a, const int64_t* 
   if (m != 0ull) atomicMax(out, m);
 }
 
+// The largest |row - column| over x's entries into out[0], and whether any of
+// its values or of d is not finite into out[1] (both zeroed by the caller).
+template <class T>
+__global__ void BandwidthKernel(CscView<T> x, const T* __restrict__ d, unsigned long long* __restrict__ out) {
+  unsigned long long widest = 0;
+  bool finite = true;
+  for (int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; j < x.cols;
+       j += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    finite = finite && isfinite(d[j]);
+    for (int64_t p = x.ptr[j]; p < x.ptr[j + 1]; ++p) {
+      const int64_t i = x.idx[p];
+      const unsigned long long w = static_cast<unsigned long long>(i > j ? i - j : j - i);
+      widest = w > widest ? w : widest;
+      finite = finite && isfinite(x.val[p]);
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long other = __shfl_xor_sync(0xffffffffu, widest, o);
+    widest = other > widest ? other : widest;
+  }
+  finite = __all_sync(0xffffffffu, finite);
+  if ((threadIdx.x & 31) == 0) {
+    if (widest != 0ull) atomicMax(&out[0], widest);
+    if (!finite) atomicOr(&out[1], 1ull);
+  }
+}
+
 // pr[j] = 1 / A(j, j) (methods_common.cpp:50-63); *bad |= 1 for a missing,
 // non-positive or non-finite diagonal, |= 2 for a non-finite inverse.
 template <class T>
@@ -1030,6 +1058,9 @@ class Solver final : public SolverBase {
       problem.a_rows_ell = a_rows_ell_.data();
       problem.a_rows_ell_val = a_rows_ell_val_.data();
       problem.pr = pr_vec_.data();
+      MeasureA();
+      problem.bandwidth = a_bandwidth_;
+      problem.finite = a_finite_;
       problem.max_iterations = opt_.max_iterations;
       problem.tolerance = opt_.tolerance;
       if (FusedMrApplicable(problem)) {
@@ -1198,6 +1229,19 @@ class Solver final : public SolverBase {
     }
   }
 
+  // A's bandwidth and whether A and Pr are finite, once per problem.
+  void MeasureA() {
+    if (a_bandwidth_ >= 0) return;
+    unsigned long long* out = ctx_.select_state.data();
+    SPAI_CUDA(cudaMemsetAsync(out, 0, 2 * sizeof(unsigned long long), ctx_.stream));
+    BandwidthKernel<T><<<GridFor(n_, 128), 128, 0, ctx_.stream>>>(View(A()), pr_vec_.data(), out);
+    SPAI_LAUNCH_CHECK();
+    SPAI_CUDA(cudaMemcpyAsync(ctx_.host_counts, out, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, ctx_.stream));
+    ctx_.Sync();
+    a_bandwidth_ = ctx_.host_counts[0];
+    a_finite_ = ctx_.host_counts[1] == 0;
+  }
+
   // Global MR with per-column top-k, a diagonal Pr and ELL copies of A, in the device order.
   bool FusedEligible() const {
     return FusedMrEnabled() && fused_allowed_ && opt_.method == Method::kGlobalMr && opt_.dropping &&
@@ -1229,6 +1273,8 @@ class Solver final : public SolverBase {
   DevBuf<T> a_rows_ell_val_;
   int ell_width_ = 0;
   int64_t a_longest_ = 0;  // longest column or row of A
+  int64_t a_bandwidth_ = -1;  // largest |i - j| over A's entries (-1: not measured)
+  bool a_finite_ = true;      // A and Pr hold finite values only
   static constexpr int kMaxEllWidth = 16;
   std::unique_ptr<FusedMrBase> fused_;
   bool fused_allowed_ = true;
