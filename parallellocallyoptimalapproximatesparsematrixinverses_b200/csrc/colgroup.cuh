@@ -167,6 +167,11 @@ __device__ __forceinline__ uint32_t MagnitudeBits(float v) {
 __device__ __forceinline__ unsigned long long MagnitudeBits(double v) {
   return static_cast<unsigned long long>(__double_as_longlong(v)) & 0x7FFFFFFFFFFFFFFFull;
 }
+// The magnitude with these bits (the second argument selects the type).
+__device__ __forceinline__ float MagnitudeFrom(uint32_t key, float) { return __int_as_float(static_cast<int>(key)); }
+__device__ __forceinline__ double MagnitudeFrom(unsigned long long key, double) {
+  return __longlong_as_double(static_cast<long long>(key));
+}
 template <class T>
 struct MagnitudeOf;
 template <>

@@ -47,6 +47,8 @@ struct Ctx {
   DevBuf<int32_t> pad_idx;               // padded rows of the union and drop steps
   DevBuf<unsigned char> pad_val;         // padded values of the union and drop steps
   DevBuf<double> dot_terms;              // products of a dot in the reference's order
+  DevBuf<double> cut_abs;                // per-column top-k cut: magnitude
+  DevBuf<int32_t> cut_row;               // and smallest row kept at it
   double* host_scalars = nullptr;   // pinned, kScalarSlots
   int64_t* host_counts = nullptr;   // pinned, 8
   int32_t* host_flags = nullptr;    // pinned, 8

@@ -1,0 +1,33 @@
+"""Per-column sums and the per-column top-k of a direction against the oracle,
+bit for bit: column counts that do not fill a warp's four, columns from one
+entry to about a thousand, equal and different patterns, ties at the cut (the
+Laplacian's repeated magnitudes), caps of one entry and of more than a warp."""
+import numpy as np
+import pytest
+
+from oracle import pyoracle
+from parallellocallyoptimalapproximatesparsematrixinverses_b200 import global_spai, inner_outer, problems
+from tests.helpers import assert_same_result
+
+pytestmark = pytest.mark.gpu
+
+OPERATORS = {
+    "tridiagonal_6": lambda: problems.tridiagonal(6),
+    "laplacian_33": lambda: problems.laplacian_2d(33),
+    "diffusion_3d_9": lambda: problems.diffusion_3d(9, 1.0, 2),
+    "banded_1001": lambda: problems.random_banded_spd(1001, 4, 3, seed=5),
+}
+
+
+@pytest.mark.parametrize("topk", [1, 7, 40])
+@pytest.mark.parametrize("operator", sorted(OPERATORS))
+@pytest.mark.parametrize("family,name", [("global_spai", "cg"), ("global_spai", "lomr"), ("inner_outer", "lomr")])
+def test_sums_and_topk_match_the_oracle(require_gpu, family, name, operator, topk):
+    A = OPERATORS[operator]()
+    kw = dict(M0=problems.diagonal_inverse(A), max_iterations=4, tolerance=0.0,
+              max_density=min(1.0, max(topk, 2) / A.shape[0]))
+    method = getattr({"global_spai": global_spai, "inner_outer": inner_outer}[family], name)
+    got = method(A, topk_per_column=topk, summation="device", **kw)
+    want = pyoracle.run(family, name, A, topk_per_column=topk, order=pyoracle.ORDER_DEVICE, **kw)
+    assert_same_result(got, want, f"{family}.{name} {operator} top-{topk}")
+    assert np.all(np.isfinite(got.history["residual_norm"]))
