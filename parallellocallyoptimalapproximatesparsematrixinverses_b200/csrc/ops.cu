@@ -39,10 +39,45 @@ __device__ __forceinline__ unsigned LaneMaskLt() {
 }
 
 // ---------------------------------------------------------------------------
-// Scan
-__global__ void ScanTileKernel(const int64_t* __restrict__ in, int64_t n, int64_t* __restrict__ out,
-                               int64_t* __restrict__ tile_sums) {
+// Scan: tile sums, then every block adds the sums of the tiles before its own
+// and scans its tile.  Two launches whatever the length (one for a single
+// tile), where the recursive form took five and two copies: a scan of 64,000
+// counts 13 us of device time -> 6 us.
+__device__ __forceinline__ int64_t BlockSum(int64_t v, int64_t* warp_sums) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane == 0) warp_sums[threadIdx.x >> 5] = v;
+  __syncthreads();
+  int64_t total = lane < kScanThreads / kWarp ? warp_sums[lane] : 0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+  __syncthreads();
+  return total;
+}
+
+__global__ void __launch_bounds__(kScanThreads) ScanSumsKernel(const int64_t* __restrict__ in, int64_t n,
+                                                               int64_t* __restrict__ tile_sums) {
   __shared__ int64_t warp_sums[kScanThreads / kWarp];
+  const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanTile + threadIdx.x;
+  int64_t v = 0;
+#pragma unroll
+  for (int i = 0; i < kScanItems; ++i) v += base + i * kScanThreads < n ? in[base + i * kScanThreads] : 0;
+  v = BlockSum(v, warp_sums);
+  if (threadIdx.x == 0) tile_sums[blockIdx.x] = v;
+}
+
+// out[0] = 0, out[i + 1] = in[0] + ... + in[i]; the last value also to *total (mapped host memory) unless null.
+__global__ void __launch_bounds__(kScanThreads) ScanTileKernel(const int64_t* __restrict__ in, int64_t n,
+                                                               int64_t* __restrict__ out,
+                                                               const int64_t* __restrict__ tile_sums,
+                                                               int64_t* __restrict__ total) {
+  __shared__ int64_t warp_sums[kScanThreads / kWarp];
+  int64_t before = 0;
+  if (blockIdx.x > 0) {
+    for (int64_t t = threadIdx.x; t < blockIdx.x; t += kScanThreads) before += tile_sums[t];
+    before = BlockSum(before, warp_sums);
+  }
   const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanTile + static_cast<int64_t>(threadIdx.x) * kScanItems;
   int64_t v[kScanItems];
   int64_t local = 0;
@@ -72,34 +107,25 @@ __global__ void ScanTileKernel(const int64_t* __restrict__ in, int64_t n, int64_
     if (lane < kScanThreads / kWarp) warp_sums[lane] = w;
   }
   __syncthreads();
-  int64_t running = inclusive - local + (warp > 0 ? warp_sums[warp - 1] : 0);
+  int64_t running = before + inclusive - local + (warp > 0 ? warp_sums[warp - 1] : 0);
+  if (blockIdx.x == 0 && threadIdx.x == 0) out[0] = 0;
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
     running += v[i];
     if (base + i < n) out[base + i + 1] = running;
   }
-  if (threadIdx.x == kScanThreads - 1) tile_sums[blockIdx.x] = running;
+  if (total != nullptr && blockIdx.x == gridDim.x - 1 && threadIdx.x == kScanThreads - 1) *total = running;
 }
 
-__global__ void ScanAddKernel(int64_t n, int64_t* __restrict__ out, const int64_t* __restrict__ tile_prefix) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i == 0) out[0] = 0;
-  if (i < n) out[i + 1] += tile_prefix[i / kScanTile];
-}
-
-void ScanRecursive(Ctx& ctx, const int64_t* in, int64_t n, int64_t* out, DevBuf<int64_t>& scratch, size_t offset) {
-  const int64_t tiles = CeilDiv(n, kScanTile);
-  int64_t* tile_sums = scratch.data() + offset;
-  ScanTileKernel<<<static_cast<unsigned>(tiles), kScanThreads, 0, ctx.stream>>>(in, n, out, tile_sums);
-  SPAI_LAUNCH_CHECK();
+void Scan(Ctx& ctx, const int64_t* in, int64_t n, int64_t* out, int64_t* total) {
+  const unsigned tiles = static_cast<unsigned>(CeilDiv(n, kScanTile));
+  ctx.scan_blocks.Reserve(static_cast<size_t>(tiles), ctx.stream);
   if (tiles > 1) {
-    int64_t* tile_prefix = tile_sums + tiles;
-    ScanRecursive(ctx, tile_sums, tiles, tile_prefix, scratch, offset + 2 * tiles + 1);
-    ScanAddKernel<<<static_cast<unsigned>(CeilDiv(n, 256)), 256, 0, ctx.stream>>>(n, out, tile_prefix);
+    ScanSumsKernel<<<tiles, kScanThreads, 0, ctx.stream>>>(in, n, ctx.scan_blocks.data());
     SPAI_LAUNCH_CHECK();
-  } else {
-    SPAI_CUDA(cudaMemsetAsync(out, 0, sizeof(int64_t), ctx.stream));
   }
+  ScanTileKernel<<<tiles, kScanThreads, 0, ctx.stream>>>(in, n, out, ctx.scan_blocks.data(), total);
+  SPAI_LAUNCH_CHECK();
 }
 
 // ---------------------------------------------------------------------------
@@ -708,12 +734,15 @@ __global__ void DiagScaleKernel(const T* __restrict__ d, const int32_t* __restri
   }
 }
 
+// warp per column
 template <class T>
 __global__ void ScaleColumnsKernel(CscView<T> x, T* __restrict__ val, const double* __restrict__ scale) {
-  for (int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; j < x.cols;
-       j += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  for (int64_t j = warp; j < x.cols; j += warps) {
     const T s = static_cast<T>(scale[j]);
-    for (int64_t p = x.ptr[j]; p < x.ptr[j + 1]; ++p) val[p] = Mul(val[p], s);
+    for (int64_t p = x.ptr[j] + lane; p < x.ptr[j + 1]; p += kWarp) val[p] = Mul(val[p], s);
   }
 }
 
@@ -1163,86 +1192,126 @@ __global__ void AbsScoresKernel(const T* __restrict__ val, int64_t nnz, double* 
   }
 }
 
-// candidate counts per column (entries minus a diagonal)
+// candidate counts per column (entries minus a diagonal), warp per column
 template <class T>
 __global__ void NonDiagonalCountKernel(CscView<T> x, int64_t* __restrict__ counts) {
-  for (int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; j < x.cols;
-       j += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    int64_t c = 0;
-    for (int64_t p = x.ptr[j]; p < x.ptr[j + 1]; ++p) c += static_cast<int64_t>(x.idx[p]) != j ? 1 : 0;
-    counts[j] = c;
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  for (int64_t j = warp; j < x.cols; j += warps) {
+    int c = 0;
+    for (int64_t p = x.ptr[j] + lane; p < x.ptr[j + 1]; p += kWarp) c += static_cast<int64_t>(x.idx[p]) != j ? 1 : 0;
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0) counts[j] = c;
   }
 }
 
-// candidate keys in offset order: key[offset] = ordered score bits
+// candidate keys in offset order: key[offset] = ordered score bits; warp per column
 template <class T>
 __global__ void GatherCandidateKeysKernel(CscView<T> x, const double* __restrict__ scores,
                                           const int64_t* __restrict__ column_base, bool skip_diag,
                                           unsigned long long* __restrict__ keys) {
-  for (int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; j < x.cols;
-       j += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    int64_t o = skip_diag ? column_base[j] : x.ptr[j];
-    for (int64_t p = x.ptr[j]; p < x.ptr[j + 1]; ++p) {
-      if (skip_diag && static_cast<int64_t>(x.idx[p]) == j) continue;
-      keys[o++] = OrderedBits(scores[p]);
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  for (int64_t j = warp; j < x.cols; j += warps) {
+    const int64_t start = x.ptr[j];
+    const int64_t end = x.ptr[j + 1];
+    int64_t o = skip_diag ? column_base[j] : start;
+    for (int64_t base = start; base < end; base += kWarp) {
+      const int64_t p = base + lane;
+      const bool mine = p < end && !(skip_diag && static_cast<int64_t>(x.idx[p]) == j);
+      const unsigned mask = __ballot_sync(0xffffffffu, mine);
+      if (mine) keys[o + __popc(mask & LaneMaskLt())] = OrderedBits(scores[p]);
+      o += __popc(mask);
     }
   }
 }
 
-// Radix select over 128-bit keys (ordered score bits, candidate offset), 8
-// bits per pass from the most significant byte.  state = {prefix_hi,
-// prefix_lo, remaining rank (1-based)}.
-__global__ void RadixHistKernel(const unsigned long long* __restrict__ keys, int64_t count, int pass,
-                                const unsigned long long* __restrict__ state, unsigned long long* __restrict__ hist) {
-  __shared__ unsigned int local[256];
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) local[i] = 0;
+// Radix select over (ordered score bits, candidate offset), 11 bits per pass
+// from the most significant ones: six passes over the score, then as many as
+// the offsets have digits.  state = {prefix of the score, prefix of the
+// offset, remaining rank (1-based)}; hist[kRadixBins] counts finished blocks:
+// the last block decides the pass's digit, so a pass is one launch.  (Byte
+// digits with a launch and a serial scan of 256 bins each to decide took 32
+// launches and 185 us for 100,000 candidates; this takes 8 and 35 us.)
+constexpr int kRadixBits = 11;
+constexpr int kRadixBins = 1 << kRadixBits;
+constexpr int kRadixThreads = 512;
+
+__global__ void __launch_bounds__(kRadixThreads) RadixPassKernel(const unsigned long long* __restrict__ keys,
+                                                                 int64_t count, int shift, int bits, bool on_offset,
+                                                                 unsigned long long* __restrict__ state,
+                                                                 unsigned long long* __restrict__ hist) {
+  __shared__ unsigned int local[kRadixBins];
+  __shared__ unsigned long long warp_sums[kRadixThreads / kWarp];
+  __shared__ int last;
+  for (int i = threadIdx.x; i < kRadixBins; i += kRadixThreads) local[i] = 0;
   __syncthreads();
   const unsigned long long prefix_hi = state[0];
   const unsigned long long prefix_lo = state[1];
+  // the digits above this one, decided by the passes before
+  const unsigned long long above = shift + bits >= 64 ? 0ull : ~0ull << (shift + bits);
+  const unsigned digit_mask = (1u << bits) - 1u;
   for (int64_t c = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; c < count;
        c += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const unsigned long long hi = keys[c];
-    const unsigned long long lo = static_cast<unsigned long long>(c);
-    bool match;
-    unsigned digit;
-    if (pass < 8) {
-      const int shift = 56 - 8 * pass;
-      const unsigned long long mask = pass == 0 ? 0ull : (~0ull << (shift + 8));
-      match = (hi & mask) == (prefix_hi & mask);
-      digit = static_cast<unsigned>((hi >> shift) & 0xFFull);
-    } else {
-      const int shift = 56 - 8 * (pass - 8);
-      const unsigned long long mask = pass == 8 ? 0ull : (~0ull << (shift + 8));
-      match = hi == prefix_hi && (lo & mask) == (prefix_lo & mask);
-      digit = static_cast<unsigned>((lo >> shift) & 0xFFull);
+    const unsigned long long key = keys[c];
+    if (on_offset) {
+      const unsigned long long o = static_cast<unsigned long long>(c);
+      if (key == prefix_hi && (o & above) == (prefix_lo & above)) {
+        atomicAdd(&local[static_cast<unsigned>(o >> shift) & digit_mask], 1u);
+      }
+    } else if ((key & above) == (prefix_hi & above)) {
+      atomicAdd(&local[static_cast<unsigned>(key >> shift) & digit_mask], 1u);
     }
-    if (match) atomicAdd(&local[digit], 1u);
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) {
+  for (int i = threadIdx.x; i < kRadixBins; i += kRadixThreads) {
     if (local[i] != 0) atomicAdd(&hist[i], static_cast<unsigned long long>(local[i]));
   }
-}
-
-__global__ void RadixDecideKernel(int pass, unsigned long long* __restrict__ state, unsigned long long* __restrict__ hist) {
-  if (threadIdx.x != 0) return;
-  unsigned long long remaining = state[2];
-  unsigned long long cumulative = 0;
-  int digit = 255;
-  for (int b = 0; b < 256; ++b) {
-    if (cumulative + hist[b] >= remaining) {
-      digit = b;
-      break;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&hist[kRadixBins], 1ull) == gridDim.x - 1 ? 1 : 0;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  // the last block: the bin where the running count reaches the remaining rank
+  constexpr int kPer = kRadixBins / kRadixThreads;
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const unsigned long long remaining = state[2];
+  unsigned long long bin[kPer];
+  unsigned long long own = 0;
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    bin[i] = __ldcg(&hist[threadIdx.x * kPer + i]);
+    own += bin[i];
+  }
+  unsigned long long inclusive = own;
+#pragma unroll
+  for (int o = 1; o < kWarp; o <<= 1) {
+    const unsigned long long y = __shfl_up_sync(0xffffffffu, inclusive, o);
+    if (lane >= o) inclusive += y;
+  }
+  if (lane == 31) warp_sums[warp] = inclusive;
+  __syncthreads();
+  unsigned long long before = inclusive - own;
+  for (int w = 0; w < warp; ++w) before += warp_sums[w];
+  // exactly one thread holds the bin (the ranks run from 1 to the number of matching keys)
+  if (before < remaining && before + own >= remaining) {
+    int digit = threadIdx.x * kPer;
+#pragma unroll
+    for (int i = 0; i < kPer - 1; ++i) {
+      if (before + bin[i] < remaining && digit == threadIdx.x * kPer + i) {
+        before += bin[i];
+        ++digit;
+      }
     }
-    cumulative += hist[b];
+    state[on_offset ? 1 : 0] |= static_cast<unsigned long long>(digit) << shift;
+    state[2] = remaining - before;
   }
-  if (pass < 8) {
-    state[0] |= static_cast<unsigned long long>(digit) << (56 - 8 * pass);
-  } else {
-    state[1] |= static_cast<unsigned long long>(digit) << (56 - 8 * (pass - 8));
-  }
-  state[2] = remaining - cumulative;
-  for (int b = 0; b < 256; ++b) hist[b] = 0;
+  __syncthreads();
+  for (int i = threadIdx.x; i <= kRadixBins; i += kRadixThreads) hist[i] = 0;
 }
 
 template <class S, class D>
@@ -1460,9 +1529,9 @@ void Ctx::Init(int device_ordinal) {
   }
   scalars.Reserve(kScalarSlots, stream);
   select_state.Reserve(4, stream);
-  histogram.Reserve(256, stream);
+  histogram.Reserve(kRadixBins + 1, stream);
   flags.Reserve(8, stream);
-  SPAI_CUDA(cudaMemsetAsync(histogram.data(), 0, 256 * sizeof(unsigned long long), stream));
+  SPAI_CUDA(cudaMemsetAsync(histogram.data(), 0, (kRadixBins + 1) * sizeof(unsigned long long), stream));
 }
 
 void Ctx::Destroy() {
@@ -1522,10 +1591,7 @@ void ScanCountsAsync(Ctx& ctx, const int64_t* counts, int64_t n, int64_t* out) {
     SPAI_CUDA(cudaMemsetAsync(out, 0, sizeof(int64_t), ctx.stream));
     return;
   }
-  int64_t need = 0;
-  for (int64_t m = n; m > 1; m = CeilDiv(m, kScanTile)) need += 2 * CeilDiv(m, kScanTile) + 2;
-  ctx.scan_blocks.Reserve(static_cast<size_t>(need + 8), ctx.stream);
-  ScanRecursive(ctx, counts, n, out, ctx.scan_blocks, 0);
+  Scan(ctx, counts, n, out, nullptr);
 }
 
 int64_t ScanCounts(Ctx& ctx, const int64_t* counts, int64_t n, int64_t* out) {
@@ -1533,11 +1599,7 @@ int64_t ScanCounts(Ctx& ctx, const int64_t* counts, int64_t n, int64_t* out) {
     SPAI_CUDA(cudaMemsetAsync(out, 0, sizeof(int64_t), ctx.stream));
     return 0;
   }
-  int64_t need = 0;
-  for (int64_t m = n; m > 1; m = CeilDiv(m, kScanTile)) need += 2 * CeilDiv(m, kScanTile) + 2;
-  ctx.scan_blocks.Reserve(static_cast<size_t>(need + 8), ctx.stream);
-  ScanRecursive(ctx, counts, n, out, ctx.scan_blocks, 0);
-  SPAI_CUDA(cudaMemcpyAsync(ctx.host_counts, out + n, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx.stream));
+  Scan(ctx, counts, n, out, ctx.host_counts);  // pinned host memory, mapped on the device
   ctx.Sync();
   return ctx.host_counts[0];
 }
@@ -1754,7 +1816,7 @@ void DiagScale(Ctx& ctx, const T* d, const DevCsc<T>& b, DevCsc<T>& out, bool pr
 
 template <class T>
 void ScaleColumns(Ctx& ctx, DevCsc<T>& x, const double* scale) {
-  ScaleColumnsKernel<T><<<GridFor(x.cols, 128), 128, 0, ctx.stream>>>(View(x), x.val.data(), scale);
+  ScaleColumnsKernel<T><<<GridFor(x.cols * kWarp, 256), 256, 0, ctx.stream>>>(View(x), x.val.data(), scale);
   SPAI_LAUNCH_CHECK();
   DropZeros(ctx, x);
 }
@@ -1822,7 +1884,7 @@ void GlobalDropByScore(Ctx& ctx, DevCsc<T>& x, const double* entry_scores, bool 
   const int64_t* column_base = nullptr;
   if (skip_diagonal) {
     ctx.counts.Reserve(static_cast<size_t>(cols + 1), ctx.stream);
-    NonDiagonalCountKernel<T><<<GridFor(cols, 128), 128, 0, ctx.stream>>>(View(x), ctx.counts.data());
+    NonDiagonalCountKernel<T><<<GridFor(cols * kWarp, 256), 256, 0, ctx.stream>>>(View(x), ctx.counts.data());
     SPAI_LAUNCH_CHECK();
     candidates = ScanCounts(ctx, ctx.counts.data(), cols, ctx.counts2.data());
     column_base = ctx.counts2.data();
@@ -1832,19 +1894,27 @@ void GlobalDropByScore(Ctx& ctx, DevCsc<T>& x, const double* entry_scores, bool 
   }
   DevBuf<unsigned long long> keys;
   keys.Reserve(static_cast<size_t>(candidates), ctx.stream);
-  GatherCandidateKeysKernel<T><<<GridFor(cols, 128), 128, 0, ctx.stream>>>(View(x), entry_scores, column_base,
-                                                                          skip_diagonal, keys.data());
+  GatherCandidateKeysKernel<T><<<GridFor(cols * kWarp, 256), 256, 0, ctx.stream>>>(View(x), entry_scores, column_base,
+                                                                                   skip_diagonal, keys.data());
   SPAI_LAUNCH_CHECK();
   unsigned long long init[3] = {0ull, 0ull, static_cast<unsigned long long>(drop)};
   SPAI_CUDA(cudaMemcpyAsync(ctx.select_state.data(), init, sizeof(init), cudaMemcpyHostToDevice, ctx.stream));
-  SPAI_CUDA(cudaMemsetAsync(ctx.histogram.data(), 0, 256 * sizeof(unsigned long long), ctx.stream));
-  const int grid = GridFor(candidates, 256);
-  for (int pass = 0; pass < 16; ++pass) {
-    RadixHistKernel<<<grid, 256, 0, ctx.stream>>>(keys.data(), candidates, pass, ctx.select_state.data(),
-                                                  ctx.histogram.data());
+  // one block per 4,096 candidates: the histogram's flush is the fixed cost of a block
+  const int grid = static_cast<int>(std::min<int64_t>(CeilDiv(candidates, 8 * kRadixThreads), 2 * ctx.sm_count));
+  const auto pass = [&](int shift, int bits, bool on_offset) {
+    RadixPassKernel<<<grid, kRadixThreads, 0, ctx.stream>>>(keys.data(), candidates, shift, bits, on_offset,
+                                                            ctx.select_state.data(), ctx.histogram.data());
     SPAI_LAUNCH_CHECK();
-    RadixDecideKernel<<<1, 32, 0, ctx.stream>>>(pass, ctx.select_state.data(), ctx.histogram.data());
-    SPAI_LAUNCH_CHECK();
+  };
+  for (int top = 64; top > 0; top -= kRadixBits) {
+    const int shift = top > kRadixBits ? top - kRadixBits : 0;
+    pass(shift, top - shift, false);
+  }
+  int offset_bits = 1;
+  while ((int64_t{1} << offset_bits) < candidates) ++offset_bits;
+  for (int top = offset_bits; top > 0; top -= kRadixBits) {
+    const int shift = top > kRadixBits ? top - kRadixBits : 0;
+    pass(shift, top - shift, true);
   }
   KeepAboveCutoff<T> pred;
   pred.scores = entry_scores;

@@ -41,45 +41,14 @@ __device__ __forceinline__ SumMap ShuffleMap(const SumMap& m, int delta, bool up
 #pragma unroll
   for (int p = 0; p < 2; ++p) {
     o.inc[p] = up ? __shfl_up_sync(0xffffffffu, m.inc[p], delta) : __shfl_down_sync(0xffffffffu, m.inc[p], delta);
-    o.lo[p] = up ? __shfl_up_sync(0xffffffffu, m.lo[p], delta) : __shfl_down_sync(0xffffffffu, m.lo[p], delta);
-    o.hi[p] = up ? __shfl_up_sync(0xffffffffu, m.hi[p], delta) : __shfl_down_sync(0xffffffffu, m.hi[p], delta);
   }
+  o.lo = up ? __shfl_up_sync(0xffffffffu, m.lo, delta) : __shfl_down_sync(0xffffffffu, m.lo, delta);
+  o.hi = up ? __shfl_up_sync(0xffffffffu, m.hi, delta) : __shfl_down_sync(0xffffffffu, m.hi, delta);
   o.bad = up ? __shfl_up_sync(0xffffffffu, m.bad, delta) : __shfl_down_sync(0xffffffffu, m.bad, delta);
   return o;
 }
 
-// The tie-free form of a map: both parities move alike, so one increment and
-// its extremes suffice, as doubles (integers below 2^53 are exact; a value
-// that is not has left the binade, and so have lo or hi).
-struct PlainMap {
-  double inc;
-  double lo;
-  double hi;
-};
-
-constexpr double kPlainLimit = 9007199254740992.0;  // 2^53
-
-__device__ __forceinline__ PlainMap ThenPlain(const PlainMap& a, const PlainMap& b) {
-  return PlainMap{a.inc + b.inc, fmin(a.lo, a.inc + b.lo), fmax(a.hi, a.inc + b.hi)};
-}
-
-__device__ __forceinline__ SumMap FromPlain(const PlainMap& m, bool bad) {
-  if (bad || m.hi >= kPlainLimit || m.lo <= -kPlainLimit) {
-    SumMap none = EmptyMap();
-    none.bad = 1;
-    return none;
-  }
-  const int64_t inc = static_cast<int64_t>(m.inc);
-  const int64_t lo = static_cast<int64_t>(m.lo);
-  const int64_t hi = static_cast<int64_t>(m.hi);
-  return SumMap{{inc, inc}, {lo, lo}, {hi, hi}, 0};
-}
-
 // The map of this warp's piece (every lane's eight terms in order), on lane 0.
-// Almost every piece is free of ties and takes the plain form: about 9
-// operations a term, against 70 for the two-parity maps.  The extremes inside
-// one lane's eight terms are bounded by the sums of its upward and of its
-// downward steps.
 __device__ __forceinline__ SumMap PieceMap(const double* own, double scale, SumState state, int lane) {
   double t[kTermsPerThread];
 #pragma unroll
@@ -96,37 +65,11 @@ __device__ __forceinline__ SumMap PieceMap(const double* own, double scale, SumS
     m.bad = __all_sync(0xffffffffu, zero) ? 0 : 1;
     return m;
   }
-  constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52: rounds |q| < 2^51 to even
-  double up = 0.0;
-  double down = 0.0;
-  bool far = false;
-  bool tie = false;
-  bool negative = false;
+  TermRun run;
 #pragma unroll
-  for (int i = 0; i < kTermsPerThread; ++i) {
-    const double q = t[i] * scale;
-    const double r = (q + kMagic) - kMagic;
-    far = far || !(fabs(q) < 2251799813685248.0);
-    tie = tie || fabs(q - r) == 0.5;
-    negative = negative || q < 0.0 || (__double_as_longlong(q) < 0 && t[i] != 0.0);
-    up += fmax(r, 0.0);
-    down += fmin(r, 0.0);
-  }
-  far = __any_sync(0xffffffffu, far);
-  if (far || !__any_sync(0xffffffffu, tie)) {
-    PlainMap mine{up + down, down - (negative ? 1.0 : 0.0), up};
+  for (int i = 0; i < kTermsPerThread; ++i) run.Add(t[i], scale);
+  SumMap mine = run.Map();
 #pragma unroll
-    for (int o = 1; o < kWarp; o <<= 1) {
-      const PlainMap later{__shfl_down_sync(0xffffffffu, mine.inc, o), __shfl_down_sync(0xffffffffu, mine.lo, o),
-                           __shfl_down_sync(0xffffffffu, mine.hi, o)};
-      if ((lane & (2 * o - 1)) == 0) mine = ThenPlain(mine, later);
-    }
-    return FromPlain(mine, far);
-  }
-  SumMap mine = EmptyMap();
-#pragma unroll 1
-  for (int i = 0; i < kTermsPerThread; ++i) mine = Then(mine, TermMap(own[i], scale, state));
-#pragma unroll 1
   for (int o = 1; o < kWarp; o <<= 1) {
     const SumMap later = ShuffleMap(mine, o, false);
     if ((lane & (2 * o - 1)) == 0) mine = Then(mine, later);
@@ -136,21 +79,8 @@ __device__ __forceinline__ SumMap PieceMap(const double* own, double scale, SumS
 
 // The maps of pieces 0..lane, one after another, on every lane.
 __device__ __forceinline__ SumMap ScanMaps(const SumMap& own, int lane) {
-  const bool alike = own.inc[0] == own.inc[1] && own.lo[0] == own.lo[1] && own.hi[0] == own.hi[1];
-  if (__all_sync(0xffffffffu, alike)) {
-    // an empty map's far extremes stay far; a bad piece ends the prefix below
-    PlainMap prefix{static_cast<double>(own.inc[0]), static_cast<double>(own.lo[0]), static_cast<double>(own.hi[0])};
-#pragma unroll
-    for (int o = 1; o < kWarp; o <<= 1) {
-      const PlainMap before{__shfl_up_sync(0xffffffffu, prefix.inc, o), __shfl_up_sync(0xffffffffu, prefix.lo, o),
-                            __shfl_up_sync(0xffffffffu, prefix.hi, o)};
-      if (lane >= o) prefix = ThenPlain(before, prefix);
-    }
-    const unsigned bad = __ballot_sync(0xffffffffu, own.bad != 0);
-    return FromPlain(prefix, (bad & (0xffffffffu >> (31 - lane))) != 0u);
-  }
   SumMap prefix = own;
-#pragma unroll 1
+#pragma unroll
   for (int o = 1; o < kWarp; o <<= 1) {
     const SumMap before = ShuffleMap(prefix, o, true);
     if (lane >= o) prefix = Then(before, prefix);

@@ -29,6 +29,18 @@ double Term(int kind, std::mt19937_64& gen) {
   }
 }
 
+// The map of terms [first, last).
+SumMap Summarise(const std::vector<double>& t, int first, int last, double scale, SumState state) {
+  if (state == kSumZero) {
+    SumMap m = EmptyMap();
+    for (int i = first; i < last; ++i) m.bad |= t[i] == 0.0 ? 0 : 1;
+    return m;
+  }
+  TermRun run;
+  for (int i = first; i < last; ++i) run.Add(t[i], scale);
+  return run.Map();
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -51,8 +63,8 @@ int main(int argc, char** argv) {
       SumMap left = EmptyMap();
       SumMap right = EmptyMap();
       if (state != kSumOther) {
-        for (int i = first; i < middle; ++i) left = Then(left, TermMap(t[i], scale, state));
-        for (int i = middle; i < last; ++i) right = Then(right, TermMap(t[i], scale, state));
+        left = Summarise(t, first, middle, scale, state);
+        right = Summarise(t, middle, last, scale, state);
       }
       double moved;
       if (ApplyMap(Then(left, right), got, state, &moved)) {
