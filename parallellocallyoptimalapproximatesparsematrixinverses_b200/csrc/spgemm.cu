@@ -9,22 +9,19 @@
 //               memory beyond the largest bin).
 //  2. row-set list    (same warps, after the scan of the counts) -- writes the
 //     sorted rows of every column (bitmap: lane-blocked popcount prefix;
-//     hash: compaction + bitonic sort) and the column id of every entry.
-//  3. values          (one thread per output entry) -- entry (i, j) walks row
-//     i of X (CSR copy) in ascending k, finds each k in column j of B by a
-//     binary search (eight searches in flight per thread), and accumulates
-//     the first product x*y then += x*y in ascending k: the reference's
-//     accumulation order (Eigen's conservative sparse product), no FMA.
-//     Products and sums use the storage type's arithmetic: FP64 for double
-//     storage (bit-compatible with the reference), FP32 multiply and
-//     accumulate for float storage (the mixed-precision form); the global
-//     reductions built from them are FP64 either way.
+//     hash: compaction + bitonic sort).
+//  3. values          (one warp per output column) -- entry (i, j) walks row i
+//     of X (CSR copy) in ascending k, finds each k in column j of B through a
+//     bitmap of that column, and accumulates the first product x*y then += x*y
+//     in ascending k: the reference's accumulation order (Eigen's conservative
+//     sparse product), no FMA.  Products and sums use the storage type's
+//     arithmetic: FP64 for double storage (bit-compatible with the reference),
+//     FP32 multiply and accumulate for float storage (the mixed-precision
+//     form); the global reductions built from them are FP64 either way.
 //  4. column sums     (one thread per column) -- sequential per-column sums in
 //     row order for the global reductions (||R||^2, the MR projection).
 //
-// Stages 1-2 are latency-bound warp-per-column work on small shared-memory
-// structures; stage 3, where the arithmetic happens, is parallel over all
-// output entries so the memory system sees enough independent loads.
+// All stages are latency-bound work on small shared-memory structures.
 
 #include <cuda_runtime.h>
 
@@ -179,7 +176,6 @@ struct RowSetArgs {
   int64_t* counts;           // count mode output
   const int64_t* c_ptr;      // list mode: output offsets
   int32_t* rows;             // list mode: sorted rows
-  int32_t* cols;             // list mode: column id of every entry
   unsigned char* global_space;
 };
 
@@ -228,13 +224,11 @@ __global__ void BitmapRowSetKernel(RowSetArgs<T> a, int words_cap, int lo_words,
         if (lane >= o) inclusive += y;
       }
       int64_t out = a.c_ptr[col] + (inclusive - local);
-      const int32_t col32 = static_cast<int32_t>(col);
       for (int w = w0; w < w1; ++w) {
         uint32_t bits = bm[w];
         while (bits != 0u) {
           const int bit = __ffs(bits) - 1;
           a.rows[out] = lo + (w << 5) + bit;
-          a.cols[out] = col32;
           ++out;
           bits &= bits - 1u;
         }
@@ -317,10 +311,8 @@ __global__ void HashRowSetKernel(RowSetArgs<T> a, int slots, int64_t lo_need, in
       }
     }
     const int64_t out = a.c_ptr[col];
-    const int32_t col32 = static_cast<int32_t>(col);
     for (int i = lane; i < n; i += kWarp) {
       a.rows[out + i] = sorted[i];
-      a.cols[out + i] = col32;
     }
     __syncwarp();
   }
@@ -334,9 +326,8 @@ template <class T>
 struct ValuesArgs {
   CscView<T> x_csr;
   CscView<T> b;
-  const int32_t* rows;
-  const int32_t* cols;
-  int64_t count;
+  const int64_t* c_ptr;  // output (or mask) column offsets
+  const int32_t* rows;   // and rows
   int mode;
   bool prune;
   T* out;              // kStore/kResidual: C values; kProjection: t = pr * (X B)
@@ -346,68 +337,234 @@ struct ValuesArgs {
   int32_t* flag;       // set when a stored value is an exact zero (pruning needed)
 };
 
+// Shared memory of one warp: a bitmap of B(:, j)'s rows and the position of each word's first entry.
+__host__ __device__ inline size_t ValuesSlabBytes(int words) {
+  return Round16(static_cast<size_t>(words) * 4) + Round16(static_cast<size_t>(words) * 2);
+}
+
+constexpr int kValuesPiece = 4096;  // entries of a column that one warp takes at a time
+constexpr int kValuesMaxWords = 1024;
+
+// Warp per output column: lane r forms output rows r, r + 32, ... in ascending
+// k, eight entries of row i of X at a time.  An entry k is found in B(:, j) by
+// its bit and the position of its word's first entry plus a population count:
+// two shared-memory reads, because B's column is sorted and its entries are
+// their own ranks.  A column of B wider than the bitmap (32,768 rows at most)
+// is searched by bisection, as every column was: eight searches in lock step
+// per thread and output entry took 1,330 us for 4,096 columns of about 3,000
+// entries with 1,300 entries in B's column.
 template <class T>
-__global__ void __launch_bounds__(256) ValuesKernel(ValuesArgs<T> a) {
+__global__ void __launch_bounds__(256) ValuesKernel(ValuesArgs<T> a, int words_cap) {
+  extern __shared__ __align__(16) unsigned char values_smem[];
+  const int lane = threadIdx.x & 31;
+  unsigned char* base = values_smem + (threadIdx.x >> 5) * ValuesSlabBytes(words_cap);
+  uint32_t* bits = reinterpret_cast<uint32_t*>(base);
+  uint16_t* first = reinterpret_cast<uint16_t*>(base + Round16(static_cast<size_t>(words_cap) * 4));
+  ClearWords(bits, words_cap, lane);
+  __syncwarp();
   bool zero_seen = false;
-  for (int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < a.count;
-       p += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int32_t i = a.rows[p];
-    const int32_t j = a.cols[p];
+  const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  const auto column = [&](int64_t j) {
     const int64_t bs = a.b.ptr[j];
     const int blen = static_cast<int>(a.b.ptr[j + 1] - bs);
-    const int64_t xs = a.x_csr.ptr[i];
-    const int64_t xe = a.x_csr.ptr[i + 1];
-    T acc = T(0);  // the storage type's arithmetic (see ColumnProductKernel)
+    const int32_t* b_idx = a.b.idx + bs;
+    const T* b_val = a.b.val + bs;
+    // blockIdx.y takes every gridDim.y-th piece of the column's entries
+    const int64_t begin = a.c_ptr[j] + static_cast<int64_t>(blockIdx.y) * kValuesPiece;
+    const int64_t end = a.c_ptr[j + 1];
+    if (begin >= end) return;
+    const int32_t w0 = blen > 0 ? b_idx[0] >> 5 : 0;
+    const int words = blen > 0 ? (b_idx[blen - 1] >> 5) - w0 + 1 : 0;
+    const bool mapped = words <= words_cap && blen <= 65535;
+    if (mapped) {
+      for (int e = lane; e < blen; e += kWarp) {
+        const int32_t k = b_idx[e];
+        const int w = (k >> 5) - w0;
+        atomicOr(&bits[w], 1u << (k & 31));
+        if (e == 0 || (b_idx[e - 1] >> 5) - w0 != w) first[w] = static_cast<uint16_t>(e);
+      }
+      __syncwarp();
+    }
+    const int64_t skip = static_cast<int64_t>(gridDim.y - 1) * kValuesPiece;
+    int64_t piece_end = min(begin + kValuesPiece, end);
+    for (int64_t p = begin + lane; p < end; p += kWarp) {
+      if (p >= piece_end) {  // pieces are whole rounds of 32: every lane moves on together
+        p += skip;
+        if (p >= end) break;
+        piece_end = min(p - lane + kValuesPiece, end);
+      }
+      const int32_t i = a.rows[p];
+      const int64_t xs = a.x_csr.ptr[i];
+      const int64_t xe = a.x_csr.ptr[i + 1];
+      T acc = T(0);  // the storage type's arithmetic (see ColumnProductKernel)
+      bool has = false;
+      for (int64_t q0 = xs; q0 < xe; q0 += 8) {
+        int32_t kk[8];
+        T xv[8];
+        int at[8];  // position in B(:, j), or -1
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int64_t q = q0 + u;
+          kk[u] = q < xe ? a.x_csr.idx[q] : INT32_MAX;
+          xv[u] = q < xe ? a.x_csr.val[q] : T(0);
+        }
+        if (mapped) {
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const int w = (kk[u] >> 5) - w0;
+            const bool in = static_cast<unsigned>(w) < static_cast<unsigned>(words);
+            const uint32_t word = in ? bits[w] : 0u;
+            const uint32_t bit = 1u << (kk[u] & 31);
+            at[u] = (word & bit) != 0u ? first[w] + __popc(word & (bit - 1u)) : -1;
+          }
+        } else {
+#pragma unroll
+          for (int u = 0; u < 8; ++u) at[u] = 0;
+          int len = blen;
+          while (len > 1) {
+            const int half = len >> 1;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              if (b_idx[at[u] + half] <= kk[u]) at[u] += half;
+            }
+            len -= half;
+          }
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            if (blen == 0 || b_idx[at[u]] != kk[u]) at[u] = -1;
+          }
+        }
+        T bv[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) bv[u] = at[u] >= 0 ? b_val[at[u]] : T(0);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          if (at[u] >= 0) {
+            const T prod = Mul(xv[u], bv[u]);
+            acc = has ? Add(acc, prod) : prod;
+            has = true;
+          }
+        }
+      }
+      if (a.mode == static_cast<int>(ValueMode::kMasked)) {
+        a.out_f64[p] = has ? static_cast<double>(acc) : 0.0;
+        continue;
+      }
+      if (a.mode == static_cast<int>(ValueMode::kProjection)) {
+        a.out[p] = Mul(a.row_scale[i], acc);
+        continue;
+      }
+      T v = acc;
+      if (a.mode == static_cast<int>(ValueMode::kResidual)) {
+        v = has ? -acc : T(0);
+        if (static_cast<int64_t>(i) == j) v = has ? Add(v, T(1)) : T(1);
+      }
+      const T stored = v;
+      a.out[p] = stored;
+      if (a.z_out != nullptr) a.z_out[p] = Mul(a.row_scale[i], stored);
+      if (a.prune && stored == T(0)) zero_seen = true;  // Eigen prune(0.0): +-0 go, NaN stays
+    }
+    __syncwarp();
+    if (mapped) {
+      for (int e = lane; e < blen; e += kWarp) bits[(b_idx[e] >> 5) - w0] = 0u;
+      __syncwarp();
+    }
+  };
+  if (blockIdx.y == 0) {
+    for (int64_t j = warp; j < a.b.cols; j += warps) column(j);
+  } else {
+    // the few columns long enough to have a piece for this split
+    for (int64_t j0 = warp * kWarp; j0 < a.b.cols; j0 += warps * kWarp) {
+      const int64_t j = j0 + lane;
+      const int64_t len = j < a.b.cols ? a.c_ptr[j + 1] - a.c_ptr[j] : 0;
+      for (unsigned left = __ballot_sync(0xffffffffu, len > static_cast<int64_t>(blockIdx.y) * kValuesPiece); left != 0u;
+           left &= left - 1u) {
+        column(j0 + __ffs(left) - 1);
+      }
+    }
+  }
+  if (__any_sync(0xffffffffu, zero_seen) && lane == 0) atomicOr(a.flag, 1);
+}
+
+// The masked product for short mask columns: one thread per mask entry, its
+// eight searches of B(:, j) in lock step.  Below about 32 entries a column a
+// warp per column leaves lanes idle and its bitmap is not paid back: 200 us
+// against 278 us for the two masks of the 47^3 residual gradient (25 and 7
+// entries a column), 75 against 45 us the other way for 40 entries a column.
+constexpr int64_t kMaskedWarpEntries = 32;
+
+template <class T>
+__global__ void ColumnIdsKernel(CscView<T> m, int32_t* __restrict__ cols) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  for (int64_t j = warp; j < m.cols; j += warps) {
+    for (int64_t p = m.ptr[j] + lane; p < m.ptr[j + 1]; p += kWarp) cols[p] = static_cast<int32_t>(j);
+  }
+}
+
+template <class T>
+__global__ void __launch_bounds__(256) MaskedEntriesKernel(CscView<T> x_csr, CscView<T> b,
+                                                           const int32_t* __restrict__ rows,
+                                                           const int32_t* __restrict__ cols, int64_t count,
+                                                           double* __restrict__ out) {
+  for (int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < count;
+       p += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int32_t i = rows[p];
+    const int64_t bs = b.ptr[cols[p]];
+    const int blen = static_cast<int>(b.ptr[cols[p] + 1] - bs);
+    const int32_t* b_idx = b.idx + bs;
+    const int64_t xs = x_csr.ptr[i];
+    const int64_t xe = x_csr.ptr[i + 1];
+    T acc = T(0);
     bool has = false;
     for (int64_t q0 = xs; q0 < xe; q0 += 8) {
       int32_t kk[8];
       T xv[8];
-      int64_t at[8];
+      int at[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         const int64_t q = q0 + u;
-        kk[u] = q < xe ? a.x_csr.idx[q] : INT32_MAX;
-        xv[u] = q < xe ? a.x_csr.val[q] : T(0);
-        at[u] = bs;
+        kk[u] = q < xe ? x_csr.idx[q] : INT32_MAX;
+        xv[u] = q < xe ? x_csr.val[q] : T(0);
+        at[u] = 0;
       }
-      // eight lower-bound searches in column j of B, in lock step
       int len = blen;
       while (len > 1) {
         const int half = len >> 1;
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-          if (a.b.idx[at[u] + half] <= kk[u]) at[u] += half;
+          if (b_idx[at[u] + half] <= kk[u]) at[u] += half;
         }
         len -= half;
       }
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        if (blen > 0 && q0 + u < xe && a.b.idx[at[u]] == kk[u]) {
-          const T prod = Mul(xv[u], a.b.val[at[u]]);
+        if (blen > 0 && q0 + u < xe && b_idx[at[u]] == kk[u]) {
+          const T prod = Mul(xv[u], b.val[bs + at[u]]);
           acc = has ? Add(acc, prod) : prod;
           has = true;
         }
       }
     }
-    if (a.mode == static_cast<int>(ValueMode::kMasked)) {
-      a.out_f64[p] = has ? static_cast<double>(acc) : 0.0;
-      continue;
-    }
-    if (a.mode == static_cast<int>(ValueMode::kProjection)) {
-      a.out[p] = Mul(a.row_scale[i], acc);
-      continue;
-    }
-    T v = acc;
-    if (a.mode == static_cast<int>(ValueMode::kResidual)) {
-      v = has ? -acc : T(0);
-      if (i == j) v = has ? Add(v, T(1)) : T(1);
-    }
-    const T stored = v;
-    a.out[p] = stored;
-    if (a.z_out != nullptr) a.z_out[p] = Mul(a.row_scale[i], stored);
-    if (a.prune && stored == T(0)) zero_seen = true;  // Eigen prune(0.0): +-0 go, NaN stays
+    out[p] = has ? static_cast<double>(acc) : 0.0;
   }
-  if (__any_sync(0xffffffffu, zero_seen) && (threadIdx.x & 31) == 0) atomicOr(a.flag, 1);
+}
+
+template <class T>
+void LaunchValues(Ctx& ctx, const ValuesArgs<T>& args) {
+  // a bitmap over all rows of B, up to 32,768 of them (wider ones would cost resident warps)
+  const int words = static_cast<int>(std::min<int64_t>(kValuesMaxWords, CeilDiv(args.b.rows, 32) + 1));
+  constexpr int kWarps = 8;
+  const size_t smem = ValuesSlabBytes(words) * kWarps;
+  SPAI_CUDA(cudaFuncSetAttribute(ValuesKernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(ValuesSlabBytes(kValuesMaxWords) * kWarps)));
+  // a column long enough to keep a warp busy for long is split over up to eight
+  const unsigned split = static_cast<unsigned>(std::min<int64_t>(8, CeilDiv(args.x_csr.cols, 2 * kValuesPiece)));
+  const dim3 grid(static_cast<unsigned>(GridFor(args.b.cols * kWarp, kWarps * kWarp)), split);
+  ValuesKernel<T><<<grid, kWarps * kWarp, smem, ctx.stream>>>(args, words);
+  SPAI_LAUNCH_CHECK();
 }
 
 // ---------------------------------------------------------------------------
@@ -821,14 +978,6 @@ __global__ void __launch_bounds__(256) NeedKernel(CscView<T> x, const int32_t* _
   }
 }
 
-template <class T>
-__global__ void ColumnIdsKernel(CscView<T> m, int32_t* __restrict__ cols) {
-  for (int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; j < m.cols;
-       j += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    for (int64_t p = m.ptr[j]; p < m.ptr[j + 1]; ++p) cols[p] = static_cast<int32_t>(j);
-  }
-}
-
 struct HashBin {
   int slots;
   int warps;
@@ -1195,28 +1344,22 @@ bool Spgemm(Ctx& ctx, const DevCsc<T>& x_csc, const DevCsc<T>& x_csr, const DevC
     }
     prof::Scope scope(ctx.stream, "spgemm_numeric", bytes);
     {
-      ctx.sg_cols.Reserve(static_cast<size_t>(nnz > 0 ? nnz : 1), ctx.stream);
       rs.list = true;
       rs.c_ptr = c_ptr;
       rs.rows = rows;
-      rs.cols = ctx.sg_cols.data();
       LaunchRowSets(ctx, rs, host_max);
       ValuesArgs<T> va{};
       va.x_csr = View(x_csr);
       va.b = View(b);
+      va.c_ptr = c_ptr;
       va.rows = rows;
-      va.cols = ctx.sg_cols.data();
-      va.count = nnz;
       va.mode = static_cast<int>(mode);
       va.prune = prune;
       va.out = vals;
       va.z_out = want_z ? zbuf.data() : nullptr;
       va.row_scale = static_cast<const T*>(extras.row_scale);
       va.flag = ctx.flags.data();
-      if (nnz > 0) {
-        ValuesKernel<T><<<GridFor(nnz, 256), 256, 0, ctx.stream>>>(va);
-        SPAI_LAUNCH_CHECK();
-      }
+      if (nnz > 0) LaunchValues(ctx, va);
       if (projection || extras.col_squares != nullptr) {
         SumsArgs<T> sa{c_ptr, rows, vals, View(b), projection, extras.col_squares, extras.proj_tt, extras.proj_bt,
                        cols};
@@ -1256,20 +1399,24 @@ bool Spgemm(Ctx& ctx, const DevCsc<T>& x_csc, const DevCsc<T>& x_csr, const DevC
 template <class T>
 void SpgemmMasked(Ctx& ctx, const DevCsc<T>& x_csr, const DevCsc<T>& b, const DevCsc<T>& mask, double* out) {
   if (mask.nnz == 0) return;
-  ctx.sg_cols.Reserve(static_cast<size_t>(mask.nnz), ctx.stream);
-  ColumnIdsKernel<T><<<GridFor(mask.cols, 128), 128, 0, ctx.stream>>>(View(mask), ctx.sg_cols.data());
-  SPAI_LAUNCH_CHECK();
+  if (mask.nnz < kMaskedWarpEntries * mask.cols) {
+    ctx.sg_cols.Reserve(static_cast<size_t>(mask.nnz), ctx.stream);
+    ColumnIdsKernel<T><<<GridFor(mask.cols * kWarp, 256), 256, 0, ctx.stream>>>(View(mask), ctx.sg_cols.data());
+    SPAI_LAUNCH_CHECK();
+    MaskedEntriesKernel<T><<<GridFor(mask.nnz, 256), 256, 0, ctx.stream>>>(
+        View(x_csr), View(b), mask.idx.data(), ctx.sg_cols.data(), mask.nnz, out);
+    SPAI_LAUNCH_CHECK();
+    return;
+  }
   ValuesArgs<T> va{};
   va.x_csr = View(x_csr);
   va.b = View(b);
+  va.c_ptr = mask.ptr.data();
   va.rows = mask.idx.data();
-  va.cols = ctx.sg_cols.data();
-  va.count = mask.nnz;
   va.mode = static_cast<int>(ValueMode::kMasked);
   va.out_f64 = out;
   va.flag = ctx.flags.data();
-  ValuesKernel<T><<<GridFor(mask.nnz, 256), 256, 0, ctx.stream>>>(va);
-  SPAI_LAUNCH_CHECK();
+  LaunchValues(ctx, va);
 }
 
 template bool Spgemm<double>(Ctx&, const DevCsc<double>&, const DevCsc<double>&, const DevCsc<double>&,

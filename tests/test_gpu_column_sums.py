@@ -31,3 +31,30 @@ def test_sums_and_topk_match_the_oracle(require_gpu, family, name, operator, top
     want = pyoracle.run(family, name, A, topk_per_column=topk, order=pyoracle.ORDER_DEVICE, **kw)
     assert_same_result(got, want, f"{family}.{name} {operator} top-{topk}")
     assert np.all(np.isfinite(got.history["residual_norm"]))
+
+
+# masks of one entry, of a few and of many entries a column (a thread per entry, or a warp per column), against
+# columns of R that the bitmap holds and columns spread over more rows than it takes
+@pytest.mark.parametrize("operator,per_column", [("diffusion", 1), ("diffusion", 20), ("diffusion", 60), ("spread", 20),
+                                                 ("spread", 34)])
+def test_masked_products_match_the_oracle(require_gpu, operator, per_column):
+    from scipy import sparse
+
+    from oracle import adjoint_oracle
+    from parallellocallyoptimalapproximatesparsematrixinverses_b200 import adjoint
+    if operator == "diffusion":
+        A = problems.diffusion_2d(45, 1.0, 3)
+    else:
+        A = problems.random_banded_spd(40_000, half_width=1, extra=1, seed=2)
+    n = A.shape[0]
+    rng = np.random.default_rng(per_column)
+    cols = np.repeat(np.arange(n), per_column)
+    rows = (cols + rng.integers(-40, 41, cols.size)) % n if operator == "diffusion" else rng.integers(0, n, cols.size)
+    M = sparse.csc_matrix(sparse.coo_matrix((rng.standard_normal(cols.size), (rows, cols)), shape=(n, n)))
+    M.sum_duplicates()
+    M.sort_indices()
+    loss, grad_m, grad_a = adjoint.residual_adjoint(A, M)
+    want_loss, want_m, want_a = adjoint_oracle.residual_adjoint(A, M)
+    assert loss == want_loss
+    assert np.array_equal(grad_m.data.view(np.int64), want_m.view(np.int64))
+    assert np.array_equal(grad_a.data.view(np.int64), want_a.view(np.int64))
