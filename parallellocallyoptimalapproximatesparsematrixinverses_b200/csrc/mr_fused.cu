@@ -115,6 +115,7 @@ struct FusedArgs {
   double* tt;          // per-column ||Pr A Z(:, j)||^2
   double* bt;          // per-column <Z(:, j), Pr A Z(:, j)>
   double* chunk;       // 3 * chunks
+  const double* alpha; // step length of every column (batched runs), or null: state->alpha
   FusedRow* history;   // max_iterations + 1 rows
   FusedState* state;
 };
@@ -362,7 +363,7 @@ __device__ __noinline__ int DropColumn(const FusedArgs<T>& a, unsigned char* bas
   FusedState* state = a.state;
   const int64_t parity = state->parity;
   const int64_t other = parity ^ 1;
-  const T alpha = static_cast<T>(state->alpha);
+  const T alpha = static_cast<T>(a.alpha != nullptr ? a.alpha[j] : state->alpha);
   int overflow = 0;
   __syncwarp();
   {
@@ -658,7 +659,7 @@ struct HeldSlots {
 
 // False when the group does not fit (nothing written): its columns go one by one.
 template <class T, int kEll, int C>
-__device__ __forceinline__ bool DropGroup(const FusedArgs<T>& a, unsigned char* base, int64_t j0, T alpha,
+__device__ __forceinline__ bool DropGroup(const FusedArgs<T>& a, unsigned char* base, int64_t j0, T step,
                                           int64_t parity, int lane, unsigned long long* written, int* overflow) {
   constexpr int kLanes = kWarp / C;  // lanes of one column
   RowWindow w = WindowAt(base, a.words, static_cast<int32_t>(j0) - a.words * 16);
@@ -799,6 +800,7 @@ __device__ __forceinline__ bool DropGroup(const FusedArgs<T>& a, unsigned char* 
   // U(:, j): M, then + alpha Z
   m_list.Entries([&](int32_t i, T v) { own[w.Rank(i)].v[c] = v; });
   __syncwarp();
+  const T alpha = a.alpha != nullptr && valid ? static_cast<T>(a.alpha[j]) : step;
   z_list.Entries([&](int32_t i, T v) {
     T& u = own[w.Rank(i)].v[c];
     u = Add(u, Mul(alpha, v));
@@ -840,8 +842,12 @@ __device__ __forceinline__ bool DropGroup(const FusedArgs<T>& a, unsigned char* 
   }
   // alpha Z(j, :) = alpha pr_j (e_j - that), then + M(j, :)
   T pr[C];
+  T steps[C];
 #pragma unroll
-  for (int q = 0; q < C; ++q) pr[q] = j0 + q < a.n ? a.pr[j0 + q] : T(0);
+  for (int q = 0; q < C; ++q) {
+    pr[q] = j0 + q < a.n ? a.pr[j0 + q] : T(0);
+    steps[q] = __shfl_sync(0xffffffffu, alpha, q * kLanes);
+  }
 #pragma unroll 1
   for (int r = lane; r < count; r += kWarp) {
     const int64_t i = static_cast<int64_t>(w.lo) + rows[r];
@@ -850,7 +856,7 @@ __device__ __forceinline__ bool DropGroup(const FusedArgs<T>& a, unsigned char* 
     for (int q = 0; q < C; ++q) {
       T rv = -t.v[q];
       if (i == j0 + q) rv = Add(rv, T(1));
-      t.v[q] = rv == T(0) ? T(0) : Mul(alpha, Mul(pr[q], rv));
+      t.v[q] = rv == T(0) ? T(0) : Mul(steps[q], Mul(pr[q], rv));
     }
     trans[r] = t;
   }
@@ -1557,6 +1563,37 @@ __global__ void ToSlotsKernel(CscView<T> x, int cap, int32_t* __restrict__ rows,
   if (overflow != 0) atomicOr(&state->overflow, overflow);
 }
 
+// A batched step is over: the M^T sets change places (the decide kernel's part in single runs).
+__global__ void FlipKernel(FusedState* __restrict__ state) { state->parity ^= 1; }
+
+// out[s] = the entries of M and out[count + s] those of Z in the columns [first[s], first[s + 1]); a block each.
+__global__ void SegmentCountsKernel(const int32_t* __restrict__ m_cnt, const int32_t* __restrict__ z_cnt,
+                                    const int64_t* __restrict__ first, int64_t count, int64_t* __restrict__ out) {
+  __shared__ unsigned long long total[2];
+  for (int64_t s = blockIdx.x; s < count; s += gridDim.x) {
+    if (threadIdx.x < 2) total[threadIdx.x] = 0ull;
+    __syncthreads();
+    unsigned long long m = 0ull;
+    unsigned long long z = 0ull;
+    for (int64_t j = first[s] + threadIdx.x; j < first[s + 1]; j += blockDim.x) {
+      m += static_cast<unsigned long long>(m_cnt[j]);
+      z += static_cast<unsigned long long>(z_cnt[j]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      m += __shfl_xor_sync(0xffffffffu, m, o);
+      z += __shfl_xor_sync(0xffffffffu, z, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+      atomicAdd(&total[0], m);
+      atomicAdd(&total[1], z);
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) out[threadIdx.x * count + s] = static_cast<int64_t>(total[threadIdx.x]);
+    __syncthreads();
+  }
+}
+
 __global__ void WidenCountsKernel(const int32_t* __restrict__ cnt, int64_t n, int64_t* __restrict__ out) {
   for (int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; j < n;
        j += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -1613,24 +1650,8 @@ class FusedMr final : public FusedMrBase {
     if (!FusedMrApplicable(problem)) return outcome;
     auto& m = *static_cast<DevCsc<T>*>(m_csc);
     const auto& z = *static_cast<const DevCsc<T>*>(z_csc);
-    const int64_t n = problem.n;
-    Reserve(ctx, problem);
-    Configure(problem);
     const cudaStream_t st = ctx.stream;
-    // state: iteration 0 is in the history; M^T set 0 is filled below
-    FusedState init{};
-    init.alpha = alpha;
-    init.nnz_dir = static_cast<unsigned long long>(z.nnz);
-    *host_state_ = init;
-    SPAI_CUDA(cudaMemcpyAsync(state_.data(), host_state_, sizeof(FusedState), cudaMemcpyHostToDevice, st));
-    for (int s = 0; s < 2; ++s) SPAI_CUDA(cudaMemsetAsync(mt_cnt_[s].data(), 0, sizeof(int32_t) * n, st));
-    const int grid = GridFor(n, 128);
-    ToSlotsKernel<T><<<grid, 128, 0, st>>>(View(m), args_.topk, args_.m_rows, args_.m_vals, args_.m_cnt, args_.cap_mt,
-                                           args_.mt_cols[0], args_.mt_vals[0], args_.mt_cnt[0], args_.state);
-    SPAI_LAUNCH_CHECK();
-    ToSlotsKernel<T><<<grid, 128, 0, st>>>(View(z), args_.cap_z, args_.z_rows, args_.z_vals, args_.z_cnt, 0,
-                                           nullptr, nullptr, nullptr, args_.state);
-    SPAI_LAUNCH_CHECK();
+    Start(ctx, problem, m, z, alpha, nullptr);
     FusedState out;
     if (prof::Enabled()) {
       out = RunStepwise(ctx, problem, m.nnz, z.nnz);
@@ -1655,18 +1676,7 @@ class FusedMr final : public FusedMrBase {
     std::vector<FusedRow> host_rows(static_cast<size_t>(rows + 1));
     SPAI_CUDA(cudaMemcpyAsync(host_rows.data(), args_.history, sizeof(FusedRow) * (rows + 1), cudaMemcpyDeviceToHost,
                               st));
-    // M back to compact CSC
-    DevCsc<T> result;
-    result.Shape(n, n, st);
-    ctx.counts.Reserve(static_cast<size_t>(n + 1), st);
-    WidenCountsKernel<<<GridFor(n, 256), 256, 0, st>>>(args_.m_cnt, n, ctx.counts.data());
-    SPAI_LAUNCH_CHECK();
-    const int64_t nnz = ScanCounts(ctx, ctx.counts.data(), n, result.ptr.data());
-    result.ReserveNnz(nnz, st);
-    FromSlotsKernel<T><<<grid, 128, 0, st>>>(n, args_.topk, args_.m_rows, args_.m_vals, result.ptr.data(),
-                                             result.idx.data(), result.val.data());
-    SPAI_LAUNCH_CHECK();
-    m.Swap(result);
+    CompactM(ctx, m);
     ctx.Sync();
     for (int64_t r = 1; r <= rows; ++r) {
       SingleIterationData row;
@@ -1681,7 +1691,84 @@ class FusedMr final : public FusedMrBase {
     return outcome;
   }
 
+  bool BeginBatch(Ctx& ctx, const FusedMrProblem& problem, const void* m_csc, const void* z_csc,
+                  const double* alpha) override {
+    if (!FusedMrApplicable(problem)) return false;
+    Start(ctx, problem, *static_cast<const DevCsc<T>*>(m_csc), *static_cast<const DevCsc<T>*>(z_csc), 0.0, alpha);
+    return true;
+  }
+
+  FusedBatchSums StepBatch(Ctx& ctx) override {
+    const cudaStream_t st = ctx.stream;
+    {
+      prof::Scope scope(st, "fused_drop", 0.0);
+      drop_kernel_<<<drop_grid_, kGroupWarps * kWarp, drop_smem_, st>>>(args_);
+      SPAI_LAUNCH_CHECK();
+    }
+    {
+      prof::Scope scope(st, "fused_residual", 0.0);
+      res_kernel_<<<res_grid_, kGroupWarps * kWarp, res_smem_, st>>>(args_);
+      SPAI_LAUNCH_CHECK();
+    }
+    FlipKernel<<<1, 1, 0, st>>>(args_.state);
+    SPAI_LAUNCH_CHECK();
+    return FusedBatchSums{args_.sq, args_.bt, args_.tt};
+  }
+
+  bool BatchCounts(Ctx& ctx, const int64_t* first, int64_t segments, int64_t* out_dev, int64_t* out) override {
+    const cudaStream_t st = ctx.stream;
+    SegmentCountsKernel<<<static_cast<unsigned>(std::min<int64_t>(segments, 65535)), 256, 0, st>>>(
+        args_.m_cnt, args_.z_cnt, first, segments, out_dev);
+    SPAI_LAUNCH_CHECK();
+    SPAI_CUDA(cudaMemcpyAsync(host_state_, state_.data(), sizeof(FusedState), cudaMemcpyDeviceToHost, st));
+    SPAI_CUDA(cudaMemcpyAsync(out, out_dev, sizeof(int64_t) * 2 * segments, cudaMemcpyDeviceToHost, st));
+    ctx.Sync();
+    return host_state_->overflow == 0;
+  }
+
+  void CompactBatch(Ctx& ctx, void* m_csc) override { CompactM(ctx, *static_cast<DevCsc<T>*>(m_csc)); }
+
  private:
+  // The slots filled from M and Z, the state at iteration 0 (M^T set 0 current).
+  void Start(Ctx& ctx, const FusedMrProblem& problem, const DevCsc<T>& m, const DevCsc<T>& z, double alpha,
+             const double* alpha_columns) {
+    const cudaStream_t st = ctx.stream;
+    const int64_t n = problem.n;
+    Reserve(ctx, problem);
+    Configure(problem);
+    args_.alpha = alpha_columns;
+    FusedState init{};
+    init.alpha = alpha;
+    init.nnz_dir = static_cast<unsigned long long>(z.nnz);
+    *host_state_ = init;
+    SPAI_CUDA(cudaMemcpyAsync(state_.data(), host_state_, sizeof(FusedState), cudaMemcpyHostToDevice, st));
+    for (int s = 0; s < 2; ++s) SPAI_CUDA(cudaMemsetAsync(mt_cnt_[s].data(), 0, sizeof(int32_t) * n, st));
+    const int grid = GridFor(n, 128);
+    ToSlotsKernel<T><<<grid, 128, 0, st>>>(View(m), args_.topk, args_.m_rows, args_.m_vals, args_.m_cnt, args_.cap_mt,
+                                           args_.mt_cols[0], args_.mt_vals[0], args_.mt_cnt[0], args_.state);
+    SPAI_LAUNCH_CHECK();
+    ToSlotsKernel<T><<<grid, 128, 0, st>>>(View(z), args_.cap_z, args_.z_rows, args_.z_vals, args_.z_cnt, 0,
+                                           nullptr, nullptr, nullptr, args_.state);
+    SPAI_LAUNCH_CHECK();
+  }
+
+  // M back to compact CSC.
+  void CompactM(Ctx& ctx, DevCsc<T>& m) {
+    const cudaStream_t st = ctx.stream;
+    const int64_t n = args_.n;
+    DevCsc<T> result;
+    result.Shape(n, n, st);
+    ctx.counts.Reserve(static_cast<size_t>(n + 1), st);
+    WidenCountsKernel<<<GridFor(n, 256), 256, 0, st>>>(args_.m_cnt, n, ctx.counts.data());
+    SPAI_LAUNCH_CHECK();
+    const int64_t nnz = ScanCounts(ctx, ctx.counts.data(), n, result.ptr.data());
+    result.ReserveNnz(nnz, st);
+    FromSlotsKernel<T><<<GridFor(n, 128), 128, 0, st>>>(n, args_.topk, args_.m_rows, args_.m_vals, result.ptr.data(),
+                                                        result.idx.data(), result.val.data());
+    SPAI_LAUNCH_CHECK();
+    m.Swap(result);
+  }
+
   // The same three kernels launched one by one with the library's CUDA-event
   // accounting around each (spai_profile_enable): the decide kernel's result
   // is read back after every iteration, in place of the graph's condition.
@@ -1805,7 +1892,7 @@ class FusedMr final : public FusedMrBase {
                 x.a_rows_ell_val == y.a_rows_ell_val && x.pr == y.pr && x.m_rows == y.m_rows &&
                 x.m_vals == y.m_vals && x.m_cnt == y.m_cnt && x.z_rows == y.z_rows && x.z_vals == y.z_vals &&
                 x.z_cnt == y.z_cnt &&
-                x.sq == y.sq && x.tt == y.tt && x.bt == y.bt && x.chunk == y.chunk && x.history == y.history &&
+                x.alpha == y.alpha && x.sq == y.sq && x.tt == y.tt && x.bt == y.bt && x.chunk == y.chunk && x.history == y.history &&
                 x.state == y.state;
     for (int s = 0; s < 2; ++s) {
       same = same && x.mt_cols[s] == y.mt_cols[s] && x.mt_vals[s] == y.mt_vals[s] && x.mt_cnt[s] == y.mt_cnt[s];

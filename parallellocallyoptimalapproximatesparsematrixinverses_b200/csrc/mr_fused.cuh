@@ -61,6 +61,13 @@ struct FusedMrOutcome {
   int64_t graph_bodies = 0;
 };
 
+// Per-column sums a batched step leaves on the device: ||R||^2, <Z, Pr A Z> and ||Pr A Z||^2.
+struct FusedBatchSums {
+  const double* residual;
+  const double* num;
+  const double* den;
+};
+
 class FusedMrBase {
  public:
   virtual ~FusedMrBase() = default;
@@ -69,6 +76,18 @@ class FusedMrBase {
   // 1.. to `history` and replaces m with the final M.
   virtual FusedMrOutcome Run(Ctx& ctx, const FusedMrProblem& problem, void* m_csc, const void* z_csc, double alpha,
                              std::vector<SingleIterationData>& history) = 0;
+
+  // Batched Global MR on a block-diagonal problem, one step per call with the
+  // step length of every column in `alpha` (device, n doubles, read by every
+  // step): BeginBatch fills the slots (false: not applicable, nothing
+  // changed), StepBatch runs the drop and residual kernels, BatchCounts
+  // fetches the entries of M, then of Z, per segment of columns and returns
+  // false when a column outgrew its slots, CompactBatch writes M.
+  virtual bool BeginBatch(Ctx& ctx, const FusedMrProblem& problem, const void* m_csc, const void* z_csc,
+                          const double* alpha) = 0;
+  virtual FusedBatchSums StepBatch(Ctx& ctx) = 0;
+  virtual bool BatchCounts(Ctx& ctx, const int64_t* first, int64_t segments, int64_t* out_dev, int64_t* out) = 0;
+  virtual void CompactBatch(Ctx& ctx, void* m_csc) = 0;
 };
 
 // Whether the fused loop can take the problem (slot and window capacities).

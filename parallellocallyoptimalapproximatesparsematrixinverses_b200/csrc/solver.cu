@@ -414,7 +414,15 @@ class Solver final : public SolverBase {
   // (SegmentTree).  A block that stops (converged, density limit, breakdown,
   // iteration limit) has its M copied out at that moment; afterwards it rides
   // along with step length 0 and its results are no longer read.
+  // With per-column top-k the steps run on the fused kernels (mr_fused.cu) where
+  // those apply, with a step length per column; a column that outgrows their
+  // slots sends the whole batch through the unfused ones, which give the same bits.
   void RunMrBatched(const std::vector<int64_t>& offsets, std::vector<SolveOutput>& outputs) override {
+    if (!RunBatch(offsets, outputs, true)) RunBatch(offsets, outputs, false);
+  }
+
+  // False when the fused steps had to be given up (outputs are then incomplete).
+  bool RunBatch(const std::vector<int64_t>& offsets, std::vector<SolveOutput>& outputs, bool allow_fused) {
     const int64_t blocks = static_cast<int64_t>(offsets.size()) - 1;
     if (blocks <= 0 || offsets.front() != 0 || offsets.back() != n_) throw std::invalid_argument("bad block offsets");
     if (!pr_diagonal_) throw std::invalid_argument("batched runs use a diagonal Pr");
@@ -448,6 +456,10 @@ class Solver final : public SolverBase {
     std::vector<int64_t> z_at(static_cast<size_t>(blocks + 1));
     std::vector<int> stopping;
 
+    bool fused = false;                   // the iterate lives in the fused slots
+    std::vector<int64_t> slot_counts;     // their entries of M and Z per block
+    std::vector<int64_t> direction(static_cast<size_t>(blocks), 0);  // entries of the Z a step used
+
     // nnz of M and Z per block: their column offsets at the block boundaries
     auto fetch_counts = [&]() {
       const int g = GridFor(blocks + 1, 128);
@@ -473,6 +485,7 @@ class Solver final : public SolverBase {
     // M of every block in `stopping` to its output (local indices, FP64 values)
     auto snapshot = [&]() {
       if (stopping.empty()) return;
+      if (fused) fused_->CompactBatch(ctx_, &m_);
       fetch_counts();
       for (const int b : stopping) {
         SolveOutput& out = outputs[b];
@@ -493,18 +506,20 @@ class Solver final : public SolverBase {
     };
     // AppendIteration (result_operations.cpp:53-67) for every live block
     auto append = [&](const std::vector<double>& residual) {
-      fetch_counts();
+      if (!fused) fetch_counts();
       for (int64_t b = 0; b < blocks; ++b) {
         if (!active[b]) continue;
         SolveOutput& out = outputs[b];
         const double nb = static_cast<double>(offsets[b + 1] - offsets[b]);
         const double entries = nb * nb;
+        const int64_t m_entries = fused ? slot_counts[b] : m_at[b + 1] - m_at[b];
+        const int64_t z_entries = fused ? direction[b] : z_at[b + 1] - z_at[b];
         SingleIterationData row;
         row.iteration = static_cast<int64_t>(out.history.size());
         out.iterations = row.iteration;
         row.residual_norm = residual[b];
-        row.density_m = static_cast<double>(m_at[b + 1] - m_at[b]) / entries;
-        row.density_direction = static_cast<double>(z_at[b + 1] - z_at[b]) / entries;
+        row.density_m = static_cast<double>(m_entries) / entries;
+        row.density_direction = static_cast<double>(z_entries) / entries;
         out.history.push_back(row);
         if (row.residual_norm < opt_.tolerance) {
           out.converged = true;
@@ -552,6 +567,16 @@ class Solver final : public SolverBase {
     if (live > 0) projection();
     std::vector<double> alpha(static_cast<size_t>(blocks));
     DevCsc<T> scaled;
+    DevBuf<int64_t> counts_dev;
+    std::vector<double> three(static_cast<size_t>(3 * blocks));
+    if (live > 0 && allow_fused && FusedMrEnabled() && opt_.dropping && opt_.topk > 0 && ell_width_ > 0) {
+      if (!fused_) fused_ = MakeFusedMr<T>();
+      for (int64_t b = 0; b < blocks; ++b) direction[b] = z_at[b + 1] - z_at[b];
+      const FusedMrProblem problem = FusedProblem();
+      fused = fused_->BeginBatch(ctx_, problem, &m_, &z_, ColVec(0));
+      slot_counts.resize(static_cast<size_t>(2 * blocks));
+      counts_dev.Reserve(static_cast<size_t>(2 * blocks), ctx_.stream);
+    }
     for (int64_t i = 1; i <= opt_.max_iterations && live > 0; ++i) {
       for (int64_t b = 0; b < blocks; ++b) {
         alpha[b] = 0.0;
@@ -573,6 +598,20 @@ class Solver final : public SolverBase {
       BroadcastBlocksKernel<<<GridFor(n_, 256), 256, 0, ctx_.stream>>>(block_of_dev.data(), alpha_dev.data(), n_,
                                                                       alpha_col);
       SPAI_LAUNCH_CHECK();
+      if (fused) {
+        const FusedBatchSums step = fused_->StepBatch(ctx_);
+        const double* parts[3] = {step.residual, step.num, step.den};
+        tree.Sums(ctx_, parts, 3, three.data());
+        if (!fused_->BatchCounts(ctx_, bounds_dev.data(), blocks, counts_dev.data(), slot_counts.data())) return false;
+        for (int64_t b = 0; b < blocks; ++b) {
+          residual[b] = std::sqrt(three[b]);
+          num[b] = three[blocks + b];
+          den[b] = three[2 * blocks + b];
+        }
+        append(residual);
+        for (int64_t b = 0; b < blocks; ++b) direction[b] = slot_counts[blocks + b];
+        continue;
+      }
       Copy(ctx_, z_, scaled);
       ScaleColumns(ctx_, scaled, alpha_col);
       Union(ctx_, m_, false, 1.0, scaled, 1.0, m_, UnionMode::kAxpby);
@@ -588,6 +627,7 @@ class Solver final : public SolverBase {
     }
     snapshot();
     ctx_.Sync();
+    return true;
   }
 
   int64_t iterations() const override { return iterations_; }
@@ -1048,21 +1088,7 @@ class Solver final : public SolverBase {
       if (opt_.max_iterations < 1 || !FiniteNonZeroHost(den)) return;
       const double alpha = num / den;
       if (!std::isfinite(alpha)) return;
-      FusedMrProblem problem;
-      problem.n = n_;
-      problem.topk = static_cast<int>(opt_.topk);
-      problem.a_nnz = a64_.nnz;
-      problem.a_longest = a_longest_;
-      problem.ell_width = ell_width_;
-      problem.a_cols_ell = a_cols_ell_.data();
-      problem.a_rows_ell = a_rows_ell_.data();
-      problem.a_rows_ell_val = a_rows_ell_val_.data();
-      problem.pr = pr_vec_.data();
-      MeasureA();
-      problem.bandwidth = a_bandwidth_;
-      problem.finite = a_finite_;
-      problem.max_iterations = opt_.max_iterations;
-      problem.tolerance = opt_.tolerance;
+      const FusedMrProblem problem = FusedProblem();
       if (FusedMrApplicable(problem)) {
         if (!fused_) fused_ = MakeFusedMr<T>();
         const FusedMrOutcome outcome = fused_->Run(ctx_, problem, &m_, &z_, alpha, history_);
@@ -1227,6 +1253,25 @@ class Solver final : public SolverBase {
         if (AppendIteration(p_)) return;
       }
     }
+  }
+
+  FusedMrProblem FusedProblem() {
+    MeasureA();
+    FusedMrProblem problem;
+    problem.n = n_;
+    problem.topk = static_cast<int>(opt_.topk);
+    problem.a_nnz = a64_.nnz;
+    problem.a_longest = a_longest_;
+    problem.ell_width = ell_width_;
+    problem.a_cols_ell = a_cols_ell_.data();
+    problem.a_rows_ell = a_rows_ell_.data();
+    problem.a_rows_ell_val = a_rows_ell_val_.data();
+    problem.pr = pr_vec_.data();
+    problem.bandwidth = a_bandwidth_;
+    problem.finite = a_finite_;
+    problem.max_iterations = opt_.max_iterations;
+    problem.tolerance = opt_.tolerance;
+    return problem;
   }
 
   // A's bandwidth and whether A and Pr are finite, once per problem.
