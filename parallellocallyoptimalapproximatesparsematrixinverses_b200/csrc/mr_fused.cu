@@ -704,7 +704,7 @@ __device__ __forceinline__ bool DropGroup(const FusedArgs<T>& a, unsigned char* 
   HeldSlots<T, kLanes, 32 / kLanes> mt_list(mt_all + j * a.cap_mt, mt_vals + j * a.cap_mt, nmt, s);
   // the first entries of the rows k of M, k in row j of A (rows of M^T), for operators of up to eight
   // entries a row; the others are read where they are used
-  constexpr bool kRowsHeld = kEll <= 8;
+  constexpr bool kRowsHeld = kEll <= 8 && C == 4;  // in groups of two (small problems) fetching the code costs more
   constexpr int kPer = kRowsHeld ? 24 / kLanes + (24 % kLanes != 0 ? 1 : 0) : 1;  // at least 24 entries of each
   constexpr int kRows = kRowsHeld ? kEll : 1;
   int32_t r_row[kRows][kPer];

@@ -881,9 +881,11 @@ class Solver final : public SolverBase {
       OrderedDots(ctx_, *x, *y, batch_first_dev_.data(), count, batch_sums_.data());
     }
     std::vector<double> out(static_cast<size_t>(count));
-    SPAI_CUDA(cudaMemcpyAsync(out.data(), batch_sums_.data(), sizeof(double) * count, cudaMemcpyDeviceToHost,
-                              ctx_.stream));
+    // through the pinned scalars while they hold the batches: a copy to pageable memory waits twice
+    double* host = count <= Ctx::kScalarSlots ? ctx_.host_scalars : out.data();
+    SPAI_CUDA(cudaMemcpyAsync(host, batch_sums_.data(), sizeof(double) * count, cudaMemcpyDeviceToHost, ctx_.stream));
     ctx_.Sync();
+    if (host != out.data()) std::copy(host, host + count, out.begin());
     return out;
   }
 

@@ -27,6 +27,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <cstring>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -1194,9 +1195,12 @@ bool Spgemm(Ctx& ctx, const DevCsc<T>& x_csc, const DevCsc<T>& x_csr, const DevC
                                                                    ctx.sg_win_lo.data(), ctx.sg_win_words.data(),
                                                                    ctx.sg_bin_cols.data(), ctx.sg_maxima.data());
   SPAI_LAUNCH_CHECK();
+  static_assert(kMaximaSlots <= Ctx::kScalarSlots, "the maxima fit the pinned scalars");
   unsigned long long host_max[kMaximaSlots];
-  SPAI_CUDA(cudaMemcpyAsync(host_max, ctx.sg_maxima.data(), sizeof(host_max), cudaMemcpyDeviceToHost, ctx.stream));
+  SPAI_CUDA(cudaMemcpyAsync(ctx.host_scalars, ctx.sg_maxima.data(), sizeof(host_max), cudaMemcpyDeviceToHost,
+                            ctx.stream));
   ctx.Sync();
+  std::memcpy(host_max, ctx.host_scalars, sizeof(host_max));
 
   const int64_t max_u = static_cast<int64_t>(host_max[kMaxUb]);
   const int64_t max_nb = static_cast<int64_t>(host_max[kMaxNb]);

@@ -82,11 +82,11 @@ def matrix_data(csc) -> _lib.MatrixData:
 
 
 def history_array(rows, count) -> np.ndarray:
-    history = np.empty(count, dtype=HISTORY_DTYPE)
-    for i in range(count):
-        h = rows[i]
-        history[i] = (h.iteration, h.residual_norm, h.density_m, h.density_direction)
-    return history
+    # SingleIterationData and HISTORY_DTYPE have one layout: an int64 and three doubles
+    if count == 0:
+        return np.empty(0, dtype=HISTORY_DTYPE)
+    size = count * ctypes.sizeof(_lib.SingleIterationData)
+    return np.frombuffer(ctypes.string_at(ctypes.addressof(rows[0]), size), dtype=HISTORY_DTYPE).copy()
 
 
 class _LibraryArray:
@@ -349,9 +349,14 @@ class Session:
         return it.value, nnz.value
 
     def history(self):
-        cap = 1 << 16
+        # a small buffer first: the returned count is the history's length, whatever fits
+        cap = 256
         rows = (_lib.SingleIterationData * cap)()
         count = self._lib.spai_session_history(self._handle, rows, cap)
+        if count > cap:
+            cap = min(count, 1 << 16)
+            rows = (_lib.SingleIterationData * cap)()
+            count = self._lib.spai_session_history(self._handle, rows, cap)
         return history_array(rows, min(count, cap))
 
     def result(self) -> OutputResult:
