@@ -78,3 +78,32 @@ def test_groups_match_the_unfused_kernels(require_gpu, case, precision):
         lib.spai_set_fused_mr(1)
     got = global_spai.mr(a, **kw)
     assert_same_result(got, want, f"{case} {precision}")
+
+
+def _star(n_hubs, leaves):
+    """Hubs of `leaves` neighbours: rows of M^T longer than a small cap's slots."""
+    n = n_hubs * (leaves + 1)
+    hub = np.repeat(np.arange(n_hubs) * (leaves + 1), leaves)
+    leaf = hub + np.tile(np.arange(1, leaves + 1), n_hubs)
+    return _spd(n, lambda rng: (hub, leaf), seed=1)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("systems", ["grids", "slots_outgrown"])
+def test_batched_steps_match_the_unfused_kernels(require_gpu, systems, precision):
+    if systems == "grids":  # groups straddle systems of odd sizes; several stop early
+        batch = [problems.diffusion_2d(m, 0.5, m) for m in (3, 17, 31)] + [problems.diffusion_3d(9, 1.0, 1),
+                                                                           problems.tridiagonal(5)]
+        kw = dict(max_iterations=12, tolerance=0.3, max_density=1.0, topk_per_column=7, precision=precision)
+    else:  # the fused steps are given up and the whole batch runs unfused
+        batch = [_star(9, 14), problems.diffusion_2d(12, 0.5, 2)]
+        kw = dict(max_iterations=6, tolerance=0.0, max_density=1.0, topk_per_column=2, precision=precision)
+    lib = _lib.load()
+    lib.spai_set_fused_mr(0)
+    try:
+        want = global_spai.mr_batched(batch, **kw)
+    finally:
+        lib.spai_set_fused_mr(1)
+    got = global_spai.mr_batched(batch, **kw)
+    for b, (g, w) in enumerate(zip(got, want)):
+        assert_same_result(g, w, f"{systems} {precision} system {b}")
