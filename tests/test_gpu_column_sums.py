@@ -4,6 +4,7 @@ entry to about a thousand, equal and different patterns, ties at the cut (the
 Laplacian's repeated magnitudes), caps of one entry and of more than a warp."""
 import numpy as np
 import pytest
+from scipy import sparse
 
 from oracle import pyoracle
 from parallellocallyoptimalapproximatesparsematrixinverses_b200 import global_spai, inner_outer, problems
@@ -11,7 +12,19 @@ from tests.helpers import assert_same_result
 
 pytestmark = pytest.mark.gpu
 
+
+
+def arrow(n):
+    """Columns of two entries beside one of n: staged rows up to 256, longer ones read in place."""
+    a = sparse.lil_matrix((n, n))
+    a[-1, :] = a[:, -1] = -0.25 + np.arange(n) / (16.0 * n)
+    a.setdiag(n)
+    return sparse.csc_matrix(a)
+
+
 OPERATORS = {
+    "arrow_256": lambda: arrow(256),
+    "arrow_257": lambda: arrow(257),
     "tridiagonal_6": lambda: problems.tridiagonal(6),
     "laplacian_33": lambda: problems.laplacian_2d(33),
     "diffusion_3d_9": lambda: problems.diffusion_3d(9, 1.0, 2),
