@@ -34,7 +34,8 @@
 // until the end, so that no square root or division is on the way to the next
 // iteration unless the stop test is close.
 //
-// What bounds it: while every cluster owns one chunk (about 70,000 rows) the
+// What bounds it: while every cluster owns one chunk (61,440 rows on the 15
+// clusters of a B200 that fit one block per SM) the
 // latency of an iteration's two reductions and gathers; the rows of both
 // matrices then stay in shared memory for the whole solve where they fit.
 // Beyond, the L2 reads of the two matrices and the gathers; the matrices are
