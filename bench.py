@@ -349,7 +349,7 @@ def run_ours(args):
             },
             "graph": {"spai_iterations": "one CUDA graph launch per build: WHILE node over the fused drop, "
                                          "residual/projection and decide kernels (mr_fused.cu)",
-                      "pcg": "one CUDA graph launch per solve: WHILE node over the PCG iteration (pcg.cu)"},
+                      "pcg": "one cooperative kernel per solve (pcg.cu)"},
             "mixed_error": mixed_error,
             "kernel_classes_mixed": kernel_table,
             "clocks": clocks.summary(),
@@ -372,11 +372,11 @@ def run_ours(args):
 
 
 KERNEL_NOTES = {
-    "fused_residual": "fused_residual (FusedResidualKernel, one warp per column: R = I - A M, Z = Pr R written "
-                      "with its transpose, ||R(:,j)||^2, then the MR projection of A Z from the Z column in "
-                      "shared memory)",
-    "fused_drop": "fused_drop (FusedDropKernel, one warp per column: 0.5 (U + U^T) with U = M + alpha Z formed "
-                  "from M, Z and their transposes, threshold and top-k)",
+    "fused_residual": "fused_residual (FusedResidualKernel, one warp per group of adjacent columns: R = I - A M, "
+                      "Z = Pr R written, ||R(:,j)||^2, then the MR projection of A Z from the Z columns in shared "
+                      "memory)",
+    "fused_drop": "fused_drop (FusedDropKernel, one warp per group of adjacent columns: 0.5 (U + U^T) with "
+                  "U = M + alpha Z formed from M, M^T, Z and the rows of A, threshold and top-k)",
     "spgemm_numeric": "spgemm_numeric (ColumnProductKernel: R = I - A M with Z and the column sums fused, and the "
                       "MR projection of A Z)",
 }
