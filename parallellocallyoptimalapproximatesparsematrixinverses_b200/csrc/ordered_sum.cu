@@ -214,6 +214,9 @@ __global__ void __cluster_dims__(kSumBlocks, 1, 1) __launch_bounds__(kSumBlockTh
     const double v = static_cast<double>(val[p]);
     return kSquares ? Mul(v, v) : v;
   };
+  // A block's shared memory may be written from outside only once that block runs; each later round's stores
+  // follow a cluster barrier of the round before.
+  cluster.sync();
   for (int64_t b = blockIdx.x / kSumBlocks; b < batches; b += gridDim.x / kSumBlocks) {
     const int64_t begin = ptr[first[b]];
     const int64_t end = ptr[first[b + 1]];
