@@ -35,7 +35,8 @@ void CountLaunches(int64_t count);
 
 namespace {
 
-constexpr int kGroupWarps = 2;      // warps per block of the drop and residual kernels
+constexpr int kGroupWarps = 2;      // warps per block of the drop and residual kernels on column groups
+constexpr int kColumnWarps = 4;     // and of those that go column by column
 constexpr int kDropWindowWords = 512;  // bitmap words of a drop column on its own: windows of 16,384 rows
 constexpr int kDropWindowRows = kDropWindowWords * 32;
 constexpr int kWindowWords = 1024;  // bitmap words of a residual column on its own: windows of 32,768 rows
@@ -175,10 +176,13 @@ __device__ __forceinline__ int FindSlot(const int32_t* keys, int bits, int32_t k
 constexpr int kMtPerLane = 4;
 static_assert(4 * kMaxTopK <= kMtPerLane * kWarp, "a row of M^T must fit the lanes' registers");
 
+// 32-row words of the bitmaps' summaries, in whole warps.
+constexpr int kDropSummary = (kDropWindowWords + kWarp * kWarp - 1) / (kWarp * kWarp) * kWarp;
+constexpr int kResidualSummary = (kWindowWords + kWarp * kWarp - 1) / (kWarp * kWarp) * kWarp;
+
 template <class T>
 __host__ __device__ size_t DropWarpBytes(int own, int mt, int r) {
-  constexpr int kSummary = (kDropWindowWords + kWarp * kWarp - 1) / (kWarp * kWarp) * kWarp;
-  return Round16(static_cast<size_t>(kDropWindowWords) * 4) + Round16(static_cast<size_t>(kSummary) * 4) +
+  return Round16(static_cast<size_t>(kDropWindowWords) * 4) + Round16(static_cast<size_t>(kDropSummary) * 4) +
          Round16(static_cast<size_t>(kDropRowsCap) * 2) +
          Round16(static_cast<size_t>(mt + r) * 4) + Round16(static_cast<size_t>(mt + r) * sizeof(T)) +
          Round16(static_cast<size_t>(own) * 4) + Round16(static_cast<size_t>(own) * sizeof(T)) +
@@ -323,49 +327,86 @@ __device__ __forceinline__ int DropAndWrite(const FusedArgs<T>& a, Row row_of, c
   return DropAndWriteIn<T, 8>(a, row_of, vals, count, j, other, lane, overflow);
 }
 
-// One column on its own, for columns whose rows do not fit the group's window.
-// Returns the overflow bits; *written grows by the column's entries.
+// A warp's shared memory while it goes column by column, and what holds for all of its columns.
 template <class T>
-__device__ __noinline__ int DropColumn(const FusedArgs<T>& a, unsigned char* base, int64_t j,
-                                       unsigned long long* written_out) {
-  constexpr int kSummary = (kDropWindowWords + kWarp * kWarp - 1) / (kWarp * kWarp) * kWarp;
+struct DropSlab {
+  uint32_t* bm;
+  uint32_t* summary;
+  uint16_t* rows;
+  int32_t* keys;  // the two tables, one after another
+  T* vals;
+  int32_t* mr;  // M(:, j) then Z(:, j): rows
+  T* mv;        // and values
+  T* s_vals;    // the nonzero entries of S(:, j)
+  int32_t* s_rows;
+  int b_mt;
+  int b_r;
+  int64_t parity;
+  T alpha;
+
+  // clear: whether the window has to be cleared.
+  __device__ __forceinline__ DropSlab(const FusedArgs<T>& a, unsigned char* base, bool clear, int lane) {
+    const int table = a.d_mt_slots + a.d_r_slots;
+    const int own = a.topk + a.cap_z;
+    bm = reinterpret_cast<uint32_t*>(base);
+    base += Round16(static_cast<size_t>(kDropWindowWords) * 4);
+    summary = reinterpret_cast<uint32_t*>(base);
+    base += Round16(static_cast<size_t>(kDropSummary) * 4);
+    rows = reinterpret_cast<uint16_t*>(base);
+    base += Round16(static_cast<size_t>(kDropRowsCap) * 2);
+    keys = reinterpret_cast<int32_t*>(base);
+    base += Round16(static_cast<size_t>(table) * 4);
+    vals = reinterpret_cast<T*>(base);
+    base += Round16(static_cast<size_t>(table) * sizeof(T));
+    mr = reinterpret_cast<int32_t*>(base);
+    base += Round16(static_cast<size_t>(own) * 4);
+    mv = reinterpret_cast<T*>(base);
+    base += Round16(static_cast<size_t>(own) * sizeof(T));
+    s_vals = reinterpret_cast<T*>(base);
+    base += Round16(kDropCap * sizeof(T));
+    s_rows = reinterpret_cast<int32_t*>(base);
+    b_mt = Log2(a.d_mt_slots);
+    b_r = Log2(a.d_r_slots);
+    parity = a.state->parity;
+    alpha = static_cast<T>(a.state->alpha);
+    if (clear) {
+      __syncwarp();
+      ClearWords(bm, kDropWindowWords, lane);
+      ClearWords(summary, kDropSummary, lane);
+      __syncwarp();
+    }
+  }
+};
+
+// One column on its own; its window is clear before and after.  Returns the
+// overflow bits; *written grows by the column's entries.  kUnroll: of the short
+// loops; 1 inside the group kernels, whose registers they would raise.
+template <class T, int kUnroll>
+__device__ __forceinline__ int DropColumn(const FusedArgs<T>& a, const DropSlab<T>& slab, int64_t j,
+                                          unsigned long long* written_out) {
   const int lane = threadIdx.x & 31;
   const int table = a.d_mt_slots + a.d_r_slots;
-  const int own = a.topk + a.cap_z;  // M(:, j) and Z(:, j), staged
-  uint32_t* bm = reinterpret_cast<uint32_t*>(base);
-  base += Round16(static_cast<size_t>(kDropWindowWords) * 4);
-  uint32_t* summary = reinterpret_cast<uint32_t*>(base);
-  base += Round16(static_cast<size_t>(kSummary) * 4);
-  uint16_t* rows = reinterpret_cast<uint16_t*>(base);
-  base += Round16(static_cast<size_t>(kDropRowsCap) * 2);
-  int32_t* keys = reinterpret_cast<int32_t*>(base);  // the two tables, one after another
-  base += Round16(static_cast<size_t>(table) * 4);
-  T* vals = reinterpret_cast<T*>(base);
-  base += Round16(static_cast<size_t>(table) * sizeof(T));
-  int32_t* mr = reinterpret_cast<int32_t*>(base);  // M(:, j) then Z(:, j): rows
+  uint32_t* bm = slab.bm;
+  uint32_t* summary = slab.summary;
+  uint16_t* rows = slab.rows;
+  int32_t* keys = slab.keys;
+  int32_t* mr = slab.mr;
   int32_t* zr = mr + a.topk;
-  base += Round16(static_cast<size_t>(own) * 4);
-  T* mv = reinterpret_cast<T*>(base);  // and values
+  T* mv = slab.mv;
   T* zv = mv + a.topk;
-  base += Round16(static_cast<size_t>(own) * sizeof(T));
-  T* s_vals = reinterpret_cast<T*>(base);  // the nonzero entries of S(:, j)
-  base += Round16(kDropCap * sizeof(T));
-  int32_t* s_rows = reinterpret_cast<int32_t*>(base);
+  T* s_vals = slab.s_vals;
+  int32_t* s_rows = slab.s_rows;
   int32_t* k_mt = keys;
   int32_t* k_r = k_mt + a.d_mt_slots;
-  T* v_mt = vals;
+  T* v_mt = slab.vals;
   T* v_r = v_mt + a.d_mt_slots;
-  const int b_mt = Log2(a.d_mt_slots);
-  const int b_r = Log2(a.d_r_slots);
+  const int b_mt = slab.b_mt;
+  const int b_r = slab.b_r;
   const int r_limit = a.d_r_slots / 2;  // distinct keys of R(j, :) the table takes
-  ClearWords(bm, kDropWindowWords, lane);
-  ClearWords(summary, kSummary, lane);
-  FusedState* state = a.state;
-  const int64_t parity = state->parity;
+  const int64_t parity = slab.parity;
   const int64_t other = parity ^ 1;
-  const T alpha = static_cast<T>(a.alpha != nullptr ? a.alpha[j] : state->alpha);
+  const T alpha = a.alpha != nullptr ? static_cast<T>(a.alpha[j]) : slab.alpha;
   int overflow = 0;
-  __syncwarp();
   {
     const int nm = a.m_cnt[j];
     const int nz = a.z_cnt[j];
@@ -375,12 +416,12 @@ __device__ __noinline__ int DropColumn(const FusedArgs<T>& a, unsigned char* bas
     }
     ClearTable(keys, table, lane);
     // M(:, j) and Z(:, j) into shared memory (sorted by row), then M(j, :) into its hash
-#pragma unroll 1
+#pragma unroll kUnroll
     for (int e = lane; e < nm; e += kWarp) {
       mr[e] = a.m_rows[j * a.topk + e];
       mv[e] = a.m_vals[j * a.topk + e];
     }
-#pragma unroll 1
+#pragma unroll kUnroll
     for (int e = lane; e < nz; e += kWarp) {
       zr[e] = a.z_rows[j * a.cap_z + e];
       zv[e] = a.z_vals[j * a.cap_z + e];
@@ -400,7 +441,7 @@ __device__ __noinline__ int DropColumn(const FusedArgs<T>& a, unsigned char* bas
       lo = min(lo, zr[0]);
       hi = max(hi, zr[nz - 1]);
     }
-#pragma unroll 1
+#pragma unroll kUnroll
     for (int e = lane; e < nmt; e += kWarp) {
       const int at = FindOrInsert(k_mt, b_mt, mtc[e], &fresh);
       v_mt[at] = mtv[e];
@@ -495,15 +536,15 @@ __device__ __noinline__ int DropColumn(const FusedArgs<T>& a, unsigned char* bas
       const int32_t seg_hi = hi - seg_lo < kDropWindowRows ? hi : seg_lo + (kDropWindowRows - 1);
       const int words = (seg_hi - seg_lo) / 32 + 1;
       if (lane == 0 && j >= seg_lo && j <= seg_hi) MarkRow(bm, summary, static_cast<int>(j - seg_lo));
-#pragma unroll 1
+#pragma unroll kUnroll
       for (int e = lane; e < nm; e += kWarp) {
         if (mr[e] >= seg_lo && mr[e] <= seg_hi) MarkRow(bm, summary, mr[e] - seg_lo);
       }
-#pragma unroll 1
+#pragma unroll kUnroll
       for (int e = lane; e < nz; e += kWarp) {
         if (zr[e] >= seg_lo && zr[e] <= seg_hi) MarkRow(bm, summary, zr[e] - seg_lo);
       }
-#pragma unroll 1
+#pragma unroll kUnroll
       for (int t = lane; t < table; t += kWarp) {
         const int32_t key = keys[t];
         if (key != kEmpty && key >= seg_lo && key <= seg_hi) MarkRow(bm, summary, key - seg_lo);
@@ -913,6 +954,26 @@ __device__ __forceinline__ bool DropGroup(const FusedArgs<T>& a, unsigned char* 
   return true;
 }
 
+// A column of a group that does not fit (a call per column: over several
+// columns the compiler keeps 157 registers in FP64, and groups of two then run
+// in two waves).
+template <class T>
+__device__ __noinline__ int DropOneColumn(const FusedArgs<T>& a, unsigned char* base, bool clear, int64_t j,
+                                          unsigned long long* written) {
+  const DropSlab<T> slab(a, base, clear, threadIdx.x & 31);
+  return DropColumn<T, 1>(a, slab, j, written);
+}
+
+// A warp's entries of M and its overflow bits into the loop's state.
+template <class T>
+__device__ __forceinline__ void FinishDrop(const FusedArgs<T>& a, unsigned long long written, int overflow, int lane) {
+  overflow = __reduce_or_sync(0xffffffffu, overflow);
+  if (lane == 0) {
+    if (written != 0ull) atomicAdd(&a.state->nnz_m, written);
+    if (overflow != 0) atomicOr(&a.state->overflow, overflow);
+  }
+}
+
 template <class T, int kEll, int C>
 __global__ void __launch_bounds__(kGroupWarps * kWarp) FusedDropKernel(const __grid_constant__ FusedArgs<T> a) {
   extern __shared__ __align__(16) unsigned char fused_drop_smem[];
@@ -927,24 +988,41 @@ __global__ void __launch_bounds__(kGroupWarps * kWarp) FusedDropKernel(const __g
   bool clear = false;  // whether the window starts clear
 #pragma unroll 1
   for (int64_t j0 = warp * C; j0 < a.n; j0 += warps * C) {
-    if (a.words > 0) {
-      if (!clear) {
-        unsigned char* at = base;
-        RowWindow w = WindowAt(at, a.words, 0);
-        ClearWindow(w, lane);
-        clear = true;
-      }
-      if (DropGroup<T, kEll, C>(a, base, j0, alpha, parity, lane, &written, &overflow)) continue;
+    if (!clear) {
+      unsigned char* at = base;
+      RowWindow w = WindowAt(at, a.words, 0);
+      ClearWindow(w, lane);
+      clear = true;
     }
+    if (DropGroup<T, kEll, C>(a, base, j0, alpha, parity, lane, &written, &overflow)) continue;
     clear = false;
 #pragma unroll 1
-    for (int64_t j = j0; j < j0 + C && j < a.n; ++j) overflow |= DropColumn<T>(a, base, j, &written);
+    for (int64_t j = j0; j < j0 + C && j < a.n; ++j) overflow |= DropOneColumn<T>(a, base, j == j0, j, &written);
   }
-  overflow = __reduce_or_sync(0xffffffffu, overflow);
-  if (lane == 0) {
-    if (written != 0ull) atomicAdd(&a.state->nnz_m, written);
-    if (overflow != 0) atomicOr(&a.state->overflow, overflow);
-  }
+  FinishDrop(a, written, overflow, lane);
+}
+
+// The drop step column by column, for operators whose groups have no window
+// (GroupWords).  What bounds it: the latency of the hash updates and of the
+// window's scans, so it is a kernel of its own with registers for 24 (FP32) or
+// 20 warps an SM.  As the fallback inside the group kernel (168 registers, the
+// window cleared for every column) it left 12, and six iterations on a randomly
+// permuted 47^3 operator in FP32 storage, 16 entries a column, took 27.2 ms;
+// now 19.2 (20.3 before there were groups).  At 90^3: 4.7 ms a launch in FP32
+// storage, 6.5 in FP64.
+template <class T>
+__global__ void __launch_bounds__(kColumnWarps * kWarp, sizeof(T) == 4 ? 6 : 5)
+    FusedDropColumnsKernel(const __grid_constant__ FusedArgs<T> a) {
+  extern __shared__ __align__(16) unsigned char fused_drop_smem[];
+  const int lane = threadIdx.x & 31;
+  unsigned char* base = fused_drop_smem + (threadIdx.x >> 5) * a.drop_bytes;
+  const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  unsigned long long written = 0;
+  int overflow = 0;
+  const DropSlab<T> slab(a, base, true, lane);
+  for (int64_t j = warp; j < a.n; j += warps) overflow |= DropColumn<T, 4>(a, slab, j, &written);
+  FinishDrop(a, written, overflow, lane);
 }
 
 // ---------------------------------------------------------------------------
@@ -978,33 +1056,64 @@ __device__ __forceinline__ double SumStaged(double s, const double* src, int cou
   return s;
 }
 
-// One column on its own, for columns whose rows do not fit the group's window.
+// A warp's shared memory while it goes column by column.
+template <class T>
+struct ResidualSlab {
+  uint32_t* bm;
+  uint32_t* summary;
+  uint16_t* rows;
+  int32_t* mkeys;
+  T* mvals;
+  int32_t* zkeys;
+  T* zvals;
+  double* stage;
+  int mbits;  // buckets of two slots
+  int zbits;
+
+  // clear: whether the window has to be cleared.
+  __device__ __forceinline__ ResidualSlab(const FusedArgs<T>& a, unsigned char* base, bool clear, int lane) {
+    bm = reinterpret_cast<uint32_t*>(base);
+    base += Round16(static_cast<size_t>(kWindowWords) * 4);
+    summary = reinterpret_cast<uint32_t*>(base);
+    base += Round16(static_cast<size_t>(kResidualSummary) * 4);
+    rows = reinterpret_cast<uint16_t*>(base);
+    base += Round16(static_cast<size_t>(kRowsCap) * 2);
+    mkeys = reinterpret_cast<int32_t*>(base);
+    base += Round16(static_cast<size_t>(a.m_hash_slots) * 4);
+    mvals = reinterpret_cast<T*>(base);
+    base += Round16(static_cast<size_t>(a.m_hash_slots) * sizeof(T));
+    zkeys = reinterpret_cast<int32_t*>(base);
+    base += Round16(static_cast<size_t>(a.z_hash_slots) * 4);
+    zvals = reinterpret_cast<T*>(base);
+    base += Round16(static_cast<size_t>(a.z_hash_slots) * sizeof(T));
+    stage = reinterpret_cast<double*>(base);
+    mbits = Log2(a.m_hash_slots) - 1;
+    zbits = Log2(a.z_hash_slots) - 1;
+    if (clear) {
+      __syncwarp();
+      ClearWords(bm, kWindowWords, lane);
+      ClearWords(summary, kResidualSummary, lane);
+      __syncwarp();
+    }
+  }
+};
+
+// One column on its own; its window is clear before and after.
 template <class T, int kEll>
-__device__ __noinline__ void ResidualColumn(const FusedArgs<T>& a, unsigned char* base, int64_t j,
-                                            unsigned long long* written_out) {
+__device__ __forceinline__ void ResidualColumn(const FusedArgs<T>& a, const ResidualSlab<T>& slab, int64_t j,
+                                               unsigned long long* written_out) {
   const int lane = threadIdx.x & 31;
-  constexpr int kSummary = (kWindowWords + kWarp * kWarp - 1) / (kWarp * kWarp) * kWarp;
-  uint32_t* bm = reinterpret_cast<uint32_t*>(base);
-  base += Round16(static_cast<size_t>(kWindowWords) * 4);
-  uint32_t* summary = reinterpret_cast<uint32_t*>(base);
-  base += Round16(static_cast<size_t>(kSummary) * 4);
-  uint16_t* rows = reinterpret_cast<uint16_t*>(base);
-  base += Round16(static_cast<size_t>(kRowsCap) * 2);
-  int32_t* mkeys = reinterpret_cast<int32_t*>(base);
-  base += Round16(static_cast<size_t>(a.m_hash_slots) * 4);
-  T* mvals = reinterpret_cast<T*>(base);
-  base += Round16(static_cast<size_t>(a.m_hash_slots) * sizeof(T));
-  int32_t* zkeys = reinterpret_cast<int32_t*>(base);
-  base += Round16(static_cast<size_t>(a.z_hash_slots) * 4);
-  T* zvals = reinterpret_cast<T*>(base);
-  base += Round16(static_cast<size_t>(a.z_hash_slots) * sizeof(T));
-  double* stage0 = reinterpret_cast<double*>(base);
+  uint32_t* bm = slab.bm;
+  uint32_t* summary = slab.summary;
+  uint16_t* rows = slab.rows;
+  int32_t* mkeys = slab.mkeys;
+  T* mvals = slab.mvals;
+  int32_t* zkeys = slab.zkeys;
+  T* zvals = slab.zvals;
+  double* stage0 = slab.stage;
   double* stage1 = stage0 + kWarp;
-  const int mbits = Log2(a.m_hash_slots) - 1;  // buckets of two slots
-  const int zbits = Log2(a.z_hash_slots) - 1;
-  ClearWords(bm, kWindowWords, lane);
-  ClearWords(summary, kSummary, lane);
-  __syncwarp();
+  const int mbits = slab.mbits;
+  const int zbits = slab.zbits;
   {
     // ---- R(:, j) = e_j - A M(:, j) ----------------------------------------
     const int nm = a.m_cnt[j];
@@ -1413,6 +1522,14 @@ __device__ __forceinline__ bool ResidualGroup(const FusedArgs<T>& a, unsigned ch
   return true;
 }
 
+// A column of a group that does not fit.
+template <class T, int kEll>
+__device__ __noinline__ void ResidualOneColumn(const FusedArgs<T>& a, unsigned char* base, bool clear, int64_t j,
+                                               unsigned long long* written) {
+  const ResidualSlab<T> slab(a, base, clear, threadIdx.x & 31);
+  ResidualColumn<T, kEll>(a, slab, j, written);
+}
+
 template <class T, int kEll, int kUse, int C>
 __global__ void __launch_bounds__(kGroupWarps * kWarp) FusedResidualKernel(const __grid_constant__ FusedArgs<T> a) {
   extern __shared__ __align__(16) unsigned char fused_res_smem[];
@@ -1426,20 +1543,39 @@ __global__ void __launch_bounds__(kGroupWarps * kWarp) FusedResidualKernel(const
 #pragma unroll 1
   for (int64_t j0 = warp * C; j0 < a.n; j0 += warps * C) {
     if (lane < C && j0 + lane < a.n) a.mt_cnt[read_set][j0 + lane] = 0;  // refilled from zero by the next drop kernel
-    if (a.words > 0) {
-      if (!clear) {
-        unsigned char* at = base;
-        RowWindow wm = WindowAt(at, a.words, 0);
-        RowWindow wr = WindowAt(at, a.words, 0);
-        ClearWindow(wm, lane);
-        ClearWindow(wr, lane);
-        clear = true;
-      }
-      if (ResidualGroup<T, kEll, kUse, C>(a, base, j0, lane, &written)) continue;
+    if (!clear) {
+      unsigned char* at = base;
+      RowWindow wm = WindowAt(at, a.words, 0);
+      RowWindow wr = WindowAt(at, a.words, 0);
+      ClearWindow(wm, lane);
+      ClearWindow(wr, lane);
+      clear = true;
     }
+    if (ResidualGroup<T, kEll, kUse, C>(a, base, j0, lane, &written)) continue;
     clear = false;
 #pragma unroll 1
-    for (int64_t j = j0; j < j0 + C && j < a.n; ++j) ResidualColumn<T, kEll>(a, base, j, &written);
+    for (int64_t j = j0; j < j0 + C && j < a.n; ++j) ResidualOneColumn<T, kEll>(a, base, j == j0, j, &written);
+  }
+  if (lane == 0 && written != 0ull) atomicAdd(&a.state->nnz_z, written);
+}
+
+// The residual and projection column by column, for operators whose groups
+// have no window: 20 to 24 warps an SM, bound by the latency of hash lookups
+// and sequential sums.  6.0 ms a launch at 90^3 in FP32 storage, 7.0 in FP64.
+template <class T, int kEll>
+__global__ void __launch_bounds__(kColumnWarps * kWarp)
+    FusedResidualColumnsKernel(const __grid_constant__ FusedArgs<T> a) {
+  extern __shared__ __align__(16) unsigned char fused_res_smem[];
+  const int lane = threadIdx.x & 31;
+  unsigned char* base = fused_res_smem + (threadIdx.x >> 5) * a.residual_bytes;
+  const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  const int64_t read_set = a.state->parity;  // the M^T set the drop kernel has just read
+  unsigned long long written = 0;
+  const ResidualSlab<T> slab(a, base, true, lane);
+  for (int64_t j = warp; j < a.n; j += warps) {
+    if (lane == 0) a.mt_cnt[read_set][j] = 0;  // refilled from zero by the next drop kernel
+    ResidualColumn<T, kEll>(a, slab, j, &written);
   }
   if (lane == 0 && written != 0ull) atomicAdd(&a.state->nnz_z, written);
 }
@@ -1715,13 +1851,13 @@ class FusedMr final : public FusedMrBase {
   FusedBatchSums StepBatch(Ctx& ctx) override {
     const cudaStream_t st = ctx.stream;
     {
-      prof::Scope scope(st, "fused_drop", 0.0);
-      drop_kernel_<<<drop_grid_, kGroupWarps * kWarp, drop_smem_, st>>>(args_);
+      prof::Scope scope(st, drop_class_, 0.0);
+      drop_kernel_<<<drop_grid_, warps_ * kWarp, drop_smem_, st>>>(args_);
       SPAI_LAUNCH_CHECK();
     }
     {
-      prof::Scope scope(st, "fused_residual", 0.0);
-      res_kernel_<<<res_grid_, kGroupWarps * kWarp, res_smem_, st>>>(args_);
+      prof::Scope scope(st, res_class_, 0.0);
+      res_kernel_<<<res_grid_, warps_ * kWarp, res_smem_, st>>>(args_);
       SPAI_LAUNCH_CHECK();
     }
     FlipKernel<<<1, 1, 0, st>>>(args_.state);
@@ -1796,13 +1932,13 @@ class FusedMr final : public FusedMrBase {
     FusedState out{};
     for (int64_t body = 0; body <= p.max_iterations; ++body) {
       {
-        prof::Scope scope(st, "fused_drop", 0.0);
-        drop_kernel_<<<drop_grid_, kGroupWarps * kWarp, drop_smem_, st>>>(args_);
+        prof::Scope scope(st, drop_class_, 0.0);
+        drop_kernel_<<<drop_grid_, warps_ * kWarp, drop_smem_, st>>>(args_);
         SPAI_LAUNCH_CHECK();
       }
       {
-        prof::Scope scope(st, "fused_residual", 0.0);
-        res_kernel_<<<res_grid_, kGroupWarps * kWarp, res_smem_, st>>>(args_);
+        prof::Scope scope(st, res_class_, 0.0);
+        res_kernel_<<<res_grid_, warps_ * kWarp, res_smem_, st>>>(args_);
         SPAI_LAUNCH_CHECK();
       }
       {
@@ -1817,8 +1953,8 @@ class FusedMr final : public FusedMrBase {
       // residual step reads M, A and Pr, writes Z, Z^T and the three column sums
       const double m_new = static_cast<double>(out.last_nnz_m);
       const double z_new = static_cast<double>(out.last_nnz_z);
-      prof::AddBytes("fused_drop", e * (2.0 * m_prev + 2.0 * z_prev + 2.0 * m_new) + 4.0 * 6.0 * n);
-      prof::AddBytes("fused_residual",
+      prof::AddBytes(drop_class_, e * (2.0 * m_prev + 2.0 * z_prev + 2.0 * m_new) + 4.0 * 6.0 * n);
+      prof::AddBytes(res_class_,
                      e * m_new + a_bytes + sizeof(T) * n + 2.0 * e * z_new + 4.0 * 3.0 * n + 24.0 * n);
       m_prev = m_new;
       z_prev = z_new;
@@ -1917,7 +2053,8 @@ class FusedMr final : public FusedMrBase {
   // Words of a group's window: a little over four bandwidths of A on either
   // side of the group, which covers the drop step's and the residual's rows of
   // nearly every column (M reaches two to three bandwidths, R one more).  Wider
-  // operators, and operators with entries that are not finite (a column group
+  // operators (a bandwidth above about 7,900: 3-D grids from 89^3 up, unordered
+  // meshes), and operators with entries that are not finite (a column group
   // multiplies them by the 0 of an absent entry), go column by column.
   static int GroupWords(const FusedMrProblem& p) {
     if (!p.finite) return 0;
@@ -1936,14 +2073,31 @@ class FusedMr final : public FusedMrBase {
     res_kernel_ = FusedResidualKernel<T, kEll, kUse, C>;
     drop_kernel_ = FusedDropKernel<T, kEll, C>;
     columns_ = C;
-    size_t drop = DropWarpBytes<T>(args_.topk + args_.cap_z, args_.d_mt_slots, args_.d_r_slots);
-    size_t residual = ResidualSlabBytes<T>(args_.m_hash_slots, args_.z_hash_slots);
-    if (args_.words > 0) {
-      drop = std::max(drop, DropGroupBytes<T, C>(args_.words));
-      residual = std::max(residual, ResidualGroupBytes<T, C>(args_.words, args_.topk));
+    warps_ = kGroupWarps;
+    drop_class_ = "fused_drop";
+    res_class_ = "fused_residual";
+    args_.drop_bytes = Round16(std::max(DropWarpBytes<T>(args_.topk + args_.cap_z, args_.d_mt_slots, args_.d_r_slots),
+                                        DropGroupBytes<T, C>(args_.words)));
+    args_.residual_bytes = Round16(std::max(ResidualSlabBytes<T>(args_.m_hash_slots, args_.z_hash_slots),
+                                            ResidualGroupBytes<T, C>(args_.words, args_.topk)));
+  }
+
+  // Without a window (GroupWords): the kernels that take one column after another.
+  void ChooseColumns(int ell) {
+    switch (ell) {
+      case 4: res_kernel_ = FusedResidualColumnsKernel<T, 4>; break;
+      case 8: res_kernel_ = FusedResidualColumnsKernel<T, 8>; break;
+      case 12: res_kernel_ = FusedResidualColumnsKernel<T, 12>; break;
+      case 16: res_kernel_ = FusedResidualColumnsKernel<T, 16>; break;
+      default: throw std::invalid_argument("fused MR: unsupported ELL width");
     }
-    args_.drop_bytes = Round16(drop);
-    args_.residual_bytes = Round16(residual);
+    drop_kernel_ = FusedDropColumnsKernel<T>;
+    columns_ = 1;
+    warps_ = kColumnWarps;
+    drop_class_ = "fused_drop_columns";
+    res_class_ = "fused_residual_columns";
+    args_.drop_bytes = Round16(DropWarpBytes<T>(args_.topk + args_.cap_z, args_.d_mt_slots, args_.d_r_slots));
+    args_.residual_bytes = Round16(ResidualSlabBytes<T>(args_.m_hash_slots, args_.z_hash_slots));
   }
 
   template <int C>
@@ -1971,25 +2125,25 @@ class FusedMr final : public FusedMrBase {
     SPAI_CUDA(cudaGetDevice(&device));
     int sms = 0;
     SPAI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    if (args_.n >= int64_t{4} * 16 * sms) {
+    if (args_.words == 0) {
+      ChooseColumns(p.ell_width);
+    } else if (args_.n >= int64_t{4} * 16 * sms) {
       ChooseEll<4>(p.ell_width, p.a_longest);
     } else {
       ChooseEll<2>(p.ell_width, p.a_longest);
     }
-    drop_smem_ = static_cast<size_t>(kGroupWarps) * args_.drop_bytes;
-    res_smem_ = static_cast<size_t>(kGroupWarps) * args_.residual_bytes;
+    drop_smem_ = static_cast<size_t>(warps_) * args_.drop_bytes;
+    res_smem_ = static_cast<size_t>(warps_) * args_.residual_bytes;
     SPAI_CUDA(cudaFuncSetAttribute(drop_kernel_, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(drop_smem_)));
     SPAI_CUDA(cudaFuncSetAttribute(res_kernel_, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(res_smem_)));
     int drop_blocks = 0;
     int res_blocks = 0;
-    SPAI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&drop_blocks, drop_kernel_, kGroupWarps * kWarp,
-                                                            drop_smem_));
-    SPAI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res_blocks, res_kernel_, kGroupWarps * kWarp,
-                                                            res_smem_));
+    SPAI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&drop_blocks, drop_kernel_, warps_ * kWarp, drop_smem_));
+    SPAI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res_blocks, res_kernel_, warps_ * kWarp, res_smem_));
     if (drop_blocks < 1 || res_blocks < 1) throw std::runtime_error("fused MR: kernels do not fit on an SM");
-    const int64_t blocks = CeilDiv(args_.n, int64_t{kGroupWarps} * columns_);
+    const int64_t blocks = CeilDiv(args_.n, int64_t{warps_} * columns_);
     drop_grid_ = static_cast<unsigned>(std::min<int64_t>(blocks, int64_t{sms} * drop_blocks));
     res_grid_ = static_cast<unsigned>(std::min<int64_t>(blocks, int64_t{sms} * res_blocks));
     decide_grid_ = static_cast<unsigned>(CeilDiv(args_.n, kTreeChunk));
@@ -2021,8 +2175,8 @@ class FusedMr final : public FusedMrBase {
       SPAI_CUDA(cudaStreamUpdateCaptureDependencies(cs, &loop_node, 1, cudaStreamSetCaptureDependencies));
       cudaGraph_t body = params.conditional.phGraph_out[0];
       SPAI_CUDA(cudaStreamBeginCaptureToGraph(bs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-      drop_kernel_<<<drop_grid_, kGroupWarps * kWarp, drop_smem_, bs>>>(a);
-      res_kernel_<<<res_grid_, kGroupWarps * kWarp, res_smem_, bs>>>(a);
+      drop_kernel_<<<drop_grid_, warps_ * kWarp, drop_smem_, bs>>>(a);
+      res_kernel_<<<res_grid_, warps_ * kWarp, res_smem_, bs>>>(a);
       FusedDecideKernel<T><<<decide_grid_, kTreeLanes, 0, bs>>>(a, loop, true);
       SPAI_CUDA(cudaGetLastError());
       cudaGraph_t body_out = nullptr;
@@ -2068,7 +2222,10 @@ class FusedMr final : public FusedMrBase {
   cudaGraphExec_t exec_ = nullptr;
   void (*res_kernel_)(const FusedArgs<T>) = nullptr;
   void (*drop_kernel_)(const FusedArgs<T>) = nullptr;
-  int columns_ = 1;
+  int columns_ = 1;  // per warp
+  int warps_ = 1;    // per block
+  const char* drop_class_ = "";  // profile classes of the two kernels
+  const char* res_class_ = "";
   size_t drop_smem_ = 0;
   size_t res_smem_ = 0;
   unsigned drop_grid_ = 1;

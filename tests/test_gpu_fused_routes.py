@@ -1,0 +1,69 @@
+"""Which kernels a fused Global MR run takes (read from the library's own
+accounting), and the same bits as the unfused kernels on each way."""
+import ctypes
+
+import numpy as np
+import pytest
+from scipy import sparse
+
+from parallellocallyoptimalapproximatesparsematrixinverses_b200 import _lib, global_spai, problems
+from tests.helpers import assert_same_result
+
+pytestmark = pytest.mark.gpu
+
+
+def _launches(lib, name):
+    ms, count, nbytes = ctypes.c_double(0), ctypes.c_int64(0), ctypes.c_double(0)
+    lib.spai_profile_read(name.encode(), ctypes.byref(ms), ctypes.byref(count), ctypes.byref(nbytes))
+    return count.value, nbytes.value
+
+
+def profiled(call, *names):
+    """call()'s result and the launches and algorithmic bytes of the named kernel classes."""
+    lib = _lib.load()
+    lib.spai_profile_reset()
+    lib.spai_profile_enable(1)
+    try:
+        result = call()
+    finally:
+        lib.spai_profile_enable(0)
+    counts = {name: _launches(lib, name) for name in names}
+    lib.spai_profile_reset()
+    return result, counts
+
+
+def unfused(call):
+    lib = _lib.load()
+    lib.spai_set_fused_mr(0)
+    try:
+        return call()
+    finally:
+        lib.spai_set_fused_mr(1)
+
+
+def band(n, distances, seed=0):
+    """Symmetric, diagonally dominant, entries at the given distances from the diagonal."""
+    rng = np.random.default_rng(seed)
+    rows = np.concatenate([np.arange(n - d) for d in distances])
+    cols = np.concatenate([np.arange(n - d) + d for d in distances])
+    off = sparse.coo_matrix((-rng.uniform(0.1, 1.0, rows.size), (rows, cols)), shape=(n, n)).tocsr()
+    off = off + off.T
+    a = sparse.csc_matrix(off + sparse.diags(1.05 * np.asarray(abs(off).sum(axis=1)).ravel() + 0.1))
+    a.sort_indices()
+    return a
+
+
+# operators wider than any window of a column group, rows of A in 4, 8, 12 and 16 slots
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("distances,topk", [([9000], 6), ([1, 9000], 8), ([1, 2, 3, 9000], 5), ([1, 2, 3, 4, 5, 9000], 5)])
+def test_wide_operators_run_on_the_column_kernels(require_gpu, distances, topk, precision):
+    a = band(18_011, distances)
+    kw = dict(M0=problems.diagonal_inverse(a), max_iterations=7, tolerance=0.0, max_density=topk / a.shape[0],
+              topk_per_column=topk, precision=precision)
+    got, counts = profiled(lambda: global_spai.mr(a, **kw), "fused_drop", "fused_drop_columns", "fused_residual",
+                           "fused_residual_columns")
+    assert counts["fused_drop"][0] == counts["fused_residual"][0] == 0
+    assert counts["fused_drop_columns"][0] == counts["fused_residual_columns"][0] == 7
+    want = unfused(lambda: global_spai.mr(a, **kw))
+    assert_same_result(got, want, f"{distances} {precision}, launched one by one")
+    assert_same_result(global_spai.mr(a, **kw), want, f"{distances} {precision}, as a graph")
