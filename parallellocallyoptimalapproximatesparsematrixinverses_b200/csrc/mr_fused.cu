@@ -57,6 +57,7 @@ constexpr int kConverged = 1;
 constexpr int kBreakdown = 2;
 constexpr int kIterationLimit = 3;
 constexpr int kOverflowStop = 4;
+constexpr int kScatteredStop = 5;  // too few column groups fit: the host goes on column by column
 
 struct FusedRow {
   int64_t iteration;
@@ -78,8 +79,9 @@ struct FusedState {
   int32_t overflow;
   int32_t stop;
   unsigned int arrive;          // blocks of the decide kernel that are done
-  int32_t pad;
+  unsigned int unfit;           // groups of this iteration's two kernels that went column by column
   int64_t bodies;               // loop-body executions
+  int64_t last_unfit;           // the last step's count (batched runs)
 };
 
 template <class T>
@@ -95,6 +97,7 @@ struct FusedArgs {
   int d_r_slots;      // drop kernel: R(j, :)
   int words;           // 32-row words of the column groups' windows (0: every column on its own)
   int64_t bandwidth;   // largest |i - k| over the entries of A
+  int64_t unfit_limit;    // groups of an iteration's two kernels that may go column by column
   size_t drop_bytes;      // shared memory of a warp
   size_t residual_bytes;
   int64_t max_iterations;
@@ -985,6 +988,7 @@ __global__ void __launch_bounds__(kGroupWarps * kWarp) FusedDropKernel(const __g
   const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
   unsigned long long written = 0;
   int overflow = 0;
+  unsigned int unfit = 0;
   bool clear = false;  // whether the window starts clear
 #pragma unroll 1
   for (int64_t j0 = warp * C; j0 < a.n; j0 += warps * C) {
@@ -996,9 +1000,11 @@ __global__ void __launch_bounds__(kGroupWarps * kWarp) FusedDropKernel(const __g
     }
     if (DropGroup<T, kEll, C>(a, base, j0, alpha, parity, lane, &written, &overflow)) continue;
     clear = false;
+    ++unfit;
 #pragma unroll 1
     for (int64_t j = j0; j < j0 + C && j < a.n; ++j) overflow |= DropOneColumn<T>(a, base, j == j0, j, &written);
   }
+  if (lane == 0 && unfit != 0u) atomicAdd(&a.state->unfit, unfit);
   FinishDrop(a, written, overflow, lane);
 }
 
@@ -1539,6 +1545,7 @@ __global__ void __launch_bounds__(kGroupWarps * kWarp) FusedResidualKernel(const
   const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
   const int64_t read_set = a.state->parity;  // the M^T set the drop kernel has just read
   unsigned long long written = 0;
+  unsigned int unfit = 0;
   bool clear = false;  // whether the windows start clear
 #pragma unroll 1
   for (int64_t j0 = warp * C; j0 < a.n; j0 += warps * C) {
@@ -1553,10 +1560,14 @@ __global__ void __launch_bounds__(kGroupWarps * kWarp) FusedResidualKernel(const
     }
     if (ResidualGroup<T, kEll, kUse, C>(a, base, j0, lane, &written)) continue;
     clear = false;
+    ++unfit;
 #pragma unroll 1
     for (int64_t j = j0; j < j0 + C && j < a.n; ++j) ResidualOneColumn<T, kEll>(a, base, j == j0, j, &written);
   }
-  if (lane == 0 && written != 0ull) atomicAdd(&a.state->nnz_z, written);
+  if (lane == 0) {
+    if (written != 0ull) atomicAdd(&a.state->nnz_z, written);
+    if (unfit != 0u) atomicAdd(&a.state->unfit, unfit);
+  }
 }
 
 // The residual and projection column by column, for operators whose groups
@@ -1641,6 +1652,8 @@ __global__ void __launch_bounds__(kTreeLanes) FusedDecideKernel(FusedArgs<T> a, 
   state->nnz_dir = state->nnz_z;
   state->nnz_m = 0ull;
   state->nnz_z = 0ull;
+  const bool scattered = static_cast<int64_t>(state->unfit) > a.unfit_limit;
+  state->unfit = 0u;
   int stop = kRunning;
   if (state->overflow != 0) {
     stop = kOverflowStop;
@@ -1660,6 +1673,7 @@ __global__ void __launch_bounds__(kTreeLanes) FusedDecideKernel(FusedArgs<T> a, 
         stop = kBreakdown;
       } else {
         state->alpha = alpha;
+        if (scattered) stop = kScatteredStop;
       }
     }
   }
@@ -1714,7 +1728,11 @@ __global__ void ToSlotsKernel(CscView<T> x, int cap, int32_t* __restrict__ rows,
 }
 
 // A batched step is over: the M^T sets change places (the decide kernel's part in single runs).
-__global__ void FlipKernel(FusedState* __restrict__ state) { state->parity ^= 1; }
+__global__ void FlipKernel(FusedState* __restrict__ state) {
+  state->parity ^= 1;
+  state->last_unfit = state->unfit;
+  state->unfit = 0u;
+}
 
 // out[s] = the entries of M and out[count + s] those of Z in the columns [first[s], first[s + 1]); a block each.
 __global__ void SegmentCountsKernel(const int32_t* __restrict__ m_cnt, const int32_t* __restrict__ z_cnt,
@@ -1806,14 +1824,14 @@ class FusedMr final : public FusedMrBase {
     if (prof::Enabled()) {
       out = RunStepwise(ctx, problem, m.nnz, z.nnz);
     } else {
-      if (exec_ == nullptr) Capture();
-      {
-        prof::Scope scope(st, "fused_mr_loop", 0.0);
+      do {
+        if (exec_ == nullptr) Capture();
         SPAI_CUDA(cudaGraphLaunch(exec_, st));
-      }
-      SPAI_CUDA(cudaMemcpyAsync(host_state_, state_.data(), sizeof(FusedState), cudaMemcpyDeviceToHost, st));
-      ctx.Sync();
-      out = *host_state_;
+        SPAI_CUDA(cudaMemcpyAsync(host_state_, state_.data(), sizeof(FusedState), cudaMemcpyDeviceToHost, st));
+        ctx.Sync();
+        out = *host_state_;
+        if (out.stop == kScatteredStop) LeaveGroups(problem);
+      } while (out.stop == kScatteredStop);
       CountLaunches(3 * out.bodies);
     }
     outcome.ran = true;
@@ -1845,6 +1863,7 @@ class FusedMr final : public FusedMrBase {
                   const double* alpha) override {
     if (!FusedMrApplicable(problem)) return false;
     Start(ctx, problem, *static_cast<const DevCsc<T>*>(m_csc), *static_cast<const DevCsc<T>*>(z_csc), 0.0, alpha);
+    problem_ = problem;
     return true;
   }
 
@@ -1873,6 +1892,7 @@ class FusedMr final : public FusedMrBase {
     SPAI_CUDA(cudaMemcpyAsync(host_state_, state_.data(), sizeof(FusedState), cudaMemcpyDeviceToHost, st));
     SPAI_CUDA(cudaMemcpyAsync(out, out_dev, sizeof(int64_t) * 2 * segments, cudaMemcpyDeviceToHost, st));
     ctx.Sync();
+    if (host_state_->last_unfit > args_.unfit_limit) LeaveGroups(problem_);
     return host_state_->overflow == 0;
   }
 
@@ -1958,7 +1978,11 @@ class FusedMr final : public FusedMrBase {
                      e * m_new + a_bytes + sizeof(T) * n + 2.0 * e * z_new + 4.0 * 3.0 * n + 24.0 * n);
       m_prev = m_new;
       z_prev = z_new;
-      if (out.stop != kRunning) break;
+      if (out.stop == kScatteredStop) {
+        LeaveGroups(p);
+      } else if (out.stop != kRunning) {
+        break;
+      }
     }
     return out;
   }
@@ -2000,7 +2024,7 @@ class FusedMr final : public FusedMrBase {
     a.z_hash_slots = NextPow2Int(std::max(2 * cap_z, kWarp));
     a.d_mt_slots = NextPow2Int(std::max(2 * cap_mt, kWarp));
     a.d_r_slots = DropRowSlots(p);
-    a.words = GroupWords(p);
+    a.words = scattered_ ? 0 : GroupWords(p);
     a.bandwidth = p.bandwidth;
     a.max_iterations = p.max_iterations;
     a.tolerance = p.tolerance;
@@ -2119,6 +2143,24 @@ class FusedMr final : public FusedMrBase {
     }
   }
 
+  // The following iterations, of this run and of later ones on this problem, go
+  // column by column: more than a sixteenth of the two kernels' groups did not
+  // fit.  Such a group costs its attempt and the slow way through its columns
+  // (few warps, generic addresses).  47^3, 16 entries a column, FP32 storage, ten
+  // iterations, rows shuffled within 10, 30, 100 and 2,000 so that 3, 16, 24 and
+  // 45 % of the groups do not fit: 12.8, 21.5, 24.8 and 31.9 ms in groups against
+  // 15.3, 14.6, 14.8 and 15.3 column by column (7.7 unshuffled); in FP64 16.3,
+  // 26.5, 28.9 and 36.2 against 19.2, 18.3, 18.6 and 19.1.
+  void LeaveGroups(const FusedMrProblem& p) {
+    scattered_ = true;
+    args_.words = 0;
+    Configure(p);
+    if (exec_ != nullptr) {
+      cudaGraphExecDestroy(exec_);
+      exec_ = nullptr;
+    }
+  }
+
   // Kernel choice, shared memory and grids (once per problem shape).
   void Configure(const FusedMrProblem& p) {
     int device = 0;
@@ -2143,6 +2185,7 @@ class FusedMr final : public FusedMrBase {
     SPAI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&drop_blocks, drop_kernel_, warps_ * kWarp, drop_smem_));
     SPAI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res_blocks, res_kernel_, warps_ * kWarp, res_smem_));
     if (drop_blocks < 1 || res_blocks < 1) throw std::runtime_error("fused MR: kernels do not fit on an SM");
+    args_.unfit_limit = columns_ > 1 ? CeilDiv(args_.n, int64_t{columns_}) / 8 : INT64_MAX;
     const int64_t blocks = CeilDiv(args_.n, int64_t{warps_} * columns_);
     drop_grid_ = static_cast<unsigned>(std::min<int64_t>(blocks, int64_t{sms} * drop_blocks));
     res_grid_ = static_cast<unsigned>(std::min<int64_t>(blocks, int64_t{sms} * res_blocks));
@@ -2222,6 +2265,8 @@ class FusedMr final : public FusedMrBase {
   cudaGraphExec_t exec_ = nullptr;
   void (*res_kernel_)(const FusedArgs<T>) = nullptr;
   void (*drop_kernel_)(const FusedArgs<T>) = nullptr;
+  FusedMrProblem problem_;   // of the running batch
+  bool scattered_ = false;   // the problem's column groups do not fit
   int columns_ = 1;  // per warp
   int warps_ = 1;    // per block
   const char* drop_class_ = "";  // profile classes of the two kernels

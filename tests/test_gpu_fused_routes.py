@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 from scipy import sparse
 
-from parallellocallyoptimalapproximatesparsematrixinverses_b200 import _lib, global_spai, problems
+from parallellocallyoptimalapproximatesparsematrixinverses_b200 import Session, _lib, global_spai, problems
 from tests.helpers import assert_same_result
 
 pytestmark = pytest.mark.gpu
@@ -67,3 +67,55 @@ def test_wide_operators_run_on_the_column_kernels(require_gpu, distances, topk, 
     want = unfused(lambda: global_spai.mr(a, **kw))
     assert_same_result(got, want, f"{distances} {precision}, launched one by one")
     assert_same_result(global_spai.mr(a, **kw), want, f"{distances} {precision}, as a graph")
+
+
+def shuffled(a, span, seed=1):
+    """Rows and columns permuted within blocks of `span`: adjacent columns share no rows, inside the window."""
+    n = a.shape[0]
+    rng = np.random.default_rng(seed)
+    p = np.concatenate([lo + rng.permutation(min(span, n - lo)) for lo in range(0, n, span)])
+    a = sparse.csc_matrix(a[p][:, p])
+    a.sort_indices()
+    return a
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_scattered_columns_leave_the_groups(require_gpu, precision):
+    a = shuffled(problems.diffusion_3d(22, 1.0, 5), 2000)
+    topk = 20
+    kw = dict(M0=problems.diagonal_inverse(a), max_iterations=8, tolerance=0.0, max_density=topk / a.shape[0],
+              topk_per_column=topk, precision=precision)
+    want = unfused(lambda: global_spai.mr(a, **kw))
+    got, counts = profiled(lambda: global_spai.mr(a, **kw), "fused_drop", "fused_drop_columns")
+    # the first steps' columns are short enough for groups, the later ones are not
+    assert counts["fused_drop"][0] > 0 and counts["fused_drop_columns"][0] > 0
+    assert counts["fused_drop"][0] + counts["fused_drop_columns"][0] == 8
+    assert_same_result(got, want, f"{precision}, launched one by one")
+    assert_same_result(global_spai.mr(a, **kw), want, f"{precision}, as graphs")
+    # a second run on the same problem starts column by column
+    session = Session("global_spai", "mr", a, **kw)
+    session.run()
+    first = session.result()
+    _, counts = profiled(session.run, "fused_drop", "fused_drop_columns")
+    assert counts["fused_drop"][0] == 0 and counts["fused_drop_columns"][0] == 8
+    assert_same_result(first, want, f"{precision}, first run")
+    assert_same_result(session.result(), want, f"{precision}, second run")
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_scattered_systems_of_a_batch_leave_the_groups(require_gpu, precision):
+    batch = [shuffled(problems.diffusion_3d(22, 1.0, 5), 2000), problems.diffusion_2d(30, 1.0, 2)]
+    kw = dict(max_iterations=7, tolerance=0.0, max_density=1.0, topk_per_column=20, precision=precision)
+    want = unfused(lambda: global_spai.mr_batched(batch, **kw))
+    got, counts = profiled(lambda: global_spai.mr_batched(batch, **kw), "fused_drop", "fused_drop_columns")
+    assert counts["fused_drop"][0] > 0 and counts["fused_drop_columns"][0] > 0
+    for b, (g, w) in enumerate(zip(got, want)):
+        assert_same_result(g, w, f"{precision} system {b}")
+
+
+def test_grids_stay_in_groups(require_gpu):
+    a = problems.diffusion_3d(22, 1.0, 5)
+    kw = dict(M0=problems.diagonal_inverse(a), max_iterations=8, tolerance=0.0, max_density=16 / a.shape[0],
+              topk_per_column=16)
+    _, counts = profiled(lambda: global_spai.mr(a, **kw), "fused_drop", "fused_drop_columns")
+    assert counts["fused_drop"][0] == 8 and counts["fused_drop_columns"][0] == 0
