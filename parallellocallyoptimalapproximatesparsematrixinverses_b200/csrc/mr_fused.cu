@@ -1543,6 +1543,7 @@ __global__ void __launch_bounds__(kGroupWarps * kWarp) FusedResidualKernel(const
   unsigned char* base = fused_res_smem + (threadIdx.x >> 5) * a.residual_bytes;
   const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  if (a.state->overflow != 0) return;  // the step is void: M^T and Z stay what it started from
   const int64_t read_set = a.state->parity;  // the M^T set the drop kernel has just read
   unsigned long long written = 0;
   unsigned int unfit = 0;
@@ -1581,6 +1582,7 @@ __global__ void __launch_bounds__(kColumnWarps * kWarp)
   unsigned char* base = fused_res_smem + (threadIdx.x >> 5) * a.residual_bytes;
   const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  if (a.state->overflow != 0) return;  // the step is void: M^T and Z stay what it started from
   const int64_t read_set = a.state->parity;  // the M^T set the drop kernel has just read
   unsigned long long written = 0;
   const ResidualSlab<T> slab(a, base, true, lane);
@@ -1727,9 +1729,10 @@ __global__ void ToSlotsKernel(CscView<T> x, int cap, int32_t* __restrict__ rows,
   if (overflow != 0) atomicOr(&state->overflow, overflow);
 }
 
-// A batched step is over: the M^T sets change places (the decide kernel's part in single runs).
+// A batched step is over: the M^T sets change places (the decide kernel's part
+// in single runs), unless the step is void.
 __global__ void FlipKernel(FusedState* __restrict__ state) {
-  state->parity ^= 1;
+  if (state->overflow == 0) state->parity ^= 1;
   state->last_unfit = state->unfit;
   state->unfit = 0u;
 }
@@ -1898,6 +1901,15 @@ class FusedMr final : public FusedMrBase {
 
   void CompactBatch(Ctx& ctx, void* m_csc) override { CompactM(ctx, *static_cast<DevCsc<T>*>(m_csc)); }
 
+  void RecoverBatch(Ctx& ctx, void* m_csc, void* z_csc) override {
+    // the drop kernel has overwritten M's columns, but not the M^T it read
+    const int64_t set = host_state_->parity;
+    DevCsc<T> mt;
+    Compact(ctx, args_.cap_mt, args_.mt_cols[set], args_.mt_vals[set], args_.mt_cnt[set], mt);
+    Transpose(ctx, mt, *static_cast<DevCsc<T>*>(m_csc));
+    Compact(ctx, args_.cap_z, args_.z_rows, args_.z_vals, args_.z_cnt, *static_cast<DevCsc<T>*>(z_csc));
+  }
+
  private:
   // The slots filled from M and Z, the state at iteration 0 (M^T set 0 current).
   void Start(Ctx& ctx, const FusedMrProblem& problem, const DevCsc<T>& m, const DevCsc<T>& z, double alpha,
@@ -1923,20 +1935,23 @@ class FusedMr final : public FusedMrBase {
   }
 
   // M back to compact CSC.
-  void CompactM(Ctx& ctx, DevCsc<T>& m) {
+  void CompactM(Ctx& ctx, DevCsc<T>& m) { Compact(ctx, args_.topk, args_.m_rows, args_.m_vals, args_.m_cnt, m); }
+
+  // Slots to compact columns, each column's entries in slot order.
+  void Compact(Ctx& ctx, int cap, const int32_t* rows, const T* vals, const int32_t* cnt, DevCsc<T>& out) {
     const cudaStream_t st = ctx.stream;
     const int64_t n = args_.n;
     DevCsc<T> result;
     result.Shape(n, n, st);
     ctx.counts.Reserve(static_cast<size_t>(n + 1), st);
-    WidenCountsKernel<<<GridFor(n, 256), 256, 0, st>>>(args_.m_cnt, n, ctx.counts.data());
+    WidenCountsKernel<<<GridFor(n, 256), 256, 0, st>>>(cnt, n, ctx.counts.data());
     SPAI_LAUNCH_CHECK();
     const int64_t nnz = ScanCounts(ctx, ctx.counts.data(), n, result.ptr.data());
     result.ReserveNnz(nnz, st);
-    FromSlotsKernel<T><<<GridFor(n, 128), 128, 0, st>>>(n, args_.topk, args_.m_rows, args_.m_vals, result.ptr.data(),
-                                                        result.idx.data(), result.val.data());
+    FromSlotsKernel<T><<<GridFor(n, 128), 128, 0, st>>>(n, cap, rows, vals, result.ptr.data(), result.idx.data(),
+                                                        result.val.data());
     SPAI_LAUNCH_CHECK();
-    m.Swap(result);
+    out.Swap(result);
   }
 
   // The same three kernels launched one by one with the library's CUDA-event

@@ -82,12 +82,15 @@ class FusedMrBase {
   // step): BeginBatch fills the slots (false: not applicable, nothing
   // changed), StepBatch runs the drop and residual kernels, BatchCounts
   // fetches the entries of M, then of Z, per segment of columns and returns
-  // false when a column outgrew its slots, CompactBatch writes M.
+  // false when a column outgrew its slots in that step, which then is void,
+  // CompactBatch writes M, and RecoverBatch, after a void step, the M and Z it
+  // started from (the last BeginBatch's when it was the first).
   virtual bool BeginBatch(Ctx& ctx, const FusedMrProblem& problem, const void* m_csc, const void* z_csc,
                           const double* alpha) = 0;
   virtual FusedBatchSums StepBatch(Ctx& ctx) = 0;
   virtual bool BatchCounts(Ctx& ctx, const int64_t* first, int64_t segments, int64_t* out_dev, int64_t* out) = 0;
   virtual void CompactBatch(Ctx& ctx, void* m_csc) = 0;
+  virtual void RecoverBatch(Ctx& ctx, void* m_csc, void* z_csc) = 0;
 };
 
 // Whether the fused loop can take the problem (slot and window capacities).

@@ -415,14 +415,10 @@ class Solver final : public SolverBase {
   // iteration limit) has its M copied out at that moment; afterwards it rides
   // along with step length 0 and its results are no longer read.
   // With per-column top-k the steps run on the fused kernels (mr_fused.cu) where
-  // those apply, with a step length per column; a column that outgrows their
-  // slots sends the whole batch through the unfused ones, which give the same bits.
+  // those apply, with a step length per column.  When a column outgrows their
+  // slots, that step and the following ones run on the unfused kernels, which
+  // give the same bits.
   void RunMrBatched(const std::vector<int64_t>& offsets, std::vector<SolveOutput>& outputs) override {
-    if (!RunBatch(offsets, outputs, true)) RunBatch(offsets, outputs, false);
-  }
-
-  // False when the fused steps had to be given up (outputs are then incomplete).
-  bool RunBatch(const std::vector<int64_t>& offsets, std::vector<SolveOutput>& outputs, bool allow_fused) {
     const int64_t blocks = static_cast<int64_t>(offsets.size()) - 1;
     if (blocks <= 0 || offsets.front() != 0 || offsets.back() != n_) throw std::invalid_argument("bad block offsets");
     if (!pr_diagonal_) throw std::invalid_argument("batched runs use a diagonal Pr");
@@ -569,7 +565,7 @@ class Solver final : public SolverBase {
     DevCsc<T> scaled;
     DevBuf<int64_t> counts_dev;
     std::vector<double> three(static_cast<size_t>(3 * blocks));
-    if (live > 0 && allow_fused && FusedMrEnabled() && opt_.dropping && opt_.topk > 0 && ell_width_ > 0) {
+    if (live > 0 && FusedMrEnabled() && opt_.dropping && opt_.topk > 0 && ell_width_ > 0) {
       if (!fused_) fused_ = MakeFusedMr<T>();
       for (int64_t b = 0; b < blocks; ++b) direction[b] = z_at[b + 1] - z_at[b];
       const FusedMrProblem problem = FusedProblem();
@@ -602,15 +598,19 @@ class Solver final : public SolverBase {
         const FusedBatchSums step = fused_->StepBatch(ctx_);
         const double* parts[3] = {step.residual, step.num, step.den};
         tree.Sums(ctx_, parts, 3, three.data());
-        if (!fused_->BatchCounts(ctx_, bounds_dev.data(), blocks, counts_dev.data(), slot_counts.data())) return false;
-        for (int64_t b = 0; b < blocks; ++b) {
-          residual[b] = std::sqrt(three[b]);
-          num[b] = three[blocks + b];
-          den[b] = three[2 * blocks + b];
+        fused = fused_->BatchCounts(ctx_, bounds_dev.data(), blocks, counts_dev.data(), slot_counts.data());
+        if (fused) {
+          for (int64_t b = 0; b < blocks; ++b) {
+            residual[b] = std::sqrt(three[b]);
+            num[b] = three[blocks + b];
+            den[b] = three[2 * blocks + b];
+          }
+          append(residual);
+          for (int64_t b = 0; b < blocks; ++b) direction[b] = slot_counts[blocks + b];
+          continue;
         }
-        append(residual);
-        for (int64_t b = 0; b < blocks; ++b) direction[b] = slot_counts[blocks + b];
-        continue;
+        // the step again, unfused, from the M and Z it started from (before the first step m_ and z_ hold them)
+        if (i > 1) fused_->RecoverBatch(ctx_, &m_, &z_);
       }
       Copy(ctx_, z_, scaled);
       ScaleColumns(ctx_, scaled, alpha_col);
@@ -627,7 +627,6 @@ class Solver final : public SolverBase {
     }
     snapshot();
     ctx_.Sync();
-    return true;
   }
 
   int64_t iterations() const override { return iterations_; }

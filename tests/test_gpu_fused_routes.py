@@ -119,3 +119,36 @@ def test_grids_stay_in_groups(require_gpu):
               topk_per_column=16)
     _, counts = profiled(lambda: global_spai.mr(a, **kw), "fused_drop", "fused_drop_columns")
     assert counts["fused_drop"][0] == 8 and counts["fused_drop_columns"][0] == 0
+
+
+def tree(degree, depth):
+    """A tree's graph Laplacian, slightly shifted: the row of M at its root grows with every step."""
+    parent, frontier = [-1], [0]
+    for _ in range(depth):
+        grown = []
+        for p in frontier:
+            for _ in range(degree if p == 0 else degree - 1):
+                parent.append(p)
+                grown.append(len(parent) - 1)
+        frontier = grown
+    n = len(parent)
+    off = sparse.coo_matrix((-np.ones(n - 1), (np.arange(1, n), parent[1:])), shape=(n, n)).tocsr()
+    off = off + off.T
+    a = sparse.csc_matrix(off + sparse.diags(1.02 * np.asarray(abs(off).sum(axis=1)).ravel()))
+    a.sort_indices()
+    return a
+
+
+# the root's row of M has 5, 15 and 44 entries after the first steps, its slots are 32: the third step is void
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_a_batch_goes_on_from_the_step_that_outgrew_its_slots(require_gpu, precision):
+    batch = [problems.diffusion_2d(19, 0.5, 3), tree(4, 5), problems.tridiagonal(40)]
+    kw = dict(max_iterations=7, tolerance=0.0, max_density=1.0, topk_per_column=8, precision=precision)
+    names = ("fused_drop", "union")
+    want, unfused_counts = unfused(lambda: profiled(lambda: global_spai.mr_batched(batch, **kw), *names))
+    got, counts = profiled(lambda: global_spai.mr_batched(batch, **kw), *names)
+    assert counts["fused_drop"][0] == 3
+    per_step = unfused_counts["union"][0] // 7
+    assert per_step >= 1 and unfused_counts["union"][0] - counts["union"][0] == 2 * per_step
+    for b, (g, w) in enumerate(zip(got, want)):
+        assert_same_result(g, w, f"{precision} system {b}")
