@@ -1825,7 +1825,7 @@ class FusedMr final : public FusedMrBase {
     Start(ctx, problem, m, z, alpha, nullptr);
     FusedState out;
     if (prof::Enabled()) {
-      out = RunStepwise(ctx, problem, m.nnz, z.nnz);
+      out = RunStepwise(ctx, problem);
     } else {
       do {
         if (exec_ == nullptr) Capture();
@@ -1895,8 +1895,18 @@ class FusedMr final : public FusedMrBase {
     SPAI_CUDA(cudaMemcpyAsync(host_state_, state_.data(), sizeof(FusedState), cudaMemcpyDeviceToHost, st));
     SPAI_CUDA(cudaMemcpyAsync(out, out_dev, sizeof(int64_t) * 2 * segments, cudaMemcpyDeviceToHost, st));
     ctx.Sync();
+    if (host_state_->overflow != 0) return false;
+    if (prof::Enabled()) {
+      int64_t m_entries = 0;
+      int64_t z_entries = 0;
+      for (int64_t s = 0; s < segments; ++s) {
+        m_entries += out[s];
+        z_entries += out[segments + s];
+      }
+      AddStepBytes(problem_, static_cast<double>(m_entries), static_cast<double>(z_entries));
+    }
     if (host_state_->last_unfit > args_.unfit_limit) LeaveGroups(problem_);
-    return host_state_->overflow == 0;
+    return true;
   }
 
   void CompactBatch(Ctx& ctx, void* m_csc) override { CompactM(ctx, *static_cast<DevCsc<T>*>(m_csc)); }
@@ -1919,6 +1929,8 @@ class FusedMr final : public FusedMrBase {
     Reserve(ctx, problem);
     Configure(problem);
     args_.alpha = alpha_columns;
+    m_entries_ = static_cast<double>(m.nnz);
+    z_entries_ = static_cast<double>(z.nnz);
     FusedState init{};
     init.alpha = alpha;
     init.nnz_dir = static_cast<unsigned long long>(z.nnz);
@@ -1954,16 +1966,25 @@ class FusedMr final : public FusedMrBase {
     out.Swap(result);
   }
 
-  // The same three kernels launched one by one with the library's CUDA-event
-  // accounting around each (spai_profile_enable): the decide kernel's result
-  // is read back after every iteration, in place of the graph's condition.
-  FusedState RunStepwise(Ctx& ctx, const FusedMrProblem& p, int64_t m_nnz, int64_t z_nnz) {
-    const cudaStream_t st = ctx.stream;
+  // Algorithmic bytes of a step that left m_new entries in M and z_new in Z: the
+  // drop step reads M, Z and both transposes and writes M and M^T; the residual
+  // step reads M, A and Pr, writes Z, Z^T and the three column sums.
+  void AddStepBytes(const FusedMrProblem& p, double m_new, double z_new) {
     const double e = static_cast<double>(sizeof(T) + sizeof(int32_t));
     const double n = static_cast<double>(p.n);
     const double a_bytes = static_cast<double>(p.a_nnz) * e + 8.0 * (n + 1.0);
-    double m_prev = static_cast<double>(m_nnz);
-    double z_prev = static_cast<double>(z_nnz);
+    prof::AddBytes(drop_class_, e * (2.0 * m_entries_ + 2.0 * z_entries_ + 2.0 * m_new) + 4.0 * 6.0 * n);
+    prof::AddBytes(res_class_, e * m_new + a_bytes + sizeof(T) * n + 2.0 * e * z_new + 4.0 * 3.0 * n + 24.0 * n);
+    m_entries_ = m_new;
+    z_entries_ = z_new;
+  }
+
+  // The same three kernels launched one by one with the library's CUDA-event
+  // accounting around each (spai_profile_enable): the decide kernel's result
+  // is read back after every iteration, in place of the graph's condition.
+  FusedState RunStepwise(Ctx& ctx, const FusedMrProblem& p) {
+    const cudaStream_t st = ctx.stream;
+    const double n = static_cast<double>(p.n);
     FusedState out{};
     for (int64_t body = 0; body <= p.max_iterations; ++body) {
       {
@@ -1984,15 +2005,7 @@ class FusedMr final : public FusedMrBase {
       SPAI_CUDA(cudaMemcpyAsync(host_state_, state_.data(), sizeof(FusedState), cudaMemcpyDeviceToHost, st));
       ctx.Sync();
       out = *host_state_;
-      // algorithmic bytes: the drop step reads M, Z and both transposes and writes M and M^T; the
-      // residual step reads M, A and Pr, writes Z, Z^T and the three column sums
-      const double m_new = static_cast<double>(out.last_nnz_m);
-      const double z_new = static_cast<double>(out.last_nnz_z);
-      prof::AddBytes(drop_class_, e * (2.0 * m_prev + 2.0 * z_prev + 2.0 * m_new) + 4.0 * 6.0 * n);
-      prof::AddBytes(res_class_,
-                     e * m_new + a_bytes + sizeof(T) * n + 2.0 * e * z_new + 4.0 * 3.0 * n + 24.0 * n);
-      m_prev = m_new;
-      z_prev = z_new;
+      AddStepBytes(p, static_cast<double>(out.last_nnz_m), static_cast<double>(out.last_nnz_z));
       if (out.stop == kScatteredStop) {
         LeaveGroups(p);
       } else if (out.stop != kRunning) {
@@ -2281,6 +2294,8 @@ class FusedMr final : public FusedMrBase {
   void (*res_kernel_)(const FusedArgs<T>) = nullptr;
   void (*drop_kernel_)(const FusedArgs<T>) = nullptr;
   FusedMrProblem problem_;   // of the running batch
+  double m_entries_ = 0.0;   // entries of M and Z that the next step starts from
+  double z_entries_ = 0.0;
   bool scattered_ = false;   // the problem's column groups do not fit
   int columns_ = 1;  // per warp
   int warps_ = 1;    // per block

@@ -152,3 +152,15 @@ def test_a_batch_goes_on_from_the_step_that_outgrew_its_slots(require_gpu, preci
     assert per_step >= 1 and unfused_counts["union"][0] - counts["union"][0] == 2 * per_step
     for b, (g, w) in enumerate(zip(got, want)):
         assert_same_result(g, w, f"{precision} system {b}")
+
+
+def test_batched_steps_account_for_their_bytes(require_gpu):
+    """A batch of one system moves what the system alone moves."""
+    a = problems.diffusion_2d(40, 0.5, 3)
+    kw = dict(max_iterations=6, tolerance=0.0, max_density=1.0, topk_per_column=8)
+    names = ("fused_drop", "fused_residual")
+    _, alone = profiled(lambda: global_spai.mr(a, **kw), *names)
+    _, batch = profiled(lambda: global_spai.mr_batched([a], **kw), *names)
+    for name in names:
+        assert alone[name][0] == batch[name][0] == 6
+        assert alone[name][1] == batch[name][1] > 0
