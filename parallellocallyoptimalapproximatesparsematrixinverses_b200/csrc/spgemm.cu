@@ -328,6 +328,8 @@ struct ValuesArgs {
   CscView<T> x_csr;
   CscView<T> b;
   const int64_t* c_ptr;  // output (or mask) column offsets
+  int64_t entries;       // in all columns
+  int64_t piece;         // entries of a column that one warp takes at a time (a multiple of 32)
   const int32_t* rows;   // and rows
   int mode;
   bool prune;
@@ -343,7 +345,7 @@ __host__ __device__ inline size_t ValuesSlabBytes(int words) {
   return Round16(static_cast<size_t>(words) * 4) + Round16(static_cast<size_t>(words) * 2);
 }
 
-constexpr int kValuesPiece = 4096;  // entries of a column that one warp takes at a time
+constexpr int kValuesPiece = 4096;  // entries of a column that one warp takes at a time, at most
 constexpr int kValuesMaxWords = 1024;
 
 // Warp per output column: lane r forms output rows r, r + 32, ... in ascending
@@ -354,7 +356,9 @@ constexpr int kValuesMaxWords = 1024;
 // is searched by bisection, as every column was: eight searches in lock step
 // per thread and output entry took 1,330 us for 4,096 columns of about 3,000
 // entries with 1,300 entries in B's column.
-template <class T>
+// kShort: the columns are split into pieces of a.piece entries over gridDim.y
+// warps each (LaunchValues).
+template <class T, bool kShort>
 __global__ void __launch_bounds__(256) ValuesKernel(ValuesArgs<T> a, int words_cap) {
   extern __shared__ __align__(16) unsigned char values_smem[];
   const int lane = threadIdx.x & 31;
@@ -363,6 +367,7 @@ __global__ void __launch_bounds__(256) ValuesKernel(ValuesArgs<T> a, int words_c
   uint16_t* first = reinterpret_cast<uint16_t*>(base + Round16(static_cast<size_t>(words_cap) * 4));
   ClearWords(bits, words_cap, lane);
   __syncwarp();
+  const int64_t piece = kShort ? a.piece : kValuesPiece;
   bool zero_seen = false;
   const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
@@ -372,7 +377,7 @@ __global__ void __launch_bounds__(256) ValuesKernel(ValuesArgs<T> a, int words_c
     const int32_t* b_idx = a.b.idx + bs;
     const T* b_val = a.b.val + bs;
     // blockIdx.y takes every gridDim.y-th piece of the column's entries
-    const int64_t begin = a.c_ptr[j] + static_cast<int64_t>(blockIdx.y) * kValuesPiece;
+    const int64_t begin = a.c_ptr[j] + static_cast<int64_t>(blockIdx.y) * piece;
     const int64_t end = a.c_ptr[j + 1];
     if (begin >= end) return;
     const int32_t w0 = blen > 0 ? b_idx[0] >> 5 : 0;
@@ -387,13 +392,13 @@ __global__ void __launch_bounds__(256) ValuesKernel(ValuesArgs<T> a, int words_c
       }
       __syncwarp();
     }
-    const int64_t skip = static_cast<int64_t>(gridDim.y - 1) * kValuesPiece;
-    int64_t piece_end = min(begin + kValuesPiece, end);
+    const int64_t skip = static_cast<int64_t>(gridDim.y - 1) * piece;
+    int64_t piece_end = min(begin + piece, end);
     for (int64_t p = begin + lane; p < end; p += kWarp) {
       if (p >= piece_end) {  // pieces are whole rounds of 32: every lane moves on together
         p += skip;
         if (p >= end) break;
-        piece_end = min(p - lane + kValuesPiece, end);
+        piece_end = min(p - lane + piece, end);
       }
       const int32_t i = a.rows[p];
       const int64_t xs = a.x_csr.ptr[i];
@@ -472,14 +477,14 @@ __global__ void __launch_bounds__(256) ValuesKernel(ValuesArgs<T> a, int words_c
       __syncwarp();
     }
   };
-  if (blockIdx.y == 0) {
+  if (kShort || blockIdx.y == 0) {
     for (int64_t j = warp; j < a.b.cols; j += warps) column(j);
   } else {
     // the few columns long enough to have a piece for this split
     for (int64_t j0 = warp * kWarp; j0 < a.b.cols; j0 += warps * kWarp) {
       const int64_t j = j0 + lane;
       const int64_t len = j < a.b.cols ? a.c_ptr[j + 1] - a.c_ptr[j] : 0;
-      for (unsigned left = __ballot_sync(0xffffffffu, len > static_cast<int64_t>(blockIdx.y) * kValuesPiece); left != 0u;
+      for (unsigned left = __ballot_sync(0xffffffffu, len > static_cast<int64_t>(blockIdx.y) * piece); left != 0u;
            left &= left - 1u) {
         column(j0 + __ffs(left) - 1);
       }
@@ -554,17 +559,30 @@ __global__ void __launch_bounds__(256) MaskedEntriesKernel(CscView<T> x_csr, Csc
 }
 
 template <class T>
-void LaunchValues(Ctx& ctx, const ValuesArgs<T>& args) {
+void LaunchValues(Ctx& ctx, ValuesArgs<T> args) {
   // a bitmap over all rows of B, up to 32,768 of them (wider ones would cost resident warps)
   const int words = static_cast<int>(std::min<int64_t>(kValuesMaxWords, CeilDiv(args.b.rows, 32) + 1));
   constexpr int kWarps = 8;
   const size_t smem = ValuesSlabBytes(words) * kWarps;
-  SPAI_CUDA(cudaFuncSetAttribute(ValuesKernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(ValuesSlabBytes(kValuesMaxWords) * kWarps)));
+  const int64_t cols = args.b.cols;
   // a column long enough to keep a warp busy for long is split over up to eight
-  const unsigned split = static_cast<unsigned>(std::min<int64_t>(8, CeilDiv(args.x_csr.cols, 2 * kValuesPiece)));
-  const dim3 grid(static_cast<unsigned>(GridFor(args.b.cols * kWarp, kWarps * kWarp)), split);
-  ValuesKernel<T><<<grid, kWarps * kWarp, smem, ctx.stream>>>(args, words);
+  auto kernel = ValuesKernel<T, false>;
+  int64_t split = std::min<int64_t>(8, CeilDiv(args.x_csr.cols, 2 * kValuesPiece));
+  if (cols < int64_t{12} * ctx.sm_count) {
+    // Too few columns to fill the chip: pieces for about 32 warps an SM.
+    // Full columns in FP64, nine products: 0.20, 5.1, 44 and 116 ms at n = 100,
+    // 400, 800 and 1,200, with a warp a column 0.57, 11.7, 61 and 192 (a thread
+    // an entry, before there were bitmaps, 0.38, 6.5, 51 and 157).  At 2,300
+    // columns a warp each takes 451 ms and pieces 472.
+    kernel = ValuesKernel<T, true>;
+    args.piece = std::clamp<int64_t>(CeilDiv(CeilDiv(args.entries, int64_t{32} * ctx.sm_count), kWarp) * kWarp, kWarp,
+                                     kValuesPiece);
+    split = std::clamp<int64_t>(CeilDiv(CeilDiv(args.entries, cols), args.piece), 1, 32);
+  }
+  SPAI_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(ValuesSlabBytes(kValuesMaxWords) * kWarps)));
+  const dim3 grid(static_cast<unsigned>(GridFor(cols * kWarp, kWarps * kWarp)), static_cast<unsigned>(split));
+  kernel<<<grid, kWarps * kWarp, smem, ctx.stream>>>(args, words);
   SPAI_LAUNCH_CHECK();
 }
 
@@ -1356,6 +1374,7 @@ bool Spgemm(Ctx& ctx, const DevCsc<T>& x_csc, const DevCsc<T>& x_csr, const DevC
       va.x_csr = View(x_csr);
       va.b = View(b);
       va.c_ptr = c_ptr;
+      va.entries = nnz;
       va.rows = rows;
       va.mode = static_cast<int>(mode);
       va.prune = prune;
@@ -1416,6 +1435,7 @@ void SpgemmMasked(Ctx& ctx, const DevCsc<T>& x_csr, const DevCsc<T>& b, const De
   va.x_csr = View(x_csr);
   va.b = View(b);
   va.c_ptr = mask.ptr.data();
+  va.entries = mask.nnz;
   va.rows = mask.idx.data();
   va.mode = static_cast<int>(ValueMode::kMasked);
   va.out_f64 = out;
