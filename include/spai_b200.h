@@ -302,6 +302,12 @@ void* spai_session_stream(SpaiSession* session);
  * path and releases what it held; the library stays usable. */
 void spai_inject_allocation_failure(int64_t after);
 
+/* Fault injection for tests: the blocks of the next PCG solve wait `ns`
+ * nanoseconds for one another (plus what the longest row of A and M may take)
+ * instead of seconds, after which the solve ends with an error (once; negative:
+ * as usual). */
+void spai_inject_pcg_wait(int64_t ns);
+
 /* The device's minimum-norm 2x2 least-squares solve (the per-column step of
  * Inner-Outer LOMR, reference src/common/sparse_operations.cpp:58-73) on
  * `count` systems: gram holds 4 doubles per system (row-major), rhs 2, out

@@ -85,7 +85,7 @@ EXPORTED_SYMBOLS = (
     "spai_pcg_device", "spai_pcg_adjoint_device", "spai_residual_adjoint_device",
     "spai_mr_batched", "spai_mtx_read", "spai_mtx_write", "spai_free_int64_array", "spai_free_double_array",
     "spai_session_create_device", "spai_session_result_device", "spai_inject_allocation_failure",
-    "spai_set_fused_mr", "spai_solve_2x2_device",
+    "spai_set_fused_mr", "spai_solve_2x2_device", "spai_inject_pcg_wait",
 )
 
 _lib = None
@@ -138,6 +138,8 @@ def _declare(lib) -> None:
                                             ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                             ctypes.c_void_p, _i64, _f64, _i64, ctypes.c_void_p, _pf64, _pi64,
                                             ctypes.c_char_p, _i64]
+    lib.spai_inject_pcg_wait.restype = None
+    lib.spai_inject_pcg_wait.argtypes = [_i64]
     lib.spai_inject_allocation_failure.restype = None
     lib.spai_inject_allocation_failure.argtypes = [_i64]
     lib.spai_set_fused_mr.restype = None

@@ -495,6 +495,8 @@ void free_mem(Result* result) {
 
 void spai_inject_allocation_failure(int64_t after) { spai::g_fail_after.store(after, std::memory_order_relaxed); }
 
+void spai_inject_pcg_wait(int64_t ns) { spai::SetNextPcgWait(ns); }
+
 namespace spai {
 namespace {
 // The device's 2x2 minimum-norm solve (the Inner-Outer LOMR step) on `count` systems.

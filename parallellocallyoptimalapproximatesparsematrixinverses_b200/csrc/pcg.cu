@@ -28,7 +28,9 @@
 // about 1,200 cycles, so it runs beside the folding), the chunk sums go to
 // global memory as 16-byte words that carry the reduction's number, and every
 // block polls both and folds the tree's next level itself.  The polls are
-// bounded: a block that gives up poisons the counter, every other block sees
+// bounded, in seconds and by the longest row that one thread walks (a count of
+// polls alone abandoned solves with rows of millions of entries): a block that
+// gives up poisons the counter, every other block sees
 // that at its next reduction, and the solve ends with an error.  Every block
 // decides the recurrence's scalars from the totals; the history keeps ||r||^2
 // until the end, so that no square root or division is on the way to the next
@@ -52,6 +54,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -75,7 +78,12 @@ namespace cg = cooperative_groups;
 constexpr int kClusterBlocks = 8;   // kTreeLanes / kWarp: one warp-wide group of tree lanes per block
 constexpr int kSolveThreads = kWarp * kTreeTerms;  // one warp per term of a lane
 constexpr int kGroupRounds = 4;     // chunks of a cluster folded at a time
-constexpr unsigned kPollLimit = 1u << 22;       // polls (seconds) before the solve is abandoned
+constexpr unsigned long long kWaitNs = 4'000'000'000ull;  // how long a block waits for others before the solve is abandoned
+// What the longest row adds to it: one thread walks a row, and an entry takes
+// it up to 0.3 us (two dependent loads for four entries).  Rows up to
+// kShortWalk entries are covered anyway.
+constexpr unsigned long long kWaitNsPerEntry = 2000;
+constexpr int64_t kShortWalk = 65536;
 constexpr unsigned long long kPoison = 1ull << 63;  // set in a cluster's counter by a block that gave up
 constexpr int kFlagStride = 16;                 // counters 128 bytes apart
 static_assert(kClusterBlocks * kWarp == kTreeLanes, "a cluster covers a chunk's lanes");
@@ -121,6 +129,9 @@ struct SolveArgs {
   SolveOutcome* outcome;
   int64_t n;
   int64_t chunks;
+  unsigned long long* longest;  // entries that one thread walks per reduction, at most; 0 up to kShortWalk
+  unsigned long long wait_ns;   // a block's patience with others
+  unsigned free_polls;          // polls before it looks at the clock
   int64_t max_iterations;
   int64_t refresh_period;
   double tolerance;
@@ -153,9 +164,10 @@ __device__ __forceinline__ int SliceWidth(const SolveMatrix<TV>& m, int64_t row,
 
 // Copies the 32 rows of a slice, one per lane, into the sliced layout when
 // that wastes at most half of it (the copy then never exceeds twice the
-// entries plus two per row, what the host reserves).
+// entries plus two per row, what the host reserves).  Returns the lane's row's
+// length.
 template <class TV>
-__device__ void SliceRows(const SolveMatrix<TV>& m, int64_t slice, int64_t n, int lane) {
+__device__ int SliceRows(const SolveMatrix<TV>& m, int64_t slice, int64_t n, int lane) {
   int64_t first;
   int len;
   bool dense;
@@ -170,6 +182,7 @@ __device__ void SliceRows(const SolveMatrix<TV>& m, int64_t slice, int64_t n, in
     }
   }
   if (lane == 0) m.slice[slice] = at;
+  return len;
 }
 
 template <class TV>
@@ -299,16 +312,29 @@ __device__ __forceinline__ void ExpectBytes(uint64_t* barrier, unsigned bytes) {
                : "memory");
 }
 
+// Whether a wait that began at *start (0: now) has run out.  Out of line: a wait
+// comes here only after thousands of polls, and the polls are on the way to the
+// next iteration (inline, solves of one or a few chunks took 2 % longer).
+__device__ __noinline__ bool WaitExpired(unsigned long long* start, unsigned long long limit_ns,
+                                         const unsigned long long* longest) {
+  unsigned long long now;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+  if (*start == 0) *start = now;
+  return now - *start >= limit_ns && now - *start >= limit_ns + kWaitNsPerEntry * LoadAcquire(longest);
+}
+
 // False when the barrier's phase did not end within the limit.
-__device__ __forceinline__ bool WaitPhase(uint64_t* barrier, unsigned parity) {
+__device__ __forceinline__ bool WaitPhase(uint64_t* barrier, unsigned parity, unsigned free_polls,
+                                          unsigned long long limit_ns, const unsigned long long* longest) {
   const uint32_t at = SharedAddress(barrier);
-  for (unsigned polls = 0; polls < kPollLimit; ++polls) {
+  unsigned long long start = 0;
+  for (unsigned polls = 0;;) {
     unsigned ended;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
                  "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ended) : "r"(at), "r"(parity) : "memory");
     if (ended) return true;
+    if (++polls >= free_polls && WaitExpired(&start, limit_ns, longest)) return false;
   }
-  return false;
 }
 
 // Shared memory of a block.
@@ -344,6 +370,7 @@ __global__ void __launch_bounds__(kSolveThreads, kOneRound ? 1 : 2) PcgSolveKern
   unsigned group_count = 0;        // groups of rounds folded so far
   unsigned long long reduction = 0;  // number of the running reduction, from 1
   bool aborted = false;
+  int64_t walk = 0;  // entries this thread walks per reduction, at most
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
@@ -363,6 +390,7 @@ __global__ void __launch_bounds__(kSolveThreads, kOneRound ? 1 : 2) PcgSolveKern
     bool dense;
     const int wa = SliceWidth(a.a, row, n, &first_a, &row_a.len, &dense);
     const int wm = SliceWidth(a.m, row, n, &first_m, &row_m.len, &dense);
+    walk = row_a.len > row_m.len ? row_a.len : row_m.len;
     constexpr int kEntryA = sizeof(double) + sizeof(int32_t);
     constexpr int kEntryM = sizeof(TM) + sizeof(int32_t);
     // bytes of the 16 warps' slices (saturated: long rows never fit)
@@ -409,15 +437,18 @@ __global__ void __launch_bounds__(kSolveThreads, kOneRound ? 1 : 2) PcgSolveKern
       }
     }
   } else {
+    int64_t walk_m = 0;
     for (int64_t c = mine; c < a.chunks; c += clusters) {
       const int64_t first = c * kTreeChunk + in_chunk - lane;
       if (first < n) {
-        SliceRows(a.a, first >> 5, n, lane);
-        SliceRows(a.m, first >> 5, n, lane);
+        walk += SliceRows(a.a, first >> 5, n, lane);
+        walk_m += SliceRows(a.m, first >> 5, n, lane);
       }
     }
+    walk = walk > walk_m ? walk : walk_m;
     __syncwarp();
   }
+  if (walk > kShortWalk) atomicMax(a.longest, static_cast<unsigned long long>(walk));
   const auto a_row = [&](int64_t row) {
     if constexpr (kOneRound) {
       return row_a;
@@ -481,7 +512,9 @@ __global__ void __launch_bounds__(kSolveThreads, kOneRound ? 1 : 2) PcgSolveKern
             ExpectBytes(&sh.barrier[gp], static_cast<unsigned>(sizeof(double) * kTreeLanes) * dots * q);
           }
           if (warp < q * dots) {
-            if (!WaitPhase(&sh.barrier[gp], (group_count >> 1) & 1)) sh.abort = 1;
+            if (!WaitPhase(&sh.barrier[gp], (group_count >> 1) & 1, a.free_polls, a.wait_ns, a.longest)) {
+              sh.abort = 1;
+            }
             const int rq = dots == 2 ? warp >> 1 : warp;
             const int d = dots == 2 ? warp & 1 : 0;
             const double* from = lanes + ((gp * kRounds + rq) * 2 + d) * kTreeLanes;
@@ -514,6 +547,7 @@ __global__ void __launch_bounds__(kSolveThreads, kOneRound ? 1 : 2) PcgSolveKern
     }
     if (warp < dots) {
       const TaggedSum* sums = a.partial + (2 * parity + warp) * a.chunks;
+      unsigned long long start = 0;
       double v[kClusterBlocks];
       bool lost = false;
 #pragma unroll
@@ -522,7 +556,7 @@ __global__ void __launch_bounds__(kSolveThreads, kOneRound ? 1 : 2) PcgSolveKern
         for (int64_t i = kWarp * g + lane; i < a.chunks; i += kTreeLanes) {
           TaggedSum t = LoadTagged(sums + i);
           for (unsigned polls = 0; t.tag != reduction && !lost; t = LoadTagged(sums + i)) {
-            lost = ++polls >= kPollLimit;
+            lost = ++polls >= a.free_polls && WaitExpired(&start, a.wait_ns, a.longest);
           }
           s = Add(s, t.sum);
         }
@@ -534,13 +568,14 @@ __global__ void __launch_bounds__(kSolveThreads, kOneRound ? 1 : 2) PcgSolveKern
       if (lane == 0) sh.totals[parity][warp] = s;
     } else if (warp == 2) {
       for (int64_t c = lane; c < clusters; c += kWarp) {
+        unsigned long long start = 0;
         for (unsigned polls = 0;;) {
           const unsigned long long seen = LoadAcquire(a.arrived + c * kFlagStride);
           if (seen >= reduction * kClusterBlocks) {
             if (seen & kPoison) sh.abort = 1;
             break;
           }
-          if (++polls >= kPollLimit) {
+          if (++polls >= a.free_polls && WaitExpired(&start, a.wait_ns, a.longest)) {
             sh.abort = 1;
             break;
           }
@@ -752,6 +787,8 @@ constexpr size_t LaunchBytes() {
   return kOneRound ? kBlockSharedBytes : SolveBytes<false>();
 }
 
+std::atomic<int64_t> g_wait_ns{static_cast<int64_t>(kWaitNs)};  // the next solve's patience (SetNextPcgWait)
+
 // Clusters of the solve kernel that fit on the current device at once (asked once per device).
 template <class TM, bool kOneRound>
 int64_t ResidentClusters(int device) {
@@ -786,6 +823,8 @@ __global__ void SpmvKernel(CscView<TM> a, const double* __restrict__ x, double* 
 }
 
 }  // namespace
+
+void SetNextPcgWait(int64_t ns) { g_wait_ns.store(ns < 0 ? static_cast<int64_t>(kWaitNs) : ns); }
 
 template <class TM>
 void Spmv(Ctx& ctx, const DevCsc<TM>& a_rows, const double* x, double* y) {
@@ -825,9 +864,10 @@ void RunPcg(Ctx& ctx, const DevCsc<double>& a, const DevCsc<TM>& m, const double
   a_val.Reserve(a_room, st);
   m_idx.Reserve(m_room, st);
   m_val.Reserve(m_room, st);
-  // two slice cursors and the outcome, zeroed
+  // two slice cursors, the longest walk and the outcome, zeroed
   struct Control {
     unsigned long long used[2];
+    unsigned long long longest;
     SolveOutcome outcome;
   };
   DevBuf<Control> control;
@@ -852,6 +892,9 @@ void RunPcg(Ctx& ctx, const DevCsc<double>& a, const DevCsc<TM>& m, const double
   args.history = history.data();
   args.partial = partial.data();
   args.outcome = &c->outcome;
+  args.longest = &c->longest;
+  args.wait_ns = static_cast<unsigned long long>(g_wait_ns.exchange(static_cast<int64_t>(kWaitNs)));
+  args.free_polls = args.wait_ns == kWaitNs ? 4096 : 0;
   args.n = n;
   args.chunks = chunks;
   args.max_iterations = opt.max_iterations;

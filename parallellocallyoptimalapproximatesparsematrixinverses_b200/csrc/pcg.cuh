@@ -30,6 +30,10 @@ template <class TM>
 void RunPcg(Ctx& ctx, const DevCsc<double>& a_rows, const DevCsc<TM>& m_rows, const double* b, double* x,
             const PcgOptions& options, PcgResult& result);
 
+// Fault injection for tests (spai_inject_pcg_wait): how long the blocks of the
+// next solve wait for one another, in nanoseconds; negative: as usual.
+void SetNextPcgWait(int64_t ns);
+
 // y = A x for a row-compressed A (reference backward_error.pyx:27-34, per row sequential).
 template <class TM>
 void Spmv(Ctx& ctx, const DevCsc<TM>& a_rows, const double* x, double* y);
