@@ -78,12 +78,14 @@ namespace cg = cooperative_groups;
 constexpr int kClusterBlocks = 8;   // kTreeLanes / kWarp: one warp-wide group of tree lanes per block
 constexpr int kSolveThreads = kWarp * kTreeTerms;  // one warp per term of a lane
 constexpr int kGroupRounds = 4;     // chunks of a cluster folded at a time
-constexpr unsigned long long kWaitNs = 4'000'000'000ull;  // how long a block waits for others before the solve is abandoned
-// What the longest row adds to it: one thread walks a row, and an entry takes
+constexpr unsigned long long kWaitNs = 4'000'000'000ull;  // how long a block waits for other clusters
+constexpr unsigned long long kOwnWaitNs = 4 * kWaitNs;    // and for its own, whose blocks may be waiting so long
+// What the longest row adds to both: one thread walks a row, and an entry takes
 // it up to 0.3 us (two dependent loads for four entries).  Rows up to
 // kShortWalk entries are covered anyway.
 constexpr unsigned long long kWaitNsPerEntry = 2000;
 constexpr int64_t kShortWalk = 65536;
+constexpr unsigned kFreePolls = 4096;  // polls before a wait looks at the clock
 constexpr unsigned long long kPoison = 1ull << 63;  // set in a cluster's counter by a block that gave up
 constexpr int kFlagStride = 16;                 // counters 128 bytes apart
 static_assert(kClusterBlocks * kWarp == kTreeLanes, "a cluster covers a chunk's lanes");
@@ -130,7 +132,7 @@ struct SolveArgs {
   int64_t n;
   int64_t chunks;
   unsigned long long* longest;  // entries that one thread walks per reduction, at most; 0 up to kShortWalk
-  unsigned long long wait_ns;   // a block's patience with others
+  unsigned long long wait_ns;   // a block's patience with other clusters
   unsigned free_polls;          // polls before it looks at the clock
   int64_t max_iterations;
   int64_t refresh_period;
@@ -323,9 +325,12 @@ __device__ __noinline__ bool WaitExpired(unsigned long long* start, unsigned lon
   return now - *start >= limit_ns && now - *start >= limit_ns + kWaitNsPerEntry * LoadAcquire(longest);
 }
 
+__device__ __forceinline__ void StoreRemote(uint32_t remote, unsigned long long v) {
+  asm volatile("st.shared::cluster.u64 [%0], %1;" :: "r"(remote), "l"(v) : "memory");
+}
+
 // False when the barrier's phase did not end within the limit.
-__device__ __forceinline__ bool WaitPhase(uint64_t* barrier, unsigned parity, unsigned free_polls,
-                                          unsigned long long limit_ns, const unsigned long long* longest) {
+__device__ __forceinline__ bool WaitPhase(uint64_t* barrier, unsigned parity, const unsigned long long* longest) {
   const uint32_t at = SharedAddress(barrier);
   unsigned long long start = 0;
   for (unsigned polls = 0;;) {
@@ -333,7 +338,7 @@ __device__ __forceinline__ bool WaitPhase(uint64_t* barrier, unsigned parity, un
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
                  "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ended) : "r"(at), "r"(parity) : "memory");
     if (ended) return true;
-    if (++polls >= free_polls && WaitExpired(&start, limit_ns, longest)) return false;
+    if (++polls >= kFreePolls && WaitExpired(&start, kOwnWaitNs, longest)) return false;
   }
 }
 
@@ -341,9 +346,69 @@ __device__ __forceinline__ bool WaitPhase(uint64_t* barrier, unsigned parity, un
 struct alignas(16) SolveShared {
   double totals[2][2];                                         // [reduction parity][dot]
   uint64_t barrier[2];                                         // lane sums of a group have arrived
+  // The reduction after which a block of the cluster first gave up (none: all
+  // ones); that block writes it into every block of the cluster.
+  volatile unsigned long long first_dead;
   int widths[kTreeTerms];
-  int abort;
+  int abort;  // this block gives up
+  int leave;  // another one gave up a reduction ago
 };
+
+// A block's part in a reduction to which it adds nothing, without a wait for
+// other clusters (see the end of the kernel): `group_count` groups of rounds
+// have been folded before, and `reduction` is its number.
+__device__ __noinline__ void Farewell(unsigned char* smem, unsigned long long* arrived, TaggedSum* partial,
+                                      const unsigned long long* longest, int64_t chunks, int group_rounds,
+                                      unsigned group_count, unsigned long long reduction, int dots) {
+  SolveShared& sh = *reinterpret_cast<SolveShared*>(smem);
+  double* lanes = reinterpret_cast<double*>(smem + sizeof(SolveShared));
+  const int64_t clusters = gridDim.x / kClusterBlocks;
+  const int64_t mine = blockIdx.x / kClusterBlocks;
+  const int64_t rounds = (chunks - mine + clusters - 1) / clusters;
+  const int rank = static_cast<int>(cg::this_cluster().block_rank());
+  const bool solo = chunks == 1;
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const int rq = dots == 2 ? warp >> 1 : warp;
+  const int d = dots == 2 ? warp & 1 : 0;
+  const int parity = static_cast<int>(reduction & 1);
+  __syncthreads();
+  for (int64_t round = 0; round < rounds; round += group_rounds, ++group_count) {
+    const int q = static_cast<int>(rounds - round < group_rounds ? rounds - round : group_rounds);
+    const bool last = round + q == rounds;
+    const unsigned gp = group_count & 1;
+    if (last && !solo && threadIdx.x == 0) {
+      // after what thread 0 may have told the cluster's blocks
+      __threadfence();
+      atomicAdd(arrived + mine * kFlagStride, 1ull);
+    }
+    if (warp < q * dots) {
+      const uint32_t slot =
+          SharedAddress(lanes + ((gp * group_rounds + rq) * 2 + d) * kTreeLanes + kWarp * rank + lane);
+      const uint32_t barrier = SharedAddress(&sh.barrier[gp]);
+      for (int k = 0; k < (solo ? kClusterBlocks : 1); ++k) {
+        StoreCounted(RemoteAddress(slot, k), RemoteAddress(barrier, k), 0.0);
+      }
+    }
+    if (solo) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    if (solo || rank == 0) {
+      if (threadIdx.x == 0) {
+        ExpectBytes(&sh.barrier[gp], static_cast<unsigned>(sizeof(double) * kTreeLanes) * dots * q);
+      }
+      if (warp < q * dots) {
+        WaitPhase(&sh.barrier[gp], (group_count >> 1) & 1, longest);
+        if (lane == 0 && !solo) {
+          StoreTagged(partial + (2 * parity + d) * chunks + mine + (round + rq) * clusters, 0.0, reduction);
+        }
+      }
+    }
+    if (solo) {
+      asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    } else if (!last) {
+      cg::this_cluster().sync();
+    }
+  }
+}
 
 // kOneRound: every cluster owns one chunk, one block per SM, and the matrices'
 // rows stay in shared memory where they fit (latency counts); otherwise two
@@ -366,7 +431,6 @@ __global__ void __launch_bounds__(kSolveThreads, kOneRound ? 1 : 2) PcgSolveKern
   const int64_t in_chunk = static_cast<int64_t>(kTreeLanes) * warp + kWarp * rank + lane;
   const int64_t n = a.n;
   const int64_t rounds = (a.chunks - mine + clusters - 1) / clusters;
-  const int64_t groups = kOneRound ? 1 : (rounds + kRounds - 1) / kRounds;
   unsigned group_count = 0;        // groups of rounds folded so far
   unsigned long long reduction = 0;  // number of the running reduction, from 1
   bool aborted = false;
@@ -376,7 +440,9 @@ __global__ void __launch_bounds__(kSolveThreads, kOneRound ? 1 : 2) PcgSolveKern
     for (int i = 0; i < 2; ++i) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(SharedAddress(&sh.barrier[i])) : "memory");
     }
+    sh.first_dead = ~0ull;
     sh.abort = 0;
+    sh.leave = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
 
@@ -512,9 +578,7 @@ __global__ void __launch_bounds__(kSolveThreads, kOneRound ? 1 : 2) PcgSolveKern
             ExpectBytes(&sh.barrier[gp], static_cast<unsigned>(sizeof(double) * kTreeLanes) * dots * q);
           }
           if (warp < q * dots) {
-            if (!WaitPhase(&sh.barrier[gp], (group_count >> 1) & 1, a.free_polls, a.wait_ns, a.longest)) {
-              sh.abort = 1;
-            }
+            if (!WaitPhase(&sh.barrier[gp], (group_count >> 1) & 1, a.longest)) sh.abort = 1;
             const int rq = dots == 2 ? warp >> 1 : warp;
             const int d = dots == 2 ? warp & 1 : 0;
             const double* from = lanes + ((gp * kRounds + rq) * 2 + d) * kTreeLanes;
@@ -542,7 +606,7 @@ __global__ void __launch_bounds__(kSolveThreads, kOneRound ? 1 : 2) PcgSolveKern
       __syncthreads();
       t0 = sh.totals[parity][0];
       t1 = sh.totals[parity][1];
-      aborted = sh.abort != 0;
+      aborted = sh.abort != 0 || sh.first_dead < reduction;
       return;
     }
     if (warp < dots) {
@@ -568,25 +632,30 @@ __global__ void __launch_bounds__(kSolveThreads, kOneRound ? 1 : 2) PcgSolveKern
       if (lane == 0) sh.totals[parity][warp] = s;
     } else if (warp == 2) {
       for (int64_t c = lane; c < clusters; c += kWarp) {
+        // The own cluster's blocks always arrive, dead or alive, and once they
+        // have, what a dead one told this block is visible.
+        const bool own = c == mine;
         unsigned long long start = 0;
         for (unsigned polls = 0;;) {
           const unsigned long long seen = LoadAcquire(a.arrived + c * kFlagStride);
-          if (seen >= reduction * kClusterBlocks) {
+          // a poisoned counter reads as full, but for the own cluster's
+          if ((own ? seen & ~kPoison : seen) >= reduction * kClusterBlocks) {
             if (seen & kPoison) sh.abort = 1;
             break;
           }
-          if (++polls >= a.free_polls && WaitExpired(&start, a.wait_ns, a.longest)) {
+          if (++polls >= (own ? kFreePolls : a.free_polls) &&
+              WaitExpired(&start, own ? kOwnWaitNs : a.wait_ns, a.longest)) {
             sh.abort = 1;
             break;
           }
         }
+        if (own && sh.first_dead < reduction) sh.leave = 1;
       }
     }
     __syncthreads();
     t0 = sh.totals[parity][0];
     t1 = sh.totals[parity][1];
-    aborted = sh.abort != 0;
-    if (aborted && threadIdx.x == 0) atomicOr(a.arrived + mine * kFlagStride, kPoison);
+    aborted = (sh.abort | sh.leave) != 0;
   };
 
   double t0 = 0.0;
@@ -616,6 +685,7 @@ __global__ void __launch_bounds__(kSolveThreads, kOneRound ? 1 : 2) PcgSolveKern
   int64_t status = 0;
   bool done = !(1 < a.max_iterations && 1.0 > tol);
   bool first = true;  // p = z on the first iteration, z + beta p afterwards
+  int next_dots = 1;  // dots of the reduction that follows: two after step 1, where the recurrence may also break down
   int pb = 0;         // buffer that holds the current p (written in step 1)
   int rb = 0;         // buffer that holds the current r
   while (!done && !aborted) {
@@ -636,6 +706,7 @@ __global__ void __launch_bounds__(kSolveThreads, kOneRound ? 1 : 2) PcgSolveKern
       a.ap[row] = ap;
       d0 = Mul(pi, ap);
     }, t0, t1);
+    next_dots = 2;
     if (aborted) break;
     pb ^= 1;
     first = false;
@@ -666,6 +737,7 @@ __global__ void __launch_bounds__(kSolveThreads, kOneRound ? 1 : 2) PcgSolveKern
       d0 = Mul(ri, ri);
       d1 = Mul(ri, zi);
     }, t0, t1);
+    next_dots = 1;
     if (aborted) break;
     rb ^= 1;
     rr = t0;
@@ -717,11 +789,12 @@ __global__ void __launch_bounds__(kSolveThreads, kOneRound ? 1 : 2) PcgSolveKern
   }
   // epilogue: the true residual at exit
   if (!aborted) {
-    reduce(1, [&](int64_t row, double& d0, double&) {
+    reduce(next_dots, [&](int64_t row, double& d0, double&) {
       const double ax = RowDot<kOneRound>(a_row(row), [&](int32_t c) { return a.x[c]; });
       const double ri = __dsub_rn(a.b[row], ax);
       d0 = Mul(ri, ri);
     }, t0, t1);
+    next_dots = 1;
   }
   if (blockIdx.x == 0) {
     __syncthreads();
@@ -743,11 +816,23 @@ __global__ void __launch_bounds__(kSolveThreads, kOneRound ? 1 : 2) PcgSolveKern
       a.outcome->aborted = aborted ? 1 : 0;
     }
   }
-  // No block leaves while a neighbour may still store to its shared memory.
-  // After an abort a neighbour may be one reduction ahead: its cluster
-  // barriers there are matched here, and its own exit is the last one.
-  if (aborted) {
-    for (int64_t g = 1; g < groups; ++g) cluster.sync();
+  // No block leaves while a neighbour may still store to its shared memory.  All
+  // blocks of a cluster take part in the same reductions, so that every block
+  // that receives has waited for all that was sent to it.  A block that gives up
+  // after reduction k tells its cluster and takes part in reduction k + 1 with
+  // nothing to add (how many dots that one has follows from k); one that finds
+  // itself told leaves after k + 1, where the whole cluster is by then, since
+  // each block waits for its cluster's arrival.  A block that is done takes part
+  // in one more reduction too, because another may have given up after the last
+  // one.  Clusters leave one after another; the poisoned counter spares the
+  // others their wait.
+  if (!(solo ? sh.first_dead < reduction : sh.leave != 0)) {
+    if (aborted && threadIdx.x == 0) {
+      const uint32_t slot = SharedAddress(const_cast<unsigned long long*>(&sh.first_dead));
+      for (int k = 0; k < kClusterBlocks; ++k) StoreRemote(RemoteAddress(slot, k), reduction);
+      if (!solo) atomicOr(a.arrived + mine * kFlagStride, kPoison);
+    }
+    Farewell(pcg_smem, a.arrived, a.partial, a.longest, a.chunks, kRounds, group_count, reduction + 1, next_dots);
   }
   cluster.sync();
 }
@@ -894,7 +979,7 @@ void RunPcg(Ctx& ctx, const DevCsc<double>& a, const DevCsc<TM>& m, const double
   args.outcome = &c->outcome;
   args.longest = &c->longest;
   args.wait_ns = static_cast<unsigned long long>(g_wait_ns.exchange(static_cast<int64_t>(kWaitNs)));
-  args.free_polls = args.wait_ns == kWaitNs ? 4096 : 0;
+  args.free_polls = args.wait_ns == kWaitNs ? kFreePolls : 0;
   args.n = n;
   args.chunks = chunks;
   args.max_iterations = opt.max_iterations;
