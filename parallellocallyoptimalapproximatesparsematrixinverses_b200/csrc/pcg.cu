@@ -97,7 +97,7 @@ struct SolveMatrix {
   const int32_t* idx;
   const TV* val;
   int64_t* slice;      // per slice of 32 rows: offset in the sliced copy, or -1 (rows stay in CSR)
-  int32_t* slice_idx;
+  int32_t* slice_idx;  // null: no room for a copy, all rows stay in CSR
   TV* slice_val;
   unsigned long long* used;  // entries of the sliced copy taken so far
 };
@@ -175,7 +175,7 @@ __device__ int SliceRows(const SolveMatrix<TV>& m, int64_t slice, int64_t n, int
   bool dense;
   const int width = SliceWidth(m, slice * kWarp + lane, n, &first, &len, &dense);
   long long at = -1;
-  if (dense) {
+  if (dense && m.slice_idx != nullptr) {
     if (lane == 0) at = static_cast<long long>(atomicAdd(m.used, static_cast<unsigned long long>(width) * kWarp));
     at = __shfl_sync(0xffffffffu, at, 0);
     for (int e = 0; e < len; ++e) {
@@ -937,18 +937,27 @@ void RunPcg(Ctx& ctx, const DevCsc<double>& a, const DevCsc<TM>& m, const double
   vectors.Reserve(static_cast<size_t>(6 * n), st);
   history.Reserve(static_cast<size_t>(opt.max_iterations), st);
   partial.Reserve(static_cast<size_t>(4 * chunks), st);
-  // the sliced copies (at most twice the entries plus two per row, see SliceRows) and their slice offsets
-  const size_t a_room = static_cast<size_t>(2 * a.nnz + 2 * (n + kWarp));
-  const size_t m_room = static_cast<size_t>(2 * m.nnz + 2 * (n + kWarp));
+  // the sliced copies (at most twice the entries plus two per row, see SliceRows) and their slice offsets;
+  // a matrix whose copy the device has no room for is read as it is
   DevBuf<int64_t> slice_at;
   DevBuf<int32_t> a_idx, m_idx;
   DevBuf<double> a_val;
   DevBuf<TM> m_val;
   slice_at.Reserve(static_cast<size_t>(2 * slices), st);
-  a_idx.Reserve(a_room, st);
-  a_val.Reserve(a_room, st);
-  m_idx.Reserve(m_room, st);
-  m_val.Reserve(m_room, st);
+  const auto reserve_copy = [&](int64_t nnz, DevBuf<int32_t>& idx, auto& val) {
+    const size_t room = static_cast<size_t>(2 * nnz + 2 * (n + kWarp));
+    try {
+      idx.Reserve(room, st);
+      val.Reserve(room, st);
+    } catch (const CudaError&) {
+      cudaGetLastError();
+      idx.Release();
+      val.Release();
+      CacheFlush(st);
+    }
+  };
+  reserve_copy(a.nnz, a_idx, a_val);
+  reserve_copy(m.nnz, m_idx, m_val);
   // two slice cursors, the longest walk and the outcome, zeroed
   struct Control {
     unsigned long long used[2];
