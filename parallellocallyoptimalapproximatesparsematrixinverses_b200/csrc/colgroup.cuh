@@ -25,8 +25,9 @@
 
 namespace spai {
 
+// (aligned to 16 bytes at most: the arrays are placed at multiples of 16)
 template <class T, int C>
-struct alignas(sizeof(T) * C) GroupValues {
+struct alignas(sizeof(T) * C < 16 ? sizeof(T) * C : 16) GroupValues {
   T v[C];
 };
 
