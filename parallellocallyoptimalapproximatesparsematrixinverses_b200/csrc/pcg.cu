@@ -1030,7 +1030,6 @@ void RunPcg(Ctx& ctx, const DevCsc<double>& a, const DevCsc<TM>& m, const double
   if (count < 1 || count > opt.max_iterations) throw CudaError("PCG returned an invalid iteration count");
   result.history.resize(static_cast<size_t>(count));
   result.status = outcome.status;
-  result.spmv_count = 2 + 3 * (count - 1);
   // algorithmic bytes of the solve: per iteration A and M once plus the vector traffic (17 n doubles)
   const double per_iteration = static_cast<double>(a.nnz) * 12.0 + static_cast<double>(m.nnz) * (sizeof(TM) + 4) +
                                8.0 * 17.0 * static_cast<double>(n);

@@ -22,7 +22,6 @@ struct PcgOptions {
 struct PcgResult {
   std::vector<double> history;
   int64_t status = 0;  // 0 iteration limit, 1 converged, 2 recurrence breakdown, 3 non-finite residual
-  int64_t spmv_count = 0;
 };
 
 // Solves with x0 = 0; b and x are device vectors of length a.rows.
