@@ -164,3 +164,33 @@ def test_batched_steps_account_for_their_bytes(require_gpu):
     for name in names:
         assert alone[name][0] == batch[name][0] == 6
         assert alone[name][1] == batch[name][1] > 0
+
+
+# the largest cap and the longest rows the fused kernels take, in groups of four
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("case", ["top_32", "rows_of_13", "rows_of_9"])
+def test_the_largest_groups_run_fused(require_gpu, case, precision):
+    a, topk = {"top_32": lambda: (problems.diffusion_2d(101, 1.0, 5), 32),
+               "rows_of_13": lambda: (band(9_999, [1, 2, 3, 40, 41, 90]), 5),
+               "rows_of_9": lambda: (band(9_999, [1, 2, 50, 51]), 12)}[case]()
+    kw = dict(M0=problems.diagonal_inverse(a), max_iterations=9, tolerance=0.0, max_density=topk / a.shape[0],
+              topk_per_column=topk, precision=precision)
+    want = unfused(lambda: global_spai.mr(a, **kw))
+    got, counts = profiled(lambda: global_spai.mr(a, **kw), "fused_drop", "fused_drop_columns", "drop_update")
+    assert counts["fused_drop"][0] + counts["fused_drop_columns"][0] == 9
+    assert counts["fused_drop"][0] >= 1 and counts["drop_update"][0] == 1
+    assert_same_result(got, want, f"{case} {precision}")
+
+
+# an entry of A beyond FP32's range: the column groups would multiply it by the 0 of an absent entry
+def test_a_system_that_is_not_finite_in_fp32_storage(require_gpu):
+    bad = problems.diffusion_2d(20, 1.0, 4).tolil()
+    bad[7, 8] = bad[8, 7] = 1e39
+    batch = [problems.diffusion_2d(31, 1.0, 2), sparse.csc_matrix(bad), problems.diffusion_3d(9, 1.0, 1)]
+    kw = dict(max_iterations=6, tolerance=0.0, max_density=1.0, topk_per_column=6, precision="mixed")
+    want = unfused(lambda: global_spai.mr_batched(batch, **kw))
+    got, counts = profiled(lambda: global_spai.mr_batched(batch, **kw), "fused_drop", "fused_drop_columns")
+    assert counts["fused_drop"][0] == 0 and counts["fused_drop_columns"][0] >= 1
+    for b, (g, w) in enumerate(zip(got, want)):
+        assert_same_result(g, w, f"system {b}")
+    assert not np.isfinite(got[1].history["residual_norm"][0]) and np.all(np.isfinite(got[0].history["residual_norm"]))
