@@ -95,7 +95,7 @@ def test_batched_steps_match_the_unfused_kernels(require_gpu, systems, precision
         batch = [problems.diffusion_2d(m, 0.5, m) for m in (3, 17, 31)] + [problems.diffusion_3d(9, 1.0, 1),
                                                                            problems.tridiagonal(5)]
         kw = dict(max_iterations=12, tolerance=0.3, max_density=1.0, topk_per_column=7, precision=precision)
-    else:  # the fused steps are given up and the whole batch runs unfused
+    else:  # the fused steps are given up and the rest of the batch runs unfused
         batch = [_star(9, 14), problems.diffusion_2d(12, 0.5, 2)]
         kw = dict(max_iterations=6, tolerance=0.0, max_density=1.0, topk_per_column=2, precision=precision)
     lib = _lib.load()

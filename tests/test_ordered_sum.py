@@ -31,8 +31,8 @@ def test_pieces_give_the_loops_bits(program, kind):
         assert int(done.stdout) > 0  # summaries were used, not only the term-by-term path
 
 
-# batches of one column up to the whole matrix: blocks of 32, 256 and 1024
-# threads, tiles that end inside a piece, sums with ties (the Laplacian's dyadic values)
+# batches of one column up to the whole matrix: blocks of 32 and 256 threads and
+# clusters of eight blocks, tiles that end inside a piece, sums with ties (the Laplacian's dyadic values)
 @pytest.mark.gpu
 @pytest.mark.parametrize("threads", [1, 2, 37, 1521])
 @pytest.mark.parametrize("method", ["cg", "mr", "lomr"])
