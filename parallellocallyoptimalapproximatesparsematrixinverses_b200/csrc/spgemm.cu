@@ -578,6 +578,10 @@ void LaunchValues(Ctx& ctx, ValuesArgs<T> args) {
     args.piece = std::clamp<int64_t>(CeilDiv(CeilDiv(args.entries, int64_t{32} * ctx.sm_count), kWarp) * kWarp, kWarp,
                                      kValuesPiece);
     split = std::clamp<int64_t>(CeilDiv(CeilDiv(args.entries, cols), args.piece), 1, 32);
+  } else if (split > 1 && args.entries >= cols * (kValuesPiece / 4)) {
+    // many long columns: every split looks at every column, not at 32 per warp
+    kernel = ValuesKernel<T, true>;
+    args.piece = kValuesPiece;
   }
   SPAI_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(ValuesSlabBytes(kValuesMaxWords) * kWarps)));
