@@ -345,6 +345,28 @@ __host__ __device__ inline size_t ValuesSlabBytes(int words) {
   return Round16(static_cast<size_t>(words) * 4) + Round16(static_cast<size_t>(words) * 2);
 }
 
+// Entry p = (i, j) of the output from its sum (`has`: from any product at all);
+// true when a stored value is an exact zero that has to be pruned.
+template <class T>
+__device__ __forceinline__ bool StoreValue(const ValuesArgs<T>& a, int64_t p, int32_t i, int64_t j, T acc, bool has) {
+  if (a.mode == static_cast<int>(ValueMode::kMasked)) {
+    a.out_f64[p] = has ? static_cast<double>(acc) : 0.0;
+    return false;
+  }
+  if (a.mode == static_cast<int>(ValueMode::kProjection)) {
+    a.out[p] = Mul(a.row_scale[i], acc);
+    return false;
+  }
+  T v = acc;
+  if (a.mode == static_cast<int>(ValueMode::kResidual)) {
+    v = has ? -acc : T(0);
+    if (static_cast<int64_t>(i) == j) v = has ? Add(v, T(1)) : T(1);
+  }
+  a.out[p] = v;
+  if (a.z_out != nullptr) a.z_out[p] = Mul(a.row_scale[i], v);
+  return a.prune && v == T(0);  // Eigen prune(0.0): +-0 go, NaN stays
+}
+
 constexpr int kValuesPiece = 4096;  // entries of a column that one warp takes at a time, at most
 constexpr int kValuesMaxWords = 1024;
 
@@ -453,23 +475,7 @@ __global__ void __launch_bounds__(256) ValuesKernel(ValuesArgs<T> a, int words_c
           }
         }
       }
-      if (a.mode == static_cast<int>(ValueMode::kMasked)) {
-        a.out_f64[p] = has ? static_cast<double>(acc) : 0.0;
-        continue;
-      }
-      if (a.mode == static_cast<int>(ValueMode::kProjection)) {
-        a.out[p] = Mul(a.row_scale[i], acc);
-        continue;
-      }
-      T v = acc;
-      if (a.mode == static_cast<int>(ValueMode::kResidual)) {
-        v = has ? -acc : T(0);
-        if (static_cast<int64_t>(i) == j) v = has ? Add(v, T(1)) : T(1);
-      }
-      const T stored = v;
-      a.out[p] = stored;
-      if (a.z_out != nullptr) a.z_out[p] = Mul(a.row_scale[i], stored);
-      if (a.prune && stored == T(0)) zero_seen = true;  // Eigen prune(0.0): +-0 go, NaN stays
+      zero_seen |= StoreValue(a, p, i, j, acc, has);
     }
     __syncwarp();
     if (mapped) {
@@ -493,36 +499,37 @@ __global__ void __launch_bounds__(256) ValuesKernel(ValuesArgs<T> a, int words_c
   if (__any_sync(0xffffffffu, zero_seen) && lane == 0) atomicOr(a.flag, 1);
 }
 
-// The masked product for short mask columns: one thread per mask entry, its
-// eight searches of B(:, j) in lock step.  Below about 32 entries a column a
-// warp per column leaves lanes idle and its bitmap is not paid back: 200 us
-// against 278 us for the two masks of the 47^3 residual gradient (25 and 7
-// entries a column), 75 against 45 us the other way for 40 entries a column.
-constexpr int64_t kMaskedWarpEntries = 32;
+// Short columns: one thread per output entry, its eight searches of B(:, j) in
+// lock step.  Below about 32 entries a column a warp per column leaves lanes
+// idle and its bitmap is not paid back: 200 us against 278 us for the two masks
+// of the 47^3 residual gradient (25 and 7 entries a column), 75 against 45 us
+// the other way for 40 entries a column.  Where some rows of X are long, the
+// one lane that has such a row holds up its warp: an arrow matrix of 200,000
+// rows (two entries a column, one row of 200,000) takes about 80 ms against
+// 1,680.
+constexpr int64_t kWarpEntries = 32;
 
-template <class T>
-__global__ void ColumnIdsKernel(CscView<T> m, int32_t* __restrict__ cols) {
+__global__ void ColumnIdsKernel(const int64_t* __restrict__ ptr, int64_t count, int32_t* __restrict__ cols) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t j = warp; j < m.cols; j += warps) {
-    for (int64_t p = m.ptr[j] + lane; p < m.ptr[j + 1]; p += kWarp) cols[p] = static_cast<int32_t>(j);
+  for (int64_t j = warp; j < count; j += warps) {
+    for (int64_t p = ptr[j] + lane; p < ptr[j + 1]; p += kWarp) cols[p] = static_cast<int32_t>(j);
   }
 }
 
 template <class T>
-__global__ void __launch_bounds__(256) MaskedEntriesKernel(CscView<T> x_csr, CscView<T> b,
-                                                           const int32_t* __restrict__ rows,
-                                                           const int32_t* __restrict__ cols, int64_t count,
-                                                           double* __restrict__ out) {
-  for (int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < count;
+__global__ void __launch_bounds__(256) EntriesKernel(ValuesArgs<T> a, const int32_t* __restrict__ cols) {
+  bool zero_seen = false;
+  for (int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < a.entries;
        p += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int32_t i = rows[p];
-    const int64_t bs = b.ptr[cols[p]];
-    const int blen = static_cast<int>(b.ptr[cols[p] + 1] - bs);
-    const int32_t* b_idx = b.idx + bs;
-    const int64_t xs = x_csr.ptr[i];
-    const int64_t xe = x_csr.ptr[i + 1];
+    const int32_t i = a.rows[p];
+    const int32_t j = cols[p];
+    const int64_t bs = a.b.ptr[j];
+    const int blen = static_cast<int>(a.b.ptr[j + 1] - bs);
+    const int32_t* b_idx = a.b.idx + bs;
+    const int64_t xs = a.x_csr.ptr[i];
+    const int64_t xe = a.x_csr.ptr[i + 1];
     T acc = T(0);
     bool has = false;
     for (int64_t q0 = xs; q0 < xe; q0 += 8) {
@@ -532,8 +539,8 @@ __global__ void __launch_bounds__(256) MaskedEntriesKernel(CscView<T> x_csr, Csc
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         const int64_t q = q0 + u;
-        kk[u] = q < xe ? x_csr.idx[q] : INT32_MAX;
-        xv[u] = q < xe ? x_csr.val[q] : T(0);
+        kk[u] = q < xe ? a.x_csr.idx[q] : INT32_MAX;
+        xv[u] = q < xe ? a.x_csr.val[q] : T(0);
         at[u] = 0;
       }
       int len = blen;
@@ -548,18 +555,28 @@ __global__ void __launch_bounds__(256) MaskedEntriesKernel(CscView<T> x_csr, Csc
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         if (blen > 0 && q0 + u < xe && b_idx[at[u]] == kk[u]) {
-          const T prod = Mul(xv[u], b.val[bs + at[u]]);
+          const T prod = Mul(xv[u], a.b.val[bs + at[u]]);
           acc = has ? Add(acc, prod) : prod;
           has = true;
         }
       }
     }
-    out[p] = has ? static_cast<double>(acc) : 0.0;
+    zero_seen |= StoreValue(a, p, i, j, acc, has);
   }
+  if (__any_sync(0xffffffffu, zero_seen) && (threadIdx.x & 31) == 0) atomicOr(a.flag, 1);
 }
 
 template <class T>
 void LaunchValues(Ctx& ctx, ValuesArgs<T> args) {
+  if (args.entries < kWarpEntries * args.b.cols) {
+    ctx.sg_cols.Reserve(static_cast<size_t>(args.entries), ctx.stream);
+    ColumnIdsKernel<<<GridFor(args.b.cols * kWarp, 256), 256, 0, ctx.stream>>>(args.c_ptr, args.b.cols,
+                                                                             ctx.sg_cols.data());
+    SPAI_LAUNCH_CHECK();
+    EntriesKernel<T><<<GridFor(args.entries, 256), 256, 0, ctx.stream>>>(args, ctx.sg_cols.data());
+    SPAI_LAUNCH_CHECK();
+    return;
+  }
   // a bitmap over all rows of B, up to 32,768 of them (wider ones would cost resident warps)
   const int words = static_cast<int>(std::min<int64_t>(kValuesMaxWords, CeilDiv(args.b.rows, 32) + 1));
   constexpr int kWarps = 8;
@@ -1426,15 +1443,6 @@ bool Spgemm(Ctx& ctx, const DevCsc<T>& x_csc, const DevCsc<T>& x_csr, const DevC
 template <class T>
 void SpgemmMasked(Ctx& ctx, const DevCsc<T>& x_csr, const DevCsc<T>& b, const DevCsc<T>& mask, double* out) {
   if (mask.nnz == 0) return;
-  if (mask.nnz < kMaskedWarpEntries * mask.cols) {
-    ctx.sg_cols.Reserve(static_cast<size_t>(mask.nnz), ctx.stream);
-    ColumnIdsKernel<T><<<GridFor(mask.cols * kWarp, 256), 256, 0, ctx.stream>>>(View(mask), ctx.sg_cols.data());
-    SPAI_LAUNCH_CHECK();
-    MaskedEntriesKernel<T><<<GridFor(mask.nnz, 256), 256, 0, ctx.stream>>>(
-        View(x_csr), View(b), mask.idx.data(), ctx.sg_cols.data(), mask.nnz, out);
-    SPAI_LAUNCH_CHECK();
-    return;
-  }
   ValuesArgs<T> va{};
   va.x_csr = View(x_csr);
   va.b = View(b);
