@@ -369,7 +369,8 @@ void LaunchOrderedSum(Ctx& ctx, const T* val, const int64_t* ptr, int64_t entrie
     SPAI_LAUNCH_CHECK();
     return;
   }
-  // short batches: a block each, small enough that a round is not padding
+  // short batches: a block each, small enough that a round is not padding.  With 32 and 256 threads: 8.3 and 13.6 us
+  // for batches of 128 squares, 11.9 and 11.9 for 256, 18.9 and 17.7 for 512, 31.8 and 25.8 for 1,024 (140,000 in all).
   const int threads = average >= 512 ? 256 : kWarp;
   const size_t smem = sizeof(double) * static_cast<size_t>(threads) * (kTermsPerThread + 2);
   OrderedSumKernel<T, kSquares><<<static_cast<unsigned>(batches < cap ? batches : cap), threads, smem, ctx.stream>>>(
