@@ -22,7 +22,7 @@
 // is formed with the same operations, in the same order, as the unfused
 // kernels (update.cu, spgemm.cu), so results are bit-identical.  A column
 // that does not fit its slots flags an overflow: the loop stops and the
-// caller reruns the solve on the unfused path.
+// caller reruns the solve, or goes on with the batch, on the unfused path.
 
 #include <cuda_runtime.h>
 

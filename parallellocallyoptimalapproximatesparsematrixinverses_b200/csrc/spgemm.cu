@@ -10,9 +10,10 @@
 //  2. row-set list    (same warps, after the scan of the counts) -- writes the
 //     sorted rows of every column (bitmap: lane-blocked popcount prefix;
 //     hash: compaction + bitonic sort).
-//  3. values          (one warp per output column) -- entry (i, j) walks row i
-//     of X (CSR copy) in ascending k, finds each k in column j of B through a
-//     bitmap of that column, and accumulates the first product x*y then += x*y
+//  3. values          (one or more warps per output column; a thread per
+//     entry where columns are short) -- entry (i, j) walks row i of X (CSR copy)
+//     in ascending k, finds each k in column j of B through a bitmap of that
+//     column (by bisection), and accumulates the first product x*y then += x*y
 //     in ascending k: the reference's accumulation order (Eigen's conservative
 //     sparse product), no FMA.  Products and sums use the storage type's
 //     arithmetic: FP64 for double storage (bit-compatible with the reference),
